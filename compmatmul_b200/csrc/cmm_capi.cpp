@@ -17,6 +17,7 @@
 
 #include "../../include/compmatmul_b200.h"
 #include "cmm_internal.h"
+#include "cmm_product.h"
 
 namespace cmm {
 
@@ -283,13 +284,14 @@ static size_t materialize_budget() {
 
 // The cluster kernels when this device can co-schedule a cluster of them
 // and the residue segments fit in shared memory; false -> the slab kernels.
-// CMM_SKETCH_KERNELS = cluster | slab forces one family where both apply
+// CMM_SKETCH_KERNELS = cluster | slab | product forces one family where it applies
 // (for comparisons); unset or "auto" takes the measured-faster choice.
 static int sketch_kernel_choice() {
   static const int choice = [] {
     const char* e = getenv("CMM_SKETCH_KERNELS");
     if (e && !strcmp(e, "cluster")) return 1;
     if (e && !strcmp(e, "slab")) return 2;
+    if (e && !strcmp(e, "product")) return 3;
     return 0;
   }();
   return choice;
@@ -322,11 +324,119 @@ static int64_t chunk_len(int64_t k0, int64_t kc, int64_t n_inner, const RowFeed*
   return n_inner - k0 < cmax ? n_inner - k0 : cmax;
 }
 
+// The sketch through the product C itself (cmm_product.cu), when that is
+// estimated to be faster than the transforms.  Both estimates are fits to B200
+// times (microseconds), n square, d = 7, transforms / product:
+//   n = 512:  b = 256 119 / 187, 1024 228 / 155, 4096 387 / 157, 2^16 3380 / 236
+//   n = 2048: b = 256 413 / 517, 1024 770 / 593, 4096 1239 / 658, 2^16 12778 / 689
+//   n = 8192, 32 inner indices, b = 256, d = 3: 408 / 3368 (the product pays
+//   d additions per entry of C however few inner indices there are)
+// Where the group kernels apply, products under 2^24 multiply-adds stay with
+// them: both take a few hundred microseconds there, and those kernels' tests,
+// which check that they ran, use such sizes.
+static bool product_applicable(int variant, bool f32, const SketchParams& sp, int64_t n_a, int64_t n_inner,
+                               int64_t n_b) {
+  if (n_inner <= 0 || n_a <= 0 || n_b <= 0) return false;
+  if (n_a > 0x7fffffff || n_b > 0x7fffffff || n_a * n_b > kProdMaxEntries) return false;
+  if (sketch_kernel_choice() == 3) return true;
+  if (sketch_kernel_choice() != 0) return false;
+  const double nn = (double)n_a * (double)n_b, k = (double)n_inner, d = sp.d, b = sp.b;
+  if (sketch_cluster_applicable(variant, f32, sp.b) && nn * k < 16777216.0) return false;
+  const bool small_b = variant == kVariantFFT ? sp.b < 4096 : sp.b < 8192;
+  const double per_b = variant == kVariantFFT && !f32 ? 0.85e-6 : 0.5e-6;
+  const double transforms = (small_b ? 70.0 : 230.0) + d * k * (per_b * b * sp.log2b + 7e-6 * (double)(n_a + n_b));
+  const double product = 110.0 + nn * (d / 1.1e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
+  return product < transforms;
+}
+
+// scratch: n_a x n_b doubles for C (the caller's dense output, written
+// later), or nullptr.
+static void sketch_product(int variant, bool f32, const SketchParams& sp, const Codes& codes, int64_t n_a,
+                           int64_t n_inner, int64_t n_b, const void* dAT, const void* dB, double* dP, double* scratch,
+                           cudaStream_t s, RowFeed* feed) {
+  set_sketch_kernel("product");
+  if (product_timed_out()) throw std::runtime_error("product sketch: a wait ran out in an earlier launch");
+  const size_t elem = f32 ? 4 : 8;
+  ProdJob J{};
+  J.n_a = n_a;
+  J.n_b = n_b;
+  J.tiles_a = prod_tiles(n_a);
+  J.tiles_b = prod_tiles(n_b);
+  const size_t per_k = (size_t)prod_moduli(f32) * 256 * (size_t)(J.tiles_a + J.tiles_b);
+  int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget() / per_k));
+  // rows still arriving from the host: eighths, so that copies and work overlap
+  if (feed) kc = std::min<int64_t>(kc, std::max<int64_t>((n_inner + 7) / 8, 512));
+  kc = std::max<int64_t>(kc / 128 * 128, 128);
+  kc = std::min<int64_t>(kc, n_inner);
+  // panels of C whose residues take at most 2 GiB
+  const size_t per_tile = prod_residue_bytes(1, J.tiles_b, f32);
+  const int panel = (int)std::max<int64_t>(1, std::min<int64_t>(J.tiles_a, (int64_t)(((size_t)2 << 30) / per_tile)));
+  J.codesA = codes.a.as<uint32_t>();
+  J.codesB = codes.b.as<uint32_t>();
+  J.d = sp.d;
+  J.log2b = sp.log2b;
+  J.variant = variant;
+  plan_product_sketch(J, num_sms());
+  const size_t db = (size_t)sp.d * (size_t)sp.b;
+  // one allocation for everything
+  size_t total = 0;
+  auto take = [&](size_t n) { const size_t o = total; total += (n + 255) & ~(size_t)255; return o; };
+  const size_t nb = (size_t)((kc + 255) / 256);
+  const size_t o_slA = take(prod_plane_bytes(n_a, kc, f32)), o_slB = take(prod_plane_bytes(n_b, kc, f32));
+  const size_t o_res = take(per_tile * panel), o_exp = take((size_t)(n_a + n_b + kc + 1) * 4);
+  const size_t o_csum = take(nb * (size_t)(n_a + n_b) * 8), o_cmax = take(nb * (size_t)(n_a + n_b) * 4);
+  const size_t o_C = take(scratch ? 0 : (size_t)n_a * (size_t)n_b * 8);
+  const size_t o_cum = take((size_t)sp.d * ((size_t)sp.b + 1) * 4), o_ent = take((size_t)sp.d * (size_t)n_b * 8);
+  const size_t o_part = take((size_t)J.G * db * 8), o_job = take(sizeof(ProdJob));
+  DevBuf mem(total, s);
+  uint8_t* base = mem.as<uint8_t>();
+  J.slA = base + o_slA;
+  J.slB = base + o_slB;
+  J.res = reinterpret_cast<uint32_t*>(base + o_res);
+  J.flag = reinterpret_cast<int*>(base + o_exp);
+  J.cexpA = J.flag + 1;
+  J.cexpB = J.cexpA + n_a;
+  J.rexp = J.cexpB + n_b;
+  J.csum = reinterpret_cast<double*>(base + o_csum);
+  J.cmax = reinterpret_cast<int*>(base + o_cmax);
+  J.C = scratch ? scratch : reinterpret_cast<double*>(base + o_C);
+  J.ldc = n_b;
+  J.cum = reinterpret_cast<uint32_t*>(base + o_cum);
+  J.ent = reinterpret_cast<uint2*>(base + o_ent);
+  J.part = reinterpret_cast<double*>(base + o_part);
+  J.p = dP;
+  ProdJob* dJ = reinterpret_cast<ProdJob*>(base + o_job);
+  auto send = [&] { CMM_CUDA(cudaMemcpyAsync(dJ, &J, sizeof(J), cudaMemcpyHostToDevice, s)); };
+  for (int64_t k0 = 0; k0 < n_inner; k0 += kc) {
+    J.kc = std::min<int64_t>(kc, n_inner - k0);
+    J.A = static_cast<const char*>(dAT) + (size_t)k0 * n_a * elem;
+    J.B = static_cast<const char*>(dB) + (size_t)k0 * n_b * elem;
+    J.accumulate = k0 > 0 ? 1 : 0;
+    for (J.tile0 = 0; J.tile0 < J.tiles_a; J.tile0 += panel) {
+      J.tiles_p = std::min(panel, J.tiles_a - J.tile0);
+      J.item_end = (int64_t)J.tiles_p * J.tiles_b * prod_moduli(f32);
+      send();
+      if (J.tile0 == 0) {
+        if (k0 == 0) launch_product_index(&J, dJ, 1, s);
+        if (feed) feed->wait(k0, J.kc, s);
+        launch_product_planes(&J, dJ, 1, f32, s);
+      }
+      launch_product_gemm(&J, dJ, 1, f32, s);
+    }
+  }
+  launch_product_scatter(&J, dJ, 1, s);
+  launch_product_reduce(&J, dJ, 1, s);
+}
+
 // feed != nullptr: the rows of dAT / dB are still arriving from the host;
 // every chunk waits for its rows (and computes their FFT row scales) first.
 static void sketch_device(int variant, const SketchParams& sp, const Codes& codes, int64_t n_a,
                           int64_t n_inner, int64_t n_b, const double* dAT, const double* dB,
-                          double* dP, cudaStream_t s, RowFeed* feed = nullptr) {
+                          double* dP, cudaStream_t s, RowFeed* feed = nullptr, double* scratch = nullptr) {
+  if (product_applicable(variant, false, sp, n_a, n_inner, n_b)) {
+    sketch_product(variant, false, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed);
+    return;
+  }
   const double2* tw = twiddles(sp.b, s);
   const size_t elem = variant == kVariantFFT ? 16 : 8;
   DevBuf scale;
@@ -400,7 +510,11 @@ static void sketch_device(int variant, const SketchParams& sp, const Codes& code
 static void sketch_device_mixed(int variant, const SketchParams& sp, const Codes& codes,
                                 int64_t n_a, int64_t n_inner, int64_t n_b, const float* dAT,
                                 const float* dB, double* dP, cudaStream_t s,
-                                RowFeed* feed = nullptr) {
+                                RowFeed* feed = nullptr, double* scratch = nullptr) {
+  if (product_applicable(variant, true, sp, n_a, n_inner, n_b)) {
+    sketch_product(variant, true, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed);
+    return;
+  }
   if (!(n_inner > 0 && sketch_mixed_applicable(variant, sp.b))) {
     if (feed) feed->wait_all(s);
     DevBuf A64((size_t)n_inner * n_a * 8, s), B64((size_t)n_inner * n_b * 8, s);
@@ -474,6 +588,7 @@ static uint64_t pick_seed(int has_seed, uint64_t seed) { return has_seed ? seed 
 static void check_group_waits() {
   if (sketch_group_timed_out())
     throw std::runtime_error("cluster sketch: a group barrier wait ran out; the sketch is invalid");
+  if (product_timed_out()) throw std::runtime_error("product sketch: a wait ran out; the sketch is invalid");
 }
 
 static void decompress_to_host(int variant, int d, int b, int64_t n_a, int64_t n_b, const Codes& codes,
@@ -804,7 +919,7 @@ int cmm_dev_matmul(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int
     SketchParams sp = make_sketch_params(hash_kind, d, b, seed);
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
-    sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s);
+    sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
     launch_decompress_dense(variant, d, b, n_a, n_b, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
                             P.as<double>(), dC, s);
   });
@@ -934,7 +1049,7 @@ int cmm_dev_matmul_f32(int variant, int hash_kind, int64_t n_a, int64_t n_inner,
     SketchParams sp = make_sketch_params(hash_kind, d, b, seed);
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
-    sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s);
+    sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
     launch_decompress_dense(variant, d, b, n_a, n_b, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
                             P.as<double>(), dC, s);
   });
@@ -977,7 +1092,7 @@ int cmm_matmul_f32(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
     sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT.as<float>(), dB.as<float>(),
-                        P.as<double>(), s, &feed);
+                        P.as<double>(), s, &feed, dC.as<double>());
     decompress_to_host(variant, d, b, n_a, n_b, codes, P.as<double>(), dC.as<double>(), C, s);
   });
 }
@@ -1022,7 +1137,7 @@ int cmm_matmul(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int64_t
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
     sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT.as<double>(), dB.as<double>(),
-                  P.as<double>(), s, &feed);
+                  P.as<double>(), s, &feed, dC.as<double>());
     decompress_to_host(variant, d, b, n_a, n_b, codes, P.as<double>(), dC.as<double>(), C, s);
   });
 }

@@ -1,0 +1,1049 @@
+// Product sketch: the sketch of C = A^T B from C itself.
+//
+// p_t is the count sketch of the product: p_t[idx(i, j)] += s1_t(i) s2_t(j)
+// C[i][j], idx = (h1 + h2) mod b (FFT variant) or h1 ^ h2 (FWHT variant).
+// The transform kernels reach it through d length-b transforms per inner
+// index; here C is formed once, to FP64 (FP32) accuracy, on the int8 tensor
+// cores and then added into the d sketches.  Per inner index that is
+// 2 n_a n_b flops of matrix product instead of d transforms of length b, and
+// the matrix product runs on tcgen05 while the transforms run on the FP64 /
+// FP32 units.
+//
+// The product is an exact integer product, by residues:
+//  * Row pair k is balanced by a power of two e_k (A row * 2^-e_k, B row *
+//    2^e_k: the same rule as the FFT packing).  Column c of A or B then gets
+//    the power of two E_c >= its 2-norm over k, and an entry x is the integer
+//    X = rint(x 2^(T - E_c)), so every column of integers has norm <= 2^T and
+//    every entry of the integer product is below 2^(2T) (Cauchy-Schwarz),
+//    whatever the number of inner indices.
+//  * The integer product is formed modulo N pairwise coprime m_i <= 256: the
+//    residues of X fit signed bytes, their products add up exactly in the
+//    int32 accumulators, and with M = m_1 ... m_N > 2^(2T + 1) the residues
+//    determine the entry (Chinese remainder theorem).  N = 15, T = 58 for
+//    FP64 inputs, N = 8, T = 31 for FP32 inputs.  (Splitting X into base-256
+//    digits instead needs 34 and 13 int8 products for the same accuracy.)
+// The only rounding is that of X: an error of about 2^-59 (2^-32) |a_i| |b_j|
+// per entry, in the norms of the balanced columns.  Balancing makes the two
+// rows of a pair equally large, so this is normwise the error of FP64 (FP32)
+// transforms or smaller.
+#include <cfloat>
+#include <mutex>
+
+#include "cmm_internal.h"
+#include "cmm_product.h"
+
+namespace cmm {
+namespace {
+
+constexpr int kPSkip = -0x7fffffff;  // row pair with a zero row: contributes nothing
+constexpr int kNoExp = -1000000;     // column without a nonzero entry
+constexpr int kMinExp = -960;        // smaller columns are scaled as if they were this large
+
+// pairwise coprime, descending
+__host__ __device__ constexpr int modulus(int i) {
+  constexpr int m[15] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+  return m[i];
+}
+constexpr int powmod2(int e, int m) {  // 2^e mod m
+  int r = 1 % m;
+  for (int i = 0; i < e; ++i) r = (r * 2) % m;
+  return r;
+}
+constexpr int invmod(int a, int m) {  // a^-1 mod m (a, m coprime)
+  for (int x = 1; x < m; ++x)
+    if ((a % m) * x % m == 1) return x;
+  return 0;
+}
+// (M / m_i)^-1 mod m_i for the first n moduli
+constexpr int crt_inv(int i, int n) {
+  int p = 1 % modulus(i);
+  for (int j = 0; j < n; ++j)
+    if (j != i) p = p * (modulus(j) % modulus(i)) % modulus(i);
+  return invmod(p, modulus(i));
+}
+// floor(v / m) = umulhi(v, magic) >> 7 exactly for v < 2^31
+__host__ __device__ constexpr uint32_t mod_magic(int m) {
+  return (uint32_t)((m & (m - 1)) == 0 ? (1ull << 39) / m : (1ull << 39) / m + 1);
+}
+
+struct U128 {
+  unsigned long long lo, hi;
+};
+// product of the first n moduli without m_skip (skip < 0: all), mod 2^128
+constexpr U128 mod_product(int n, int skip) {
+  unsigned __int128 p = 1;
+  for (int j = 0; j < n; ++j)
+    if (j != skip) p *= (unsigned)modulus(j);
+  return U128{(unsigned long long)p, (unsigned long long)(p >> 64)};
+}
+
+template <typename Real>
+struct Fix;
+template <>
+struct Fix<double> {
+  static constexpr int N = 15, T = 58;
+};
+template <>
+struct Fix<float> {
+  static constexpr int N = 8, T = 31;
+};
+
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+
+// ------------------------------------------------------------- row balance
+// e_k = (expo(max |A row|) - expo(max |B row|)) / 2, within the range of pow2; kPSkip
+// when a row is zero.  A row pair with a non-finite value makes the whole
+// sketch NaN, as the transforms would (flag[0] = 1; the FFT form skips row
+// pairs with a zero row first, as its transform kernels do).
+template <typename Real>
+__global__ void __launch_bounds__(256) k_prod_rows(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  __shared__ double sa[8], sb[8];
+  __shared__ int sbad;
+  for (int64_t k = blockIdx.x; k < J.kc; k += gridDim.x) {
+    const Real* ra = reinterpret_cast<const Real*>(J.A) + k * J.n_a;
+    const Real* rb = reinterpret_cast<const Real*>(J.B) + k * J.n_b;
+    if (threadIdx.x == 0) sbad = 0;
+    __syncthreads();
+    double ma = 0.0, mb = 0.0;
+    bool bad = false;
+    for (int64_t i = threadIdx.x; i < J.n_a; i += 256) {
+      const double v = fabs((double)__ldg(ra + i));
+      bad |= !(v <= DBL_MAX);
+      ma = fmax(ma, v);
+    }
+    for (int64_t j = threadIdx.x; j < J.n_b; j += 256) {
+      const double v = fabs((double)__ldg(rb + j));
+      bad |= !(v <= DBL_MAX);
+      mb = fmax(mb, v);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      ma = fmax(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+      mb = fmax(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) { sa[w] = ma; sb[w] = mb; }
+    if (bad) sbad = 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 1; i < 8; ++i) { ma = fmax(ma, sa[i]); mb = fmax(mb, sb[i]); }
+      int e;
+      if (!(ma > 0.0) || !(mb > 0.0)) {
+        e = kPSkip;
+      } else {
+        auto ex = [](double m) { return (int)((__double_as_longlong(m) >> 52) & 0x7ff) - 1023; };
+        e = (ex(ma) - ex(mb)) / 2;
+        e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
+      }
+      J.rexp[k] = e;
+      if (sbad && (e != kPSkip || J.variant != kVariantFFT)) *J.flag = 1;
+    }
+    __syncthreads();
+  }
+}
+
+// --------------------------------------------------------- column exponents
+// E_c = the least power of two at or above the 2-norm of balanced column c.
+// Thread = column; block = 128 columns x kColRows inner indices, whose sums of
+// squares and largest exponents go to csum / cmax (k_prod_cexp adds them up in
+// a fixed order; with one block of rows it is done here).  When the sum of
+// squares leaves the FP64 range, the bound from the largest entry serves.
+constexpr int kColRows = 256;
+__device__ __forceinline__ int norm_exp(double sum, int mx, int64_t kc) {
+  if (mx <= kNoExp) return kNoExp;
+  if (sum > 1e-270 && sum < 1e300) {
+    const int q = (int)((__double_as_longlong(sum * (1.0 + 1e-9)) >> 52) & 0x7ff) - 1022;  // sum < 2^q
+    return (q + 1) >> 1;
+  }
+  return mx + 1 + (64 - __clzll((unsigned long long)kc) + 1) / 2;
+}
+template <typename Real>
+__global__ void __launch_bounds__(128) k_prod_cols(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.z >> 1];
+  const int side = blockIdx.z & 1;
+  const int64_t n = side ? J.n_b : J.n_a;
+  const int64_t c = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int64_t k0 = (int64_t)blockIdx.y * kColRows;
+  if (c >= n || k0 >= J.kc) return;
+  const Real* X = reinterpret_cast<const Real*>(side ? J.B : J.A) + c;
+  const int64_t k1 = k0 + kColRows < J.kc ? k0 + kColRows : J.kc;
+  int m = 2 * kNoExp;
+  double sum = 0.0;
+#pragma unroll 8
+  for (int64_t k = k0; k < k1; ++k) {
+    const int e = __ldg(J.rexp + k);
+    const double v = (double)__ldg(X + k * n);
+    if (e != kPSkip && v != 0.0) {
+      const int hi = __double2hiint(v) & 0x7fffffff;
+      m = max(m, max((hi >> 20) - 1023, -1023) + (side ? e : -e));
+      const double w = v * pow2(side ? e : -e);
+      sum = fma(w, w, sum);
+    }
+  }
+  if (J.kc <= kColRows) {
+    (side ? J.cexpB : J.cexpA)[c] = norm_exp(sum, m, J.kc);
+  } else {
+    const size_t at = (size_t)blockIdx.y * (J.n_a + J.n_b) + (side ? J.n_a : 0) + c;
+    J.csum[at] = sum;
+    J.cmax[at] = m;
+  }
+}
+__global__ void __launch_bounds__(128) k_prod_cexp(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  const int64_t n = J.n_a + J.n_b, c = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (c >= n || J.kc <= kColRows) return;
+  const int nb = (int)((J.kc + kColRows - 1) / kColRows);
+  double sum = 0.0;
+  int m = 2 * kNoExp;
+#pragma unroll 4
+  for (int r = 0; r < nb; ++r) {
+    sum += J.csum[(size_t)r * n + c];
+    m = max(m, J.cmax[(size_t)r * n + c]);
+  }
+  (c < J.n_a ? J.cexpA[c] : J.cexpB[c - J.n_a]) = norm_exp(sum, m, J.kc);
+}
+
+// ------------------------------------------------------------ residue planes
+// Planes in the order and layout that the tensor cores read: [modulus][tile of
+// 128 columns][32 inner indices][16 inner indices][column][byte], i.e.
+// no-swizzle K-major core matrices of 8 columns x 16 bytes.  Thread = column:
+// it reads 16 rows (coalesced over the columns) and writes one 16-byte
+// core-matrix row per modulus.  Columns and inner indices are padded with
+// zeros to whole tiles and stages.  The residues of A carry the factor
+// (M / m_i)^-1 mod m_i of the reconstruction.
+//
+// X + 2^58 (2^31) is split into three 20-bit (two 16-bit) parts with fixed
+// residues of their weights; the sum v < 2^30 has the residue v - m floor((v +
+// h) / m) in [-h, m - 1 - h], h = (m - 1) / 2 (128 for m = 256).
+template <typename Real, int SIDE, int I>
+__device__ __forceinline__ int residue(uint32_t x0, uint32_t x1, uint32_t x2) {
+  constexpr int N = Fix<Real>::N, T = Fix<Real>::T, m = modulus(I);
+  constexpr int P = sizeof(Real) == 8 ? 20 : 16;
+  constexpr int f = SIDE == 0 ? crt_inv(I, N) : 1;
+  constexpr int h = m == 256 ? 128 : (m - 1) / 2;
+  constexpr uint32_t c0 = f % m, c1 = powmod2(P, m) * f % m, c2 = powmod2(2 * P, m) * f % m;
+  constexpr uint32_t bias = (uint32_t)((m - powmod2(T, m) * f % m) % m);
+  uint32_t v = x0 * c0 + bias + x1 * c1;
+  if (sizeof(Real) == 8) v += x2 * c2;
+  const uint32_t q = __umulhi(v + h, mod_magic(m)) >> 7;
+  return (int)(v - q * (uint32_t)m);
+}
+template <typename Real, int SIDE, int I>
+__device__ __forceinline__ void plane_store(const uint32_t (&x0)[16], const uint32_t (&x1)[16], const uint32_t (&x2)[16],
+                                            uint8_t* dst, size_t plane) {
+  constexpr int N = Fix<Real>::N;
+  uint32_t w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    int r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = residue<Real, SIDE, I>(x0[4 * q + u], x1[4 * q + u], x2[4 * q + u]);
+    const uint32_t lo = __byte_perm((uint32_t)r[0], (uint32_t)r[1], 0x0040);
+    const uint32_t hi = __byte_perm((uint32_t)r[2], (uint32_t)r[3], 0x0040);
+    w[q] = __byte_perm(lo, hi, 0x5410);
+  }
+  *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+  if constexpr (I + 1 < N) plane_store<Real, SIDE, I + 1>(x0, x1, x2, dst + plane, plane);
+}
+
+template <typename Real, int SIDE>
+__global__ void __launch_bounds__(128) k_prod_slice(const ProdJob* __restrict__ jobs) {
+  constexpr int T = Fix<Real>::T, P = sizeof(Real) == 8 ? 20 : 16;
+  const ProdJob& J = jobs[blockIdx.z];
+  const int64_t n = SIDE ? J.n_b : J.n_a;
+  const int tiles = 2 * (SIDE ? J.tiles_b : J.tiles_a);
+  const int tile = blockIdx.x;
+  if (tile >= tiles) return;
+  const int KS = prod_ksteps(J.kc);
+  const size_t plane = (size_t)tiles * KS * kProdSlab;
+  const int64_t c = (int64_t)tile * kProdTile + threadIdx.x;
+  const Real* X = reinterpret_cast<const Real*>(SIDE ? J.B : J.A) + c;
+  uint8_t* out = (SIDE ? J.slB : J.slA) + (size_t)tile * KS * kProdSlab + threadIdx.x * 16;
+  const int E = c < n ? (SIDE ? J.cexpB : J.cexpA)[c] : kNoExp;
+  const bool live = E > kNoExp;
+  const double g = live ? pow2(T - max(E, kMinExp)) : 0.0;
+  for (int kh = blockIdx.y; kh < 2 * KS; kh += gridDim.y) {  // 16 inner indices
+    const int64_t k0 = (int64_t)kh * 16;
+    Real x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = live && k0 + u < J.kc ? __ldg(X + (k0 + u) * n) : (Real)0;
+    uint32_t x0[16], x1[16], x2[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int e = k0 + u < J.kc ? __ldg(J.rexp + k0 + u) : kPSkip;
+      const double y = e == kPSkip ? 0.0 : (double)x[u] * pow2(SIDE ? e : -e) * g;
+      const unsigned long long w = (unsigned long long)__double2ll_rn(y) + (1ull << T);
+      x0[u] = (uint32_t)w & ((1u << P) - 1u);
+      x1[u] = (uint32_t)(w >> P) & ((1u << P) - 1u);
+      x2[u] = sizeof(Real) == 8 ? (uint32_t)(w >> (2 * P)) : 0u;
+    }
+    plane_store<Real, SIDE, 0>(x0, x1, x2, out + (size_t)(kh >> 1) * kProdSlab + (kh & 1) * (kProdSlab / 2), plane);
+  }
+}
+
+// ------------------------------------------------------- tcgen05 primitives
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// arrives on the barrier at the same offset in CTA 0 of the pair
+__device__ __forceinline__ void bar_arrive_lead(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded wait (about a second of polls); gives up at once when another role
+// of the CTA has given up
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  for (int it = 0; it < 64; ++it)
+    if (bar_test(bar, parity)) return true;
+  for (uint32_t it = 0; it < (1u << 22); ++it) {
+    if (bar_test(bar, parity)) return true;
+    if (*abort) return false;
+    __nanosleep(20);
+  }
+  *abort = 1;
+  return false;
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so
+// far are done
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int u = 0; u < 32; ++u) asm volatile("" : "+r"(r[u]));  // not used before the wait
+}
+
+// shared-memory matrix descriptor: start address >> 4, leading byte offset
+// 2048 (between the two 16-byte K halves), stride byte offset 128 (between
+// 8-row groups), descriptor version 1, no swizzle
+__device__ __forceinline__ uint64_t plane_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(2048 >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) |
+         (1ull << 46);
+}
+// instruction descriptor, kind::i8: D int32 (bits 4-5 = 2), A and B signed
+// (bits 7-9 and 10-12 = 1), both K-major, N = 256 (>> 3 at bit 17), M = 256
+// (>> 4 at bit 24)
+constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+
+// ------------------------------------------------------------- the product
+// One work item = (tile of 256 columns of B x 256 columns of A, modulus),
+// computed by a pair of CTAs with tcgen05.mma.cta_group::2 (M = 256: CTA r
+// holds the rows 128 r .. 128 r + 127 of the tile, columns of B, in its 128
+// TMEM lanes; N = 256: each CTA stages half of the columns of A).  Per 32
+// inner indices and CTA that is 8 KB of operands for 128 cycles of tensor
+// core, half of what single-CTA tiles of 128 x 256 would stage.  TMEM holds
+// two accumulators of 256 columns, so an item's epilogue (int32 -> residue
+// byte) runs behind the next item's MMAs.  Roles in each CTA: warps 0-7 the
+// epilogue, warp 8 the bulk copies of this CTA's half of both operands, warp
+// 9 the MMAs (CTA 0) or the relay (CTA 1: passes "my half of the stage has
+// landed" on to CTA 0).
+constexpr int kStageK = 4;                               // 32-index steps per stage
+constexpr int kStageBytes = 2 * kStageK * kProdSlab;     // 32 KB: both operands of this CTA
+constexpr int kStages = 6;
+constexpr int kProdThreads = 320;
+constexpr int kProdSmem = kStages * kStageBytes + 128;
+
+struct ProdItem {
+  int job, mod, mt, nt;
+};
+// item index -> (job, modulus, tile of B, tile of A); indices ascend, `job` is
+// kept.  The tiles of one modulus come in groups of 8 tiles of A, so that the
+// pairs in flight share their planes through L2.
+__device__ __forceinline__ ProdItem prod_item(const ProdJob* __restrict__ jobs, int64_t idx, int job, int nmod) {
+  while (idx >= jobs[job].item_end) ++job;
+  const int tm = jobs[job].tiles_b, tn = jobs[job].tiles_p;
+  const int64_t tiles = (int64_t)tm * tn;
+  const int64_t e = idx - (jobs[job].item_end - tiles * nmod);
+  ProdItem p;
+  p.job = job;
+  p.mod = (int)(e / tiles);
+  const int64_t w = e - p.mod * tiles;
+  const int gh = 8;
+  const int grp = (int)(w / ((int64_t)gh * tm));
+  const int h = min(gh, tn - grp * gh);
+  const int v = (int)(w - (int64_t)grp * gh * tm);
+  p.mt = v / h;
+  p.nt = grp * gh + v % h;
+  return p;
+}
+
+__device__ __forceinline__ int prod_modulus(int i) {
+  constexpr uint64_t lo = 0xE9EFF1F7FBFDFF00ull, hi = 0x00C5C7D3D9DFE3E5ull;  // modulus(i) mod 256, a byte each
+  const int b = (int)(((i < 8 ? lo : hi) >> (8 * (i & 7))) & 0xff);
+  return b ? b : 256;
+}
+
+// residues of the int32 accumulators (this warp's 32 lanes x 128 columns)
+__device__ __forceinline__ void prod_epilogue(const ProdJob& J, const ProdItem& it, int rank, uint32_t tbase, int warp,
+                                              int lane, int m, uint32_t magic) {
+  const int64_t ldr = (int64_t)J.tiles_b * 256;
+  const int64_t j = (int64_t)it.mt * 256 + 128 * rank + 32 * (warp & 3) + lane;
+  uint32_t* out = J.res + ((int64_t)it.mod * J.tiles_p + it.nt) * 64 * ldr + j;
+  const int up = (0x20000000 + m - 1) / m * m;  // a multiple of m above every |accumulator|
+#pragma unroll 1
+  for (int c0 = (warp >> 2) * 128; c0 < (warp >> 2) * 128 + 128; c0 += 32) {
+    int a[32];
+    tmem_ld32(tbase + ((uint32_t)(32 * (warp & 3)) << 16) + c0, a);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      uint32_t r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t v = (uint32_t)(a[4 * q + u] + up);
+        r[u] = v - (__umulhi(v, magic) >> 7) * (uint32_t)m;
+      }
+      out[(int64_t)(c0 / 4 + q) * ldr] = (r[0] | r[1] << 8) | (r[2] | r[3] << 8) << 16;
+    }
+  }
+}
+
+template <int NMOD>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
+    k_prod_gemm(const ProdJob* __restrict__ jobs, int64_t items, int* __restrict__ timeout) {
+  extern __shared__ __align__(1024) unsigned char psm[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)psm + 127) & ~(uintptr_t)127);
+  __shared__ uint64_t full[kStages], empty[kStages], accfull[2], accempty[2], drain;
+  __shared__ uint32_t tmem_base;
+  __shared__ int s_abort;
+  __shared__ unsigned s_issued;  // stages whose copies were issued
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x & 1;
+  const int64_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    // CTA 0's stage is full when both CTAs' halves are there
+    for (int s = 0; s < kStages; ++s) { bar_init(&full[s], rank == 0 ? 2 : 1); bar_init(&empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { bar_init(&accfull[s], 1); bar_init(&accempty[s], 16); }
+    bar_init(&drain, 1);
+    s_abort = 0;
+    s_issued = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  cluster_sync();
+  fence_after();
+  const uint32_t tbase = tmem_base;
+  volatile int* abort = &s_abort;
+
+  if (warp == 8) {
+    if (lane == 0) {
+      unsigned it = 0;
+      int job = 0;
+      bool ok = true;
+      for (int64_t idx = pair; idx < items && ok; idx += pairs) {
+        const ProdItem p = prod_item(jobs, idx, job, NMOD);
+        job = p.job;
+        const ProdJob& J = jobs[job];
+        const int KS = prod_ksteps(J.kc);
+        const uint8_t* gm = J.slB + ((size_t)p.mod * 2 * J.tiles_b + 2 * p.mt + rank) * KS * kProdSlab;
+        const uint8_t* gn = J.slA + ((size_t)p.mod * 2 * J.tiles_a + 2 * (J.tile0 + p.nt) + rank) * KS * kProdSlab;
+        for (int ks = 0; ks < KS; ks += kStageK, ++it) {
+          const unsigned st = it % kStages;
+          if (!bar_wait(&empty[st], ((it / kStages) & 1u) ^ 1u, abort)) { ok = false; break; }
+          unsigned char* dst = ring + st * kStageBytes;
+          bar_expect(&full[st], kStageBytes);
+          bulk_load(dst, gm + (size_t)ks * kProdSlab, kStageBytes / 2, &full[st]);
+          bulk_load(dst + kStageBytes / 2, gn + (size_t)ks * kProdSlab, kStageBytes / 2, &full[st]);
+        }
+      }
+      s_issued = it;
+    }
+  } else if (warp == 9) {
+    if (lane == 0) {
+      unsigned it = 0, acc = 0;
+      int job = 0;
+      bool ok = true;
+      for (int64_t idx = pair; idx < items && ok; idx += pairs, ++acc) {
+        job = prod_item(jobs, idx, job, NMOD).job;
+        const int KS = prod_ksteps(jobs[job].kc);
+        const unsigned ab = acc & 1u;
+        if (rank == 0) {
+          if (!bar_wait(&accempty[ab], ((acc >> 1) & 1u) ^ 1u, abort)) break;
+          fence_after();
+        }
+        for (int ks = 0; ks < KS; ks += kStageK, ++it) {
+          const unsigned st = it % kStages;
+          if (!bar_wait(&full[st], (it / kStages) & 1u, abort)) { ok = false; break; }
+          if (rank == 1) {
+            bar_arrive_lead(&full[st]);
+            continue;
+          }
+          fence_after();
+          const uint32_t sa = smem_u32(ring + st * kStageBytes);
+          const uint64_t dm = plane_desc(sa), dn = plane_desc(sa + kStageBytes / 2);
+#pragma unroll
+          for (int q = 0; q < kStageK; ++q)
+            mma_i8(tbase + ab * 256u, dm + (uint64_t)(q * (kProdSlab >> 4)), dn + (uint64_t)(q * (kProdSlab >> 4)),
+                   kIdescI8, ks == 0 && q == 0 ? 0u : 1u);
+          mma_commit(&empty[st]);
+        }
+        if (ok && rank == 0) mma_commit(&accfull[ab]);
+      }
+    }
+  } else {
+    unsigned acc = 0;
+    int job = 0;
+    for (int64_t idx = pair; idx < items; idx += pairs, ++acc) {
+      const ProdItem p = prod_item(jobs, idx, job, NMOD);
+      job = p.job;
+      const unsigned ab = acc & 1u;
+      int got = lane == 0 ? (bar_wait(&accfull[ab], (acc >> 1) & 1u, abort) ? 1 : 0) : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) break;
+      bar_test(&accfull[ab], (acc >> 1) & 1u);  // every lane observes the phase before it reads tensor memory
+      fence_after();
+      const int m = prod_modulus(p.mod);
+      prod_epilogue(jobs[job], p, rank, tbase + ab * 256u, warp, lane, m, mod_magic(m));
+      fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive_lead(&accempty[ab]);
+    }
+  }
+  __syncthreads();
+  if (s_abort) {  // a wait ran out: report, and let this CTA's MMAs and copies end before it does
+    if (rank == 0 && warp == 9 && lane == 0) {
+      mma_commit(&drain);
+      for (uint32_t it = 0; it < (1u << 20) && !bar_test(&drain, 0); ++it) __nanosleep(20);
+    }
+    if (tid == 0) {
+      *timeout = 1;
+      __threadfence_system();
+      for (unsigned b = s_issued > kStages ? s_issued - kStages : 0; b < s_issued; ++b)
+        for (uint32_t it = 0; it < (1u << 20) && !bar_test(&full[b % kStages], (b / kStages) & 1u); ++it) __nanosleep(20);
+      int job = 0;
+      for (int64_t idx = pair; idx < items; idx += pairs) {
+        job = prod_item(jobs, idx, job, NMOD).job;
+        *jobs[job].flag = 1;  // the sketch becomes NaN
+      }
+    }
+    __syncthreads();
+  }
+  // the pair ends together: CTA 0's MMAs read CTA 1's shared memory
+  fence_before();
+  cluster_sync();
+  fence_after();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(512u) : "memory");
+}
+
+// ------------------------------------------------------------ reconstruction
+// C[i][j] (+)= the integer with the N residues, in (-M / 2, M / 2), times
+// 2^(E_i + E_j - 2T).  sum r_i (M / m_i) - t M with t = round(sum r_i / m_i)
+// (24-bit fixed point: |entry| <= 2^2T < 0.34 M keeps it away from a tie) is
+// evaluated modulo 2^128 (2^64).  Thread = column j, four rows i at a time.
+template <int N, int I>
+__device__ __forceinline__ void crt_terms(const uint32_t (&w)[16], int sh, unsigned long long (&s)[4], uint32_t& t) {
+  constexpr U128 P = mod_product(N, I);
+  const uint32_t r = (w[I] >> sh) & 0xffu;
+  t += r * (uint32_t)((16777216 + modulus(I) / 2) / modulus(I));
+  s[0] += (unsigned long long)r * (uint32_t)P.lo;
+  s[1] += (unsigned long long)r * (uint32_t)(P.lo >> 32);
+  if (N > 8) {
+    s[2] += (unsigned long long)r * (uint32_t)P.hi;
+    s[3] += (unsigned long long)r * (uint32_t)(P.hi >> 32);
+  }
+  if constexpr (I + 1 < N) crt_terms<N, I + 1>(w, sh, s, t);
+}
+template <typename Real>
+__global__ void __launch_bounds__(256) k_prod_crt(const ProdJob* __restrict__ jobs) {
+  constexpr int N = Fix<Real>::N, T = Fix<Real>::T;
+  constexpr U128 M = mod_product(N, -1);
+  const ProdJob& J = jobs[blockIdx.z];
+  const int64_t ldr = (int64_t)J.tiles_b * 256, quads = (int64_t)J.tiles_p * 64;
+  const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (j >= J.n_b) return;
+  const int eB = max(__ldg(J.cexpB + j), kMinExp) - 2 * T;
+  for (int64_t r = blockIdx.y; r < quads; r += gridDim.y) {
+    const int64_t i = (int64_t)J.tile0 * 256 + r * 4;
+    if (i >= J.n_a) break;
+    uint32_t w[16];
+#pragma unroll
+    for (int q = 0; q < N; ++q) w[q] = __ldcs(J.res + ((int64_t)q * quads + r) * ldr + j);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i + u >= J.n_a) break;
+      unsigned long long s[4] = {0, 0, 0, 0};
+      uint32_t t = 1u << 23;
+      crt_terms<N, 0>(w, 8 * u, s, t);
+      t >>= 24;
+      double v;
+      if (N > 8) {
+        unsigned __int128 x = (unsigned __int128)s[0] + ((unsigned __int128)s[1] << 32) + ((unsigned __int128)s[2] << 64) +
+                              ((unsigned __int128)s[3] << 96);
+        x -= (((unsigned __int128)M.hi << 64) | M.lo) * t;
+        const bool neg = (__int128)x < 0;
+        if (neg) x = -x;
+        v = fma((double)(unsigned long long)(x >> 64), 18446744073709551616.0, (double)(unsigned long long)x);
+        if (neg) v = -v;
+      } else {
+        v = (double)(long long)(s[0] + (s[1] << 32) - M.lo * t);
+      }
+      const int e = min(max(__ldg(J.cexpA + i + u), kMinExp) + eB, 2046), h = e >> 1;
+      v = v * pow2(h) * pow2(e - h);
+      double* C = J.C + (i + u) * J.ldc + j;
+      *C = J.accumulate ? *C + v : v;
+    }
+  }
+}
+
+// ------------------------------------------------------------ sorted buckets
+// Per repetition t: the columns j of B sorted by their bucket h2 (ties by j),
+// as 8-byte entries {j | (s2 < 0) << 31, h2}, and cum[h] = entries below
+// bucket h.  One CTA per (t, job).  Counting sort with L2 atomics; each
+// bucket's entries are then put in ascending j, so the order of the sums
+// does not depend on the atomics.
+constexpr int kIdxThreads = 1024;
+__global__ void __launch_bounds__(kIdxThreads) k_prod_index(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  const int t = blockIdx.x;
+  if (t >= J.d) return;
+  if (t == 0 && threadIdx.x == 0) *J.flag = 0;
+  const uint32_t b = 1u << J.log2b;
+  const uint32_t n = (uint32_t)J.n_b;
+  uint32_t* cum = J.cum + (size_t)t * (b + 1);
+  uint2* ent = J.ent + (size_t)t * n;
+  const uint32_t* codes = J.codesB + (size_t)t * n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t ws[32];
+  __shared__ uint32_t s_carry;
+  for (uint32_t e = tid; e <= b; e += kIdxThreads) __stcg(cum + e, 0u);
+  if (tid == 0) s_carry = 0;
+  __syncthreads();
+  for (uint32_t j = tid; j < n; j += kIdxThreads) atomicAdd(cum + 1 + (codes[j] & (b - 1)), 1u);
+  __syncthreads();
+  // exclusive scan of the counts: cum[h + 1] = start of bucket h
+  for (uint32_t base = 1; base <= b; base += kIdxThreads * 4) {
+    uint32_t v[4], sum = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t e = base + tid * 4 + u;
+      v[u] = e <= b ? __ldcg(cum + e) : 0u;
+      sum += v[u];
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t w = ws[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += x;
+      }
+      ws[lane] = w;
+    }
+    __syncthreads();
+    uint32_t run = s_carry + (warp ? ws[warp - 1] : 0u) + inc - sum;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t e = base + tid * 4 + u;
+      if (e <= b) __stcg(cum + e, run);
+      run += v[u];
+    }
+    __syncthreads();
+    if (tid == 0) s_carry += ws[31];
+    __syncthreads();
+  }
+  // placement moves cum[h + 1] from the start of bucket h to its end
+  for (uint32_t j = tid; j < n; j += kIdxThreads) {
+    const uint32_t c = codes[j], h = c & (b - 1);
+    const uint32_t pos = atomicAdd(cum + 1 + h, 1u);
+    __stcg(ent + pos, make_uint2(j | ((~c) & 0x80000000u), h));
+  }
+  __syncthreads();
+  for (uint32_t h = tid; h < b; h += kIdxThreads) {
+    const uint32_t beg = __ldcg(cum + h), end = __ldcg(cum + h + 1);
+    for (uint32_t e = beg + 1; e < end; ++e) {  // insertion sort by j
+      const uint2 x = __ldcg(ent + e);
+      uint32_t f = e;
+      while (f > beg) {
+        const uint2 y = __ldcg(ent + f - 1);
+        if ((y.x & 0x7fffffffu) <= (x.x & 0x7fffffffu)) break;
+        __stcg(ent + f, y);
+        --f;
+      }
+      if (f != e) __stcg(ent + f, x);
+    }
+  }
+}
+
+// -------------------------------------------------------------- the sketches
+// A warp owns a window of W consecutive buckets of p_t (in shared memory) and
+// walks the rows i of C in order.  For row i the columns that fall into the
+// window are consecutive in the sorted list (FFT: h2 in [m0 - h1(i), + W) mod
+// b; FWHT: the aligned block (m0 ^ h1(i)) / W), so the warp reads the entries
+// coalesced, gathers their C[i][j] and adds them: equal buckets sit on
+// neighbouring lanes and are added one rank after the other, so there are
+// no atomics and the order of every sum is fixed.  Rows are split into G
+// groups with partial sketches.  blockIdx.z = job * Gmax + group.
+constexpr int kScWarps = 8;
+template <int VARIANT>
+__global__ void __launch_bounds__(kScWarps * 32) k_prod_scatter(const ProdJob* __restrict__ jobs, int gmax) {
+  extern __shared__ double sacc[];
+  const ProdJob& J = jobs[blockIdx.z / gmax];
+  const int g = blockIdx.z % gmax, t = blockIdx.y;
+  if (J.variant != VARIANT || J.dense || g >= J.G || t >= J.d) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t b = 1u << J.log2b, mask = b - 1u, W = 1u << J.logW;
+  const uint32_t win = blockIdx.x * kScWarps + warp;
+  if ((win << J.logW) >= b) return;
+  const uint32_t m0 = win << J.logW;
+  double* acc = sacc + (size_t)warp * W;
+  double* out = J.part + ((size_t)g * J.d + t) * b + m0;
+  for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
+  __syncwarp();
+  const uint32_t n_b = (uint32_t)J.n_b;
+  const uint32_t* cum = J.cum + (size_t)t * (b + 1);
+  const uint2* ent = J.ent + (size_t)t * n_b;
+  const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
+  const int64_t per = (J.n_a + J.G - 1) / J.G;
+  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
+  for (int64_t r0 = ib; r0 < ie; r0 += 32) {
+    // lane l looks row r0 + l up
+    uint32_t e0 = 0, cnt = 0, key = 0, c1 = 0;
+    if (r0 + lane < ie) {
+      c1 = __ldg(cA + r0 + lane);
+      const uint32_t h1 = c1 & mask;
+      const uint32_t s = VARIANT == kVariantFFT ? ((m0 - h1) & mask) : ((m0 ^ h1) & ~(W - 1u));
+      key = VARIANT == kVariantFFT ? s : h1;
+      e0 = __ldg(cum + s);
+      const uint32_t se = s + W;
+      cnt = se <= b ? __ldg(cum + se) - e0 : n_b - e0 + __ldg(cum + se - b);
+    }
+    const uint32_t neg1 = ~c1 & 0x80000000u;
+    const int rows = (int)min((int64_t)32, ie - r0);
+    for (int r = 0; r < rows; r += 2) {
+      // two rows and two batches of 32 entries each in flight
+      uint32_t cr[2], er[2], kr[2], sr[2];
+      double v[2][2];
+      uint32_t m[2][2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int src = (r + q) & 31;
+        cr[q] = __shfl_sync(0xffffffffu, cnt, src);
+        er[q] = __shfl_sync(0xffffffffu, e0, src);
+        kr[q] = __shfl_sync(0xffffffffu, key, src);
+        sr[q] = __shfl_sync(0xffffffffu, neg1, src);
+        if (r + q >= rows) cr[q] = 0;
+      }
+      auto fetch = [&](int q, uint32_t base, double& val, uint32_t& mm) {
+        val = 0.0;
+        mm = 0xffffffffu;
+        if (base + lane < cr[q]) {
+          uint32_t x = er[q] + base + lane;
+          if (x >= n_b) x -= n_b;
+          const uint2 e = __ldg(ent + x);
+          const long long bits = __double_as_longlong(__ldg(J.C + (r0 + r + q) * J.ldc + (e.x & 0x7fffffffu)));
+          val = __longlong_as_double(bits ^ ((long long)((e.x & 0x80000000u) ^ sr[q]) << 32));
+          mm = VARIANT == kVariantFFT ? ((e.y - kr[q]) & mask) : ((e.y ^ kr[q]) & (W - 1u));
+        }
+      };
+      auto commit = [&](double val, uint32_t mm) {
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, mm, 1);
+        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || prev != mm);
+        const int rank = lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
+        const bool ok = mm != 0xffffffffu;
+        uint32_t todo = __ballot_sync(0xffffffffu, ok);
+        for (int k = 0; todo; ++k) {
+          const bool now = ok && rank == k;
+          if (now) acc[mm] += val;
+          todo &= ~__ballot_sync(0xffffffffu, now);
+          __syncwarp();
+        }
+      };
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        fetch(q, 0, v[q][0], m[q][0]);
+        fetch(q, 32, v[q][1], m[q][1]);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        commit(v[q][0], m[q][0]);
+        if (cr[q] > 32) commit(v[q][1], m[q][1]);
+        for (uint32_t base = 64; base < cr[q]; base += 32) {
+          double vv;
+          uint32_t mm;
+          fetch(q, base, vv, mm);
+          commit(vv, mm);
+        }
+      }
+    }
+  }
+  for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
+}
+
+// The same for buckets that take several columns each (n_b > 2 b): lane =
+// bucket, its sum in a register; for row i it adds the run of entries of
+// h2 = m - h1(i) (FWHT: m ^ h1(i)).
+template <int VARIANT>
+__global__ void __launch_bounds__(256) k_prod_scatter_dense(const ProdJob* __restrict__ jobs, int gmax) {
+  const ProdJob& J = jobs[blockIdx.z / gmax];
+  const int g = blockIdx.z % gmax, t = blockIdx.y;
+  if (J.variant != VARIANT || !J.dense || g >= J.G || t >= J.d) return;
+  const uint32_t b = 1u << J.log2b, mask = b - 1u;
+  const uint32_t m = blockIdx.x * 256 + threadIdx.x;
+  if (m >= b) return;
+  const uint32_t n_b = (uint32_t)J.n_b;
+  const uint32_t* cum = J.cum + (size_t)t * (b + 1);
+  const uint2* ent = J.ent + (size_t)t * n_b;
+  const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
+  double* out = J.part + ((size_t)g * J.d + t) * b + m;
+  double acc = 0.0;
+  const int64_t per = (J.n_a + J.G - 1) / J.G;
+  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
+#pragma unroll 2
+  for (int64_t i = ib; i < ie; ++i) {
+    const uint32_t c1 = __ldg(cA + i);
+    const uint32_t h1 = c1 & mask;
+    const uint32_t h2 = VARIANT == kVariantFFT ? ((m - h1) & mask) : (m ^ h1);
+    const uint32_t beg = __ldg(cum + h2), end = __ldg(cum + h2 + 1);
+    const double* row = J.C + i * J.ldc;
+    double s = 0.0;
+    for (uint32_t e = beg; e < end; ++e) {
+      const uint32_t x = __ldg(&ent[e].x);
+      const long long bits = __double_as_longlong(__ldg(row + (x & 0x7fffffffu)));
+      s += __longlong_as_double(bits ^ ((long long)(x & 0x80000000u) << 32));
+    }
+    acc += c1 >> 31 ? s : -s;
+  }
+  *out = acc;
+}
+
+// p = sum of the row groups' partial sketches (NaN when the flag is set)
+__global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  const int64_t db = (int64_t)J.d << J.log2b;
+  const bool bad = *J.flag == 1;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < db; e += (int64_t)gridDim.x * 256) {
+    double s = 0.0;
+    for (int g = 0; g < J.G; ++g) s += J.part[(size_t)g * db + e];
+    J.p[e] = bad ? __longlong_as_double(0x7ff8000000000000ll) : s;
+  }
+}
+
+// host-mapped flag set by a wait of the product kernel that ran out
+int* product_timeout_flag(int** dev) {
+  static int* host = nullptr;
+  static int* mapped = nullptr;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> g(mu);
+  if (!host) {
+    int* h = nullptr;
+    CMM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h), sizeof(int), cudaHostAllocMapped));
+    *h = 0;
+    CMM_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), h, 0));
+    host = h;
+  }
+  if (dev) *dev = mapped;
+  return host;
+}
+
+template <int NMOD>
+void launch_gemm(const ProdJob* dJobs, int64_t items, cudaStream_t s) {
+  int* flag = nullptr;
+  product_timeout_flag(&flag);
+  CMM_CUDA(cudaFuncSetAttribute(k_prod_gemm<NMOD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProdSmem));
+  const int grid = 2 * (int)std::min<int64_t>(items, num_sms() / 2);
+  count_launch();
+  k_prod_gemm<NMOD><<<grid, kProdThreads, kProdSmem, s>>>(dJobs, items, flag);
+  CMM_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+// Window: about 32 to 64 entries of a row per warp step, at most 1024 buckets
+// (8 KB of shared memory a warp); row groups so that some 24 warps per SM run.
+void plan_product_sketch(ProdJob& J, int sms) {
+  const int64_t b = (int64_t)1 << J.log2b;
+  J.dense = J.n_b > 2 * b ? 1 : 0;
+  J.logW = 6;
+  while (J.logW < 10 && ((int64_t)2 << J.logW) * std::max<int64_t>(J.n_b, 1) <= 60 * b) ++J.logW;
+  J.logW = std::min(J.logW, J.log2b);
+  const int64_t warps = J.dense ? (J.d * b + 31) / 32 : J.d * (b >> J.logW);
+  const int64_t G = (int64_t)sms * 24 / std::max<int64_t>(warps, 1);
+  J.G = (int)std::max<int64_t>(1, std::min<int64_t>({G, (J.n_a + 31) / 32, 64}));
+}
+
+bool product_timed_out() {
+  volatile int* h = product_timeout_flag(nullptr);
+  const bool t = *h != 0;
+  *h = 0;
+  return t;
+}
+
+void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s) {
+  if (count <= 0) return;
+  int64_t kc = 0, n = 0, nn = 0;
+  int ta = 0, tb = 0;
+  for (int i = 0; i < count; ++i) {
+    const ProdJob& J = hJobs[i];
+    kc = std::max(kc, J.kc);
+    n = std::max(n, std::max(J.n_a, J.n_b));
+    nn = std::max(nn, J.n_a + J.n_b);
+    ta = std::max(ta, J.tiles_a);
+    tb = std::max(tb, J.tiles_b);
+  }
+  {
+    ProfScope prof("scale", s);
+    const dim3 gr((unsigned)std::min<int64_t>(kc, 4096), (unsigned)count);
+    const dim3 gc((unsigned)((n + 127) / 128), (unsigned)((kc + kColRows - 1) / kColRows), (unsigned)(2 * count));
+    count_launch(kc > kColRows ? 3 : 2);
+    if (f32) {
+      k_prod_rows<float><<<gr, 256, 0, s>>>(dJobs);
+      k_prod_cols<float><<<gc, 128, 0, s>>>(dJobs);
+    } else {
+      k_prod_rows<double><<<gr, 256, 0, s>>>(dJobs);
+      k_prod_cols<double><<<gc, 128, 0, s>>>(dJobs);
+    }
+    if (kc > kColRows) k_prod_cexp<<<dim3((unsigned)((nn + 127) / 128), (unsigned)count), 128, 0, s>>>(dJobs);
+    CMM_CUDA(cudaGetLastError());
+  }
+  ProfScope prof("materialize", s);
+  count_launch(2);
+  const unsigned ky = (unsigned)std::min(2 * prod_ksteps(kc), 64);
+  const dim3 ga((unsigned)(2 * ta), ky, (unsigned)count), gb((unsigned)(2 * tb), ky, (unsigned)count);
+  if (f32) {
+    k_prod_slice<float, 0><<<ga, 128, 0, s>>>(dJobs);
+    k_prod_slice<float, 1><<<gb, 128, 0, s>>>(dJobs);
+  } else {
+    k_prod_slice<double, 0><<<ga, 128, 0, s>>>(dJobs);
+    k_prod_slice<double, 1><<<gb, 128, 0, s>>>(dJobs);
+  }
+  CMM_CUDA(cudaGetLastError());
+}
+
+void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s) {
+  if (count <= 0) return;
+  ProfScope prof("sketch", s);
+  if (f32) launch_gemm<Fix<float>::N>(dJobs, hJobs[count - 1].item_end, s);
+  else launch_gemm<Fix<double>::N>(dJobs, hJobs[count - 1].item_end, s);
+  int64_t n_b = 0, rows = 0;
+  for (int i = 0; i < count; ++i) {
+    n_b = std::max(n_b, hJobs[i].n_b);
+    rows = std::max<int64_t>(rows, (int64_t)hJobs[i].tiles_p * 64);
+  }
+  count_launch();
+  const dim3 g((unsigned)((n_b + 255) / 256), (unsigned)std::min<int64_t>(rows, 4096), (unsigned)count);
+  if (f32) k_prod_crt<float><<<g, 256, 0, s>>>(dJobs);
+  else k_prod_crt<double><<<g, 256, 0, s>>>(dJobs);
+  CMM_CUDA(cudaGetLastError());
+}
+
+void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  if (count <= 0) return;
+  int d = 0;
+  for (int i = 0; i < count; ++i) d = std::max(d, hJobs[i].d);
+  ProfScope prof("plan", s);
+  count_launch();
+  k_prod_index<<<dim3((unsigned)d, (unsigned)count), kIdxThreads, 0, s>>>(dJobs);
+  CMM_CUDA(cudaGetLastError());
+}
+
+void launch_product_scatter(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  if (count <= 0) return;
+  int gmax[2][2] = {}, dmax[2][2] = {};
+  int64_t wmax[2][2] = {};
+  size_t smem[2] = {};
+  for (int i = 0; i < count; ++i) {
+    const ProdJob& J = hJobs[i];
+    const int v = J.variant, dn = J.dense ? 1 : 0;
+    gmax[v][dn] = std::max(gmax[v][dn], J.G);
+    dmax[v][dn] = std::max(dmax[v][dn], J.d);
+    const int64_t b = (int64_t)1 << J.log2b;
+    const int64_t x = dn ? (b + 255) / 256 : ((b >> J.logW) + kScWarps - 1) / kScWarps;
+    wmax[v][dn] = std::max(wmax[v][dn], x);
+    if (!dn) smem[v] = std::max(smem[v], ((size_t)kScWarps << J.logW) * 8);
+  }
+  ProfScope prof("finalize", s);
+#define CMM_SCATTER(V)                                                                                              \
+  do {                                                                                                              \
+    if (gmax[V][0]) {                                                                                               \
+      CMM_CUDA(cudaFuncSetAttribute(k_prod_scatter<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[V])); \
+      count_launch();                                                                                               \
+      k_prod_scatter<V><<<dim3((unsigned)wmax[V][0], (unsigned)dmax[V][0], (unsigned)(gmax[V][0] * count)),         \
+                          kScWarps * 32, smem[V], s>>>(dJobs, gmax[V][0]);                                          \
+      CMM_CUDA(cudaGetLastError());                                                                                 \
+    }                                                                                                               \
+    if (gmax[V][1]) {                                                                                               \
+      count_launch();                                                                                               \
+      k_prod_scatter_dense<V><<<dim3((unsigned)wmax[V][1], (unsigned)dmax[V][1], (unsigned)(gmax[V][1] * count)),   \
+                                256, 0, s>>>(dJobs, gmax[V][1]);                                                    \
+      CMM_CUDA(cudaGetLastError());                                                                                 \
+    }                                                                                                               \
+  } while (0)
+  CMM_SCATTER(0);
+  CMM_SCATTER(1);
+#undef CMM_SCATTER
+}
+
+void launch_product_reduce(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  if (count <= 0) return;
+  int64_t db = 0;
+  for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
+  ProfScope prof("finalize", s);
+  count_launch();
+  k_prod_reduce<<<dim3((unsigned)std::min<int64_t>((db + 255) / 256, 2048), (unsigned)count), 256, 0, s>>>(dJobs);
+  CMM_CUDA(cudaGetLastError());
+}
+
+}  // namespace cmm
