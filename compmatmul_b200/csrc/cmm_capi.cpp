@@ -338,6 +338,7 @@ static bool product_applicable(int variant, bool f32, const SketchParams& sp, in
                                int64_t n_b) {
   if (n_inner <= 0 || n_a <= 0 || n_b <= 0) return false;
   if (n_a > 0x7fffffff || n_b > 0x7fffffff || n_a * n_b > kProdMaxEntries) return false;
+  if (sp.b < 512 || (sp.b > 65536 && n_b > 131072)) return false;  // the forms of the additions (cmm_product_add.cu)
   if (sketch_kernel_choice() == 3) return true;
   if (sketch_kernel_choice() != 0) return false;
   const double nn = (double)n_a * (double)n_b, k = (double)n_inner, d = sp.d, b = sp.b;
@@ -385,8 +386,10 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   const size_t o_slA = take(prod_plane_bytes(n_a, kc, f32)), o_slB = take(prod_plane_bytes(n_b, kc, f32));
   const size_t o_res = take(per_tile * panel), o_exp = take((size_t)(n_a + n_b + kc + 1) * 4);
   const size_t o_csum = take(nb * (size_t)(n_a + n_b) * 8), o_cmax = take(nb * (size_t)(n_a + n_b) * 4);
-  const size_t o_C = take(scratch ? 0 : (size_t)n_a * (size_t)n_b * 8);
-  const size_t o_cum = take((size_t)sp.d * ((size_t)sp.b + 1) * 4), o_ent = take((size_t)sp.d * (size_t)n_b * 8);
+  J.ldc = prod_ldc(n_b);
+  if (J.ldc != n_b || reinterpret_cast<uintptr_t>(scratch) % 16) scratch = nullptr;  // rows must be 16-byte aligned
+  const size_t o_C = take(scratch ? 0 : (size_t)n_a * (size_t)J.ldc * 8);
+  const size_t o_cum = take(prod_cum_bytes(J)), o_ent = take(2 * (size_t)sp.d * (size_t)n_b * 4);
   const size_t o_part = take((size_t)J.G * db * 8), o_job = take(sizeof(ProdJob));
   DevBuf mem(total, s);
   uint8_t* base = mem.as<uint8_t>();
@@ -400,9 +403,8 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   J.csum = reinterpret_cast<double*>(base + o_csum);
   J.cmax = reinterpret_cast<int*>(base + o_cmax);
   J.C = scratch ? scratch : reinterpret_cast<double*>(base + o_C);
-  J.ldc = n_b;
-  J.cum = reinterpret_cast<uint32_t*>(base + o_cum);
-  J.ent = reinterpret_cast<uint2*>(base + o_ent);
+  J.cum = base + o_cum;
+  J.ent = reinterpret_cast<uint32_t*>(base + o_ent);
   J.part = reinterpret_cast<double*>(base + o_part);
   J.p = dP;
   ProdJob* dJ = reinterpret_cast<ProdJob*>(base + o_job);
@@ -424,8 +426,7 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
       launch_product_gemm(&J, dJ, 1, f32, s);
     }
   }
-  launch_product_scatter(&J, dJ, 1, s);
-  launch_product_reduce(&J, dJ, 1, s);
+  launch_product_add(&J, dJ, 1, s);
 }
 
 // feed != nullptr: the rows of dAT / dB are still arriving from the host;

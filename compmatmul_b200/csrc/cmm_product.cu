@@ -31,11 +31,11 @@
 
 #include "cmm_internal.h"
 #include "cmm_product.h"
+#include "cmm_product_dev.cuh"
 
 namespace cmm {
 namespace {
 
-constexpr int kPSkip = -0x7fffffff;  // row pair with a zero row: contributes nothing
 constexpr int kNoExp = -1000000;     // column without a nonzero entry
 constexpr int kMinExp = -960;        // smaller columns are scaled as if they were this large
 
@@ -87,8 +87,6 @@ template <>
 struct Fix<float> {
   static constexpr int N = 8, T = 31;
 };
-
-__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
 
 // ------------------------------------------------------------- row balance
 // e_k = (expo(max |A row|) - expo(max |B row|)) / 2, within the range of pow2; kPSkip
@@ -282,13 +280,6 @@ __global__ void __launch_bounds__(128) k_prod_slice(const ProdJob* __restrict__ 
 }
 
 // ------------------------------------------------------- tcgen05 primitives
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // arrives on the barrier at the same offset in CTA 0 of the pair
 __device__ __forceinline__ void bar_arrive_lead(uint64_t* bar) {
   asm volatile(
@@ -296,36 +287,6 @@ __device__ __forceinline__ void bar_arrive_lead(uint64_t* bar) {
       "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
       : "memory");
-}
-__device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P1;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, P1;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait (about a second of polls); gives up at once when another role
-// of the CTA has given up
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  for (int it = 0; it < 64; ++it)
-    if (bar_test(bar, parity)) return true;
-  for (uint32_t it = 0; it < (1u << 22); ++it) {
-    if (bar_test(bar, parity)) return true;
-    if (*abort) return false;
-    __nanosleep(20);
-  }
-  *abort = 1;
-  return false;
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
 }
 __device__ __forceinline__ void mma_i8(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -641,247 +602,9 @@ __global__ void __launch_bounds__(256) k_prod_crt(const ProdJob* __restrict__ jo
   }
 }
 
-// ------------------------------------------------------------ sorted buckets
-// Per repetition t: the columns j of B sorted by their bucket h2 (ties by j),
-// as 8-byte entries {j | (s2 < 0) << 31, h2}, and cum[h] = entries below
-// bucket h.  One CTA per (t, job).  Counting sort with L2 atomics; each
-// bucket's entries are then put in ascending j, so the order of the sums
-// does not depend on the atomics.
-constexpr int kIdxThreads = 1024;
-__global__ void __launch_bounds__(kIdxThreads) k_prod_index(const ProdJob* __restrict__ jobs) {
-  const ProdJob& J = jobs[blockIdx.y];
-  const int t = blockIdx.x;
-  if (t >= J.d) return;
-  if (t == 0 && threadIdx.x == 0) *J.flag = 0;
-  const uint32_t b = 1u << J.log2b;
-  const uint32_t n = (uint32_t)J.n_b;
-  uint32_t* cum = J.cum + (size_t)t * (b + 1);
-  uint2* ent = J.ent + (size_t)t * n;
-  const uint32_t* codes = J.codesB + (size_t)t * n;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ uint32_t ws[32];
-  __shared__ uint32_t s_carry;
-  for (uint32_t e = tid; e <= b; e += kIdxThreads) __stcg(cum + e, 0u);
-  if (tid == 0) s_carry = 0;
-  __syncthreads();
-  for (uint32_t j = tid; j < n; j += kIdxThreads) atomicAdd(cum + 1 + (codes[j] & (b - 1)), 1u);
-  __syncthreads();
-  // exclusive scan of the counts: cum[h + 1] = start of bucket h
-  for (uint32_t base = 1; base <= b; base += kIdxThreads * 4) {
-    uint32_t v[4], sum = 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t e = base + tid * 4 + u;
-      v[u] = e <= b ? __ldcg(cum + e) : 0u;
-      sum += v[u];
-    }
-    uint32_t inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += x;
-    }
-    if (lane == 31) ws[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t w = ws[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += x;
-      }
-      ws[lane] = w;
-    }
-    __syncthreads();
-    uint32_t run = s_carry + (warp ? ws[warp - 1] : 0u) + inc - sum;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t e = base + tid * 4 + u;
-      if (e <= b) __stcg(cum + e, run);
-      run += v[u];
-    }
-    __syncthreads();
-    if (tid == 0) s_carry += ws[31];
-    __syncthreads();
-  }
-  // placement moves cum[h + 1] from the start of bucket h to its end
-  for (uint32_t j = tid; j < n; j += kIdxThreads) {
-    const uint32_t c = codes[j], h = c & (b - 1);
-    const uint32_t pos = atomicAdd(cum + 1 + h, 1u);
-    __stcg(ent + pos, make_uint2(j | ((~c) & 0x80000000u), h));
-  }
-  __syncthreads();
-  for (uint32_t h = tid; h < b; h += kIdxThreads) {
-    const uint32_t beg = __ldcg(cum + h), end = __ldcg(cum + h + 1);
-    for (uint32_t e = beg + 1; e < end; ++e) {  // insertion sort by j
-      const uint2 x = __ldcg(ent + e);
-      uint32_t f = e;
-      while (f > beg) {
-        const uint2 y = __ldcg(ent + f - 1);
-        if ((y.x & 0x7fffffffu) <= (x.x & 0x7fffffffu)) break;
-        __stcg(ent + f, y);
-        --f;
-      }
-      if (f != e) __stcg(ent + f, x);
-    }
-  }
-}
-
-// -------------------------------------------------------------- the sketches
-// A warp owns a window of W consecutive buckets of p_t (in shared memory) and
-// walks the rows i of C in order.  For row i the columns that fall into the
-// window are consecutive in the sorted list (FFT: h2 in [m0 - h1(i), + W) mod
-// b; FWHT: the aligned block (m0 ^ h1(i)) / W), so the warp reads the entries
-// coalesced, gathers their C[i][j] and adds them: equal buckets sit on
-// neighbouring lanes and are added one rank after the other, so there are
-// no atomics and the order of every sum is fixed.  Rows are split into G
-// groups with partial sketches.  blockIdx.z = job * Gmax + group.
-constexpr int kScWarps = 8;
-template <int VARIANT>
-__global__ void __launch_bounds__(kScWarps * 32) k_prod_scatter(const ProdJob* __restrict__ jobs, int gmax) {
-  extern __shared__ double sacc[];
-  const ProdJob& J = jobs[blockIdx.z / gmax];
-  const int g = blockIdx.z % gmax, t = blockIdx.y;
-  if (J.variant != VARIANT || J.dense || g >= J.G || t >= J.d) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t b = 1u << J.log2b, mask = b - 1u, W = 1u << J.logW;
-  const uint32_t win = blockIdx.x * kScWarps + warp;
-  if ((win << J.logW) >= b) return;
-  const uint32_t m0 = win << J.logW;
-  double* acc = sacc + (size_t)warp * W;
-  double* out = J.part + ((size_t)g * J.d + t) * b + m0;
-  for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
-  __syncwarp();
-  const uint32_t n_b = (uint32_t)J.n_b;
-  const uint32_t* cum = J.cum + (size_t)t * (b + 1);
-  const uint2* ent = J.ent + (size_t)t * n_b;
-  const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
-  const int64_t per = (J.n_a + J.G - 1) / J.G;
-  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
-  for (int64_t r0 = ib; r0 < ie; r0 += 32) {
-    // lane l looks row r0 + l up
-    uint32_t e0 = 0, cnt = 0, key = 0, c1 = 0;
-    if (r0 + lane < ie) {
-      c1 = __ldg(cA + r0 + lane);
-      const uint32_t h1 = c1 & mask;
-      const uint32_t s = VARIANT == kVariantFFT ? ((m0 - h1) & mask) : ((m0 ^ h1) & ~(W - 1u));
-      key = VARIANT == kVariantFFT ? s : h1;
-      e0 = __ldg(cum + s);
-      const uint32_t se = s + W;
-      cnt = se <= b ? __ldg(cum + se) - e0 : n_b - e0 + __ldg(cum + se - b);
-    }
-    const uint32_t neg1 = ~c1 & 0x80000000u;
-    const int rows = (int)min((int64_t)32, ie - r0);
-    for (int r = 0; r < rows; r += 2) {
-      // two rows and two batches of 32 entries each in flight
-      uint32_t cr[2], er[2], kr[2], sr[2];
-      double v[2][2];
-      uint32_t m[2][2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int src = (r + q) & 31;
-        cr[q] = __shfl_sync(0xffffffffu, cnt, src);
-        er[q] = __shfl_sync(0xffffffffu, e0, src);
-        kr[q] = __shfl_sync(0xffffffffu, key, src);
-        sr[q] = __shfl_sync(0xffffffffu, neg1, src);
-        if (r + q >= rows) cr[q] = 0;
-      }
-      auto fetch = [&](int q, uint32_t base, double& val, uint32_t& mm) {
-        val = 0.0;
-        mm = 0xffffffffu;
-        if (base + lane < cr[q]) {
-          uint32_t x = er[q] + base + lane;
-          if (x >= n_b) x -= n_b;
-          const uint2 e = __ldg(ent + x);
-          const long long bits = __double_as_longlong(__ldg(J.C + (r0 + r + q) * J.ldc + (e.x & 0x7fffffffu)));
-          val = __longlong_as_double(bits ^ ((long long)((e.x & 0x80000000u) ^ sr[q]) << 32));
-          mm = VARIANT == kVariantFFT ? ((e.y - kr[q]) & mask) : ((e.y ^ kr[q]) & (W - 1u));
-        }
-      };
-      auto commit = [&](double val, uint32_t mm) {
-        const uint32_t prev = __shfl_up_sync(0xffffffffu, mm, 1);
-        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || prev != mm);
-        const int rank = lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
-        const bool ok = mm != 0xffffffffu;
-        uint32_t todo = __ballot_sync(0xffffffffu, ok);
-        for (int k = 0; todo; ++k) {
-          const bool now = ok && rank == k;
-          if (now) acc[mm] += val;
-          todo &= ~__ballot_sync(0xffffffffu, now);
-          __syncwarp();
-        }
-      };
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        fetch(q, 0, v[q][0], m[q][0]);
-        fetch(q, 32, v[q][1], m[q][1]);
-      }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        commit(v[q][0], m[q][0]);
-        if (cr[q] > 32) commit(v[q][1], m[q][1]);
-        for (uint32_t base = 64; base < cr[q]; base += 32) {
-          double vv;
-          uint32_t mm;
-          fetch(q, base, vv, mm);
-          commit(vv, mm);
-        }
-      }
-    }
-  }
-  for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
-}
-
-// The same for buckets that take several columns each (n_b > 2 b): lane =
-// bucket, its sum in a register; for row i it adds the run of entries of
-// h2 = m - h1(i) (FWHT: m ^ h1(i)).
-template <int VARIANT>
-__global__ void __launch_bounds__(256) k_prod_scatter_dense(const ProdJob* __restrict__ jobs, int gmax) {
-  const ProdJob& J = jobs[blockIdx.z / gmax];
-  const int g = blockIdx.z % gmax, t = blockIdx.y;
-  if (J.variant != VARIANT || !J.dense || g >= J.G || t >= J.d) return;
-  const uint32_t b = 1u << J.log2b, mask = b - 1u;
-  const uint32_t m = blockIdx.x * 256 + threadIdx.x;
-  if (m >= b) return;
-  const uint32_t n_b = (uint32_t)J.n_b;
-  const uint32_t* cum = J.cum + (size_t)t * (b + 1);
-  const uint2* ent = J.ent + (size_t)t * n_b;
-  const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
-  double* out = J.part + ((size_t)g * J.d + t) * b + m;
-  double acc = 0.0;
-  const int64_t per = (J.n_a + J.G - 1) / J.G;
-  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
-#pragma unroll 2
-  for (int64_t i = ib; i < ie; ++i) {
-    const uint32_t c1 = __ldg(cA + i);
-    const uint32_t h1 = c1 & mask;
-    const uint32_t h2 = VARIANT == kVariantFFT ? ((m - h1) & mask) : (m ^ h1);
-    const uint32_t beg = __ldg(cum + h2), end = __ldg(cum + h2 + 1);
-    const double* row = J.C + i * J.ldc;
-    double s = 0.0;
-    for (uint32_t e = beg; e < end; ++e) {
-      const uint32_t x = __ldg(&ent[e].x);
-      const long long bits = __double_as_longlong(__ldg(row + (x & 0x7fffffffu)));
-      s += __longlong_as_double(bits ^ ((long long)(x & 0x80000000u) << 32));
-    }
-    acc += c1 >> 31 ? s : -s;
-  }
-  *out = acc;
-}
-
-// p = sum of the row groups' partial sketches (NaN when the flag is set)
-__global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__ jobs) {
-  const ProdJob& J = jobs[blockIdx.y];
-  const int64_t db = (int64_t)J.d << J.log2b;
-  const bool bad = *J.flag == 1;
-  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < db; e += (int64_t)gridDim.x * 256) {
-    double s = 0.0;
-    for (int g = 0; g < J.G; ++g) s += J.part[(size_t)g * db + e];
-    J.p[e] = bad ? __longlong_as_double(0x7ff8000000000000ll) : s;
-  }
-}
-
 // host-mapped flag set by a wait of the product kernel that ran out
+}  // namespace
+
 int* product_timeout_flag(int** dev) {
   static int* host = nullptr;
   static int* mapped = nullptr;
@@ -898,6 +621,8 @@ int* product_timeout_flag(int** dev) {
   return host;
 }
 
+namespace {
+
 template <int NMOD>
 void launch_gemm(const ProdJob* dJobs, int64_t items, cudaStream_t s) {
   int* flag = nullptr;
@@ -910,19 +635,6 @@ void launch_gemm(const ProdJob* dJobs, int64_t items, cudaStream_t s) {
 }
 
 }  // namespace
-
-// Window: about 32 to 64 entries of a row per warp step, at most 1024 buckets
-// (8 KB of shared memory a warp); row groups so that some 24 warps per SM run.
-void plan_product_sketch(ProdJob& J, int sms) {
-  const int64_t b = (int64_t)1 << J.log2b;
-  J.dense = J.n_b > 2 * b ? 1 : 0;
-  J.logW = 6;
-  while (J.logW < 10 && ((int64_t)2 << J.logW) * std::max<int64_t>(J.n_b, 1) <= 60 * b) ++J.logW;
-  J.logW = std::min(J.logW, J.log2b);
-  const int64_t warps = J.dense ? (J.d * b + 31) / 32 : J.d * (b >> J.logW);
-  const int64_t G = (int64_t)sms * 24 / std::max<int64_t>(warps, 1);
-  J.G = (int)std::max<int64_t>(1, std::min<int64_t>({G, (J.n_a + 31) / 32, 64}));
-}
 
 bool product_timed_out() {
   volatile int* h = product_timeout_flag(nullptr);
@@ -986,63 +698,6 @@ void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, 
   const dim3 g((unsigned)((n_b + 255) / 256), (unsigned)std::min<int64_t>(rows, 4096), (unsigned)count);
   if (f32) k_prod_crt<float><<<g, 256, 0, s>>>(dJobs);
   else k_prod_crt<double><<<g, 256, 0, s>>>(dJobs);
-  CMM_CUDA(cudaGetLastError());
-}
-
-void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
-  if (count <= 0) return;
-  int d = 0;
-  for (int i = 0; i < count; ++i) d = std::max(d, hJobs[i].d);
-  ProfScope prof("plan", s);
-  count_launch();
-  k_prod_index<<<dim3((unsigned)d, (unsigned)count), kIdxThreads, 0, s>>>(dJobs);
-  CMM_CUDA(cudaGetLastError());
-}
-
-void launch_product_scatter(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
-  if (count <= 0) return;
-  int gmax[2][2] = {}, dmax[2][2] = {};
-  int64_t wmax[2][2] = {};
-  size_t smem[2] = {};
-  for (int i = 0; i < count; ++i) {
-    const ProdJob& J = hJobs[i];
-    const int v = J.variant, dn = J.dense ? 1 : 0;
-    gmax[v][dn] = std::max(gmax[v][dn], J.G);
-    dmax[v][dn] = std::max(dmax[v][dn], J.d);
-    const int64_t b = (int64_t)1 << J.log2b;
-    const int64_t x = dn ? (b + 255) / 256 : ((b >> J.logW) + kScWarps - 1) / kScWarps;
-    wmax[v][dn] = std::max(wmax[v][dn], x);
-    if (!dn) smem[v] = std::max(smem[v], ((size_t)kScWarps << J.logW) * 8);
-  }
-  ProfScope prof("finalize", s);
-#define CMM_SCATTER(V)                                                                                              \
-  do {                                                                                                              \
-    if (gmax[V][0]) {                                                                                               \
-      CMM_CUDA(cudaFuncSetAttribute(k_prod_scatter<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[V])); \
-      count_launch();                                                                                               \
-      k_prod_scatter<V><<<dim3((unsigned)wmax[V][0], (unsigned)dmax[V][0], (unsigned)(gmax[V][0] * count)),         \
-                          kScWarps * 32, smem[V], s>>>(dJobs, gmax[V][0]);                                          \
-      CMM_CUDA(cudaGetLastError());                                                                                 \
-    }                                                                                                               \
-    if (gmax[V][1]) {                                                                                               \
-      count_launch();                                                                                               \
-      k_prod_scatter_dense<V><<<dim3((unsigned)wmax[V][1], (unsigned)dmax[V][1], (unsigned)(gmax[V][1] * count)),   \
-                                256, 0, s>>>(dJobs, gmax[V][1]);                                                    \
-      CMM_CUDA(cudaGetLastError());                                                                                 \
-    }                                                                                                               \
-  } while (0)
-  CMM_SCATTER(0);
-  CMM_SCATTER(1);
-#undef CMM_SCATTER
-}
-
-void launch_product_reduce(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
-  if (count <= 0) return;
-  int64_t db = 0;
-  for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
-  ProfScope prof("finalize", s);
-  count_launch();
-  k_prod_reduce<<<dim3((unsigned)std::min<int64_t>((db + 255) / 256, 2048), (unsigned)count), 256, 0, s>>>(dJobs);
   CMM_CUDA(cudaGetLastError());
 }
 

@@ -14,6 +14,8 @@ constexpr int64_t kProdMaxK = 32768;           // inner indices per launch (int3
 // kProdK-index steps of a launch over kc inner indices, in whole stages of 4
 __host__ __device__ inline int prod_ksteps(int64_t kc) { return (int)((kc + 4 * kProdK - 1) / (4 * kProdK)) * 4; }
 
+enum { kAddGather = 0, kAddStaged = 1, kAddLane = 2 };  // forms of the additions
+
 struct ProdJob {
   const void *A, *B;      // kc x n_a, kc x n_b: the inner indices of this launch
   int64_t n_a, n_b, kc;
@@ -32,11 +34,13 @@ struct ProdJob {
   int accumulate;         // add to C (later chunks of the inner index)
   // the sketch
   const uint32_t *codesA, *codesB;
-  uint32_t* cum;          // d x (b + 1)
-  uint2* ent;             // d x n_b
+  void* cum;              // sorted columns (cmm_product_add.cu): positions of the buckets
+  uint32_t* ent;          //   and entries, 2 d x n_b
   double *part, *p;       // G x d x b partial sketches; d x b
   int d, log2b, variant;
-  int logW, G, dense;     // window of a warp, row groups, lane-per-bucket form
+  int form;               // which additions (plan_product_sketch)
+  int logW, G;            // window of a warp, row groups
+  int blocks;             // blocks of columns (staged and lane forms)
 };
 
 inline int prod_moduli(bool f32) { return f32 ? 8 : 15; }
@@ -49,19 +53,23 @@ inline size_t prod_residue_bytes(int tiles_p, int tiles_b, bool f32) {
   return (size_t)prod_moduli(f32) * 65536 * tiles_p * tiles_b;
 }
 
-// sketch geometry of a job from its sizes (logW, G, dense)
+// geometry of the additions of a job from its sizes (form, logW, G, blocks)
 void plan_product_sketch(ProdJob& J, int sms);
+size_t prod_cum_bytes(const ProdJob& J);
+// C's row stride: even, so that rows can be copied in 16-byte units
+inline int64_t prod_ldc(int64_t n_b) { return (n_b + 1) & ~(int64_t)1; }
 // the largest n_a n_b whose product is formed (8 GiB of FP64)
 constexpr int64_t kProdMaxEntries = (int64_t)1 << 30;
 
-// hJobs: the host copy of dJobs.  Sorted bucket lists (also clears the flags);
-// exponents and residue planes; the product; the partial sketches; their sum.
+// hJobs: the host copy of dJobs.  Sorted columns (also clears the flags);
+// exponents and residue planes; the product; the additions and their sum.
 void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
 void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
 void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
-void launch_product_scatter(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
-void launch_product_reduce(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
-// true (and cleared) when a wait of the product kernel ran out since the last call
+void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
+// host-mapped flag set by a wait of these kernels that ran out (*dev: its device address)
+int* product_timeout_flag(int** dev);
+// true (and cleared) when such a wait ran out since the last call
 bool product_timed_out();
 
 }  // namespace cmm

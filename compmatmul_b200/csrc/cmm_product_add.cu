@@ -1,0 +1,651 @@
+// Additions of the product sketch: p_t[idx(i, j)] += s1_t(i) s2_t(j) C[i][j] for
+// every entry of C = A^T B and every repetition t (cmm_product.cu forms C).
+//
+// d n_a n_b additions of 8-byte values to pseudo-random buckets.  Done without
+// atomics and in a fixed order, from the side of the buckets: for a row i the
+// columns that fall into consecutive buckets [m, m + W) of p_t are
+// consecutive in the order of h2 (FFT: h2 in [m - h1(i), + W) mod b; FWHT: the
+// aligned block (m ^ h1(i)) / W), so a warp that owns W buckets reads its
+// entries of the sorted columns coalesced, looks up their C[i][j] and adds.
+// Three forms, chosen by plan_product_sketch:
+//  staged  b <= 2^16: rows of C staged in shared memory, a CTA of 16 windows;
+//  lane    a block of columns holds more columns than there are buckets: lane
+//          = bucket, rows and sorted columns in shared memory;
+//  gather  b > 2^16: values gathered from L2.
+// Rows are split into G groups with partial sketches, added up by
+// k_prod_reduce.
+#include <algorithm>
+
+#include "cmm_internal.h"
+#include "cmm_product.h"
+#include "cmm_product_dev.cuh"
+
+namespace cmm {
+namespace {
+
+constexpr int kIdxThreads = 1024;
+constexpr int kScCols = 4096;  // columns per block of the staged and lane forms (12 bits of an entry)
+constexpr int kScWin = 16;     // windows (warps) per CTA of the staged form
+constexpr int kScThreads = 32 * (kScWin + 1);
+constexpr size_t kScSmemMax = 227 * 1024 - 1024;
+constexpr int kGaWarps = 8;    // windows (warps) per CTA of the gather form
+
+// A sorted column, in the order in which the additions take it apart: rank |
+// j << 3 | (s2 < 0) << (3 + JB) | h2 << (4 + JB) (low bits), JB = 12 (16 bits
+// of h2) or, gather form, 17 (11 bits).  rank counts the entries of the same
+// bucket before it (6: six or more; 7: no entry), j << 3 is the offset of the
+// value in the row.  Every list is stored twice in a row, so that a run that
+// wraps around b (FFT) is read without a test.
+constexpr uint32_t kNoEntry = 7;
+template <int JB>
+constexpr uint32_t kColMask = ((1u << JB) - 1u) << 3;
+
+// ------------------------------------------------------------ sorted columns
+// One CTA per (t, block of kScCols columns, job).  The keys (h2, j) are unique,
+// so a bitonic sort in shared memory gives the fixed order without atomics.
+// cum[h] = entries below bucket h, 16 bits, row stride b + 8 (16-byte stores
+// of eight: the first by binary search, the others by walking on).
+__host__ __device__ inline size_t cum16_stride(int log2b) { return ((size_t)1 << log2b) + 8; }
+__global__ void __launch_bounds__(kIdxThreads) k_prod_index_blocks(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.z];
+  const int t = blockIdx.x, jb = blockIdx.y;
+  if (J.form == kAddGather || t >= J.d || (int64_t)jb * kScCols >= J.n_b) return;
+  if (t == 0 && jb == 0 && threadIdx.x == 0) *J.flag = 0;
+  __shared__ uint32_t key[kScCols];
+  const int tid = threadIdx.x;
+  const uint32_t b = 1u << J.log2b;
+  const uint32_t n = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
+  const uint32_t* codes = J.codesB + (size_t)t * J.n_b + (size_t)jb * kScCols;
+  uint32_t len = 32;
+  while (len < n) len <<= 1;
+  for (uint32_t e = tid; e < len; e += kIdxThreads) {
+    const uint32_t c = e < n ? codes[e] : 0u;
+    key[e] = e < n ? ((~c) >> 31) << 28 | (c & (b - 1)) << 12 | e : 0xffffffffu;
+  }
+  __syncthreads();
+  // the sign is carried, not compared; padding compares as the largest
+  auto order = [&](uint32_t k) { return k == 0xffffffffu ? k : (k & 0x0fffffffu); };
+  for (uint32_t size = 2; size <= len; size <<= 1)
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t q = tid; q < len / 2; q += kIdxThreads) {
+        const uint32_t lo = 2 * q - (q & (stride - 1)), hi = lo + stride;
+        const uint32_t x = key[lo], y = key[hi];
+        if ((order(x) > order(y)) == ((lo & size) == 0)) {
+          key[lo] = y;
+          key[hi] = x;
+        }
+      }
+      __syncthreads();
+    }
+  auto bucket = [&](uint32_t e) { return (key[e] >> 12) & 0xffffu; };
+  uint32_t* ent = J.ent + 2 * ((size_t)t * J.n_b + (size_t)jb * kScCols);
+  for (uint32_t e = tid; e < n; e += kIdxThreads) {
+    uint32_t rank = 0;
+    while (rank < 6 && rank < e && bucket(e - rank - 1) == bucket(e)) ++rank;
+    const uint32_t x = rank | (key[e] & 0xfffu) << 3 | (key[e] >> 28) << 15 | bucket(e) << 16;
+    ent[e] = x;
+    ent[n + e] = x;
+  }
+  uint16_t* cum = reinterpret_cast<uint16_t*>(J.cum) + ((size_t)t * J.blocks + jb) * cum16_stride(J.log2b);
+  for (uint32_t h0 = tid * 8; h0 <= b; h0 += kIdxThreads * 8) {
+    uint32_t lo = 0, hi = n;  // the first entry with bucket >= h0
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (bucket(mid) >= h0) hi = mid;
+      else lo = mid + 1;
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 8; ++u) {
+      while (lo < n && bucket(lo) < h0 + u) ++lo;
+      if (u & 1) w[u >> 1] |= lo << 16;
+      else w[u >> 1] = lo;
+    }
+    *reinterpret_cast<uint4*>(cum + h0) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// The same over all columns (at most 2^17) for the gather form: counting sort
+// with L2 atomics; each bucket's entries are then put in ascending j, so the
+// order does not depend on the atomics.  One CTA per (t, job).
+__global__ void __launch_bounds__(kIdxThreads) k_prod_index(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  const int t = blockIdx.x;
+  if (J.form != kAddGather || t >= J.d) return;
+  if (t == 0 && threadIdx.x == 0) *J.flag = 0;
+  const uint32_t b = 1u << J.log2b;
+  const uint32_t n = (uint32_t)J.n_b;
+  uint32_t* cum = reinterpret_cast<uint32_t*>(J.cum) + (size_t)t * (b + 1);
+  uint32_t* ent = J.ent + 2 * (size_t)t * n;
+  const uint32_t* codes = J.codesB + (size_t)t * n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t ws[32];
+  __shared__ uint32_t s_carry;
+  for (uint32_t e = tid; e <= b; e += kIdxThreads) __stcg(cum + e, 0u);
+  if (tid == 0) s_carry = 0;
+  __syncthreads();
+  for (uint32_t j = tid; j < n; j += kIdxThreads) atomicAdd(cum + 1 + (codes[j] & (b - 1)), 1u);
+  __syncthreads();
+  // exclusive scan of the counts: cum[h + 1] = start of bucket h
+  for (uint32_t base = 1; base <= b; base += kIdxThreads * 8) {
+    uint32_t v[8], sum = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t e = base + tid * 8 + u;
+      v[u] = e <= b ? __ldcg(cum + e) : 0u;
+      sum += v[u];
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t w = ws[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += x;
+      }
+      ws[lane] = w;
+    }
+    __syncthreads();
+    uint32_t run = s_carry + (warp ? ws[warp - 1] : 0u) + inc - sum;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t e = base + tid * 8 + u;
+      if (e <= b) __stcg(cum + e, run);
+      run += v[u];
+    }
+    __syncthreads();
+    if (tid == 0) s_carry += ws[31];
+    __syncthreads();
+  }
+  // placement moves cum[h + 1] from the start of bucket h to its end
+  for (uint32_t j = tid; j < n; j += kIdxThreads) {
+    const uint32_t c = codes[j], h = c & (b - 1);
+    __stcg(ent + atomicAdd(cum + 1 + h, 1u), j << 3 | ((~c) >> 31) << 20 | (h & 0x7ffu) << 21);
+  }
+  __syncthreads();
+  for (uint32_t h = tid; h < b; h += kIdxThreads) {
+    const uint32_t beg = __ldcg(cum + h), end = __ldcg(cum + h + 1);
+    for (uint32_t e = beg + 1; e < end; ++e) {  // insertion sort by j
+      const uint32_t x = __ldcg(ent + e);
+      uint32_t f = e;
+      while (f > beg) {
+        const uint32_t y = __ldcg(ent + f - 1);
+        if ((y & kColMask<17>) <= (x & kColMask<17>)) break;
+        __stcg(ent + f, y);
+        --f;
+      }
+      if (f != e) __stcg(ent + f, x);
+    }
+    for (uint32_t e = beg; e < end; ++e) {
+      const uint32_t x = __ldcg(ent + e) | min(e - beg, 6u);
+      __stcg(ent + e, x);
+      __stcg(ent + n + e, x);
+    }
+  }
+}
+
+// ----------------------------------------------------------------- additions
+// A warp's look-up of 32 rows (one a lane): first entry, count and key of the
+// window in each row
+struct RowKeys {
+  uint32_t e0, cnt, key, neg1;
+};
+template <int VARIANT, int JB, typename CumT>
+__device__ __forceinline__ RowKeys row_keys(const uint32_t* cA, const CumT* cum, int64_t i, int64_t ie, uint32_t m0,
+                                            uint32_t W, uint32_t b, uint32_t cols) {
+  RowKeys k{0, 0, 0, 0};
+  if (i < ie) {
+    const uint32_t c1 = __ldg(cA + i);
+    const uint32_t h1 = c1 & (b - 1);
+    const uint32_t s = VARIANT == kVariantFFT ? ((m0 - h1) & (b - 1)) : ((m0 ^ h1) & ~(W - 1u));
+    k.key = (VARIANT == kVariantFFT ? s : h1) << (JB + 4);
+    k.neg1 = ~c1 & 0x80000000u;
+    k.e0 = __ldg(cum + s);
+    const uint32_t se = s + W;
+    k.cnt = se <= b ? __ldg(cum + se) - k.e0 : cols - k.e0 + __ldg(cum + se - b);
+  }
+  return k;
+}
+__device__ __forceinline__ uint32_t entry_at(const uint32_t* ent, uint32_t count, uint32_t at) {
+  return at < count ? __ldg(ent + at) : kNoEntry;
+}
+template <int JB>
+__device__ __forceinline__ double signed_value(double c, uint32_t e, uint32_t neg1) {
+  return __longlong_as_double(__double_as_longlong(c) ^ ((long long)(((e << (28 - JB)) & 0x80000000u) ^ neg1) << 32));
+}
+// Adds a batch (one entry and its signed value a lane) to the warp's window of
+// W = wmask / 8 + 1 buckets.  Entries of one bucket are neighbours and are
+// added one rank after the other.
+template <int VARIANT, int JB>
+__device__ __forceinline__ void add_batch(double* acc, uint32_t e, double v, uint32_t key, uint32_t wmask, int lane) {
+  const uint32_t rank = e & 7u;
+  const uint32_t at = ((VARIANT == kVariantFFT ? e - key : e ^ key) >> (JB + 1)) & wmask;
+  double* a = reinterpret_cast<double*>(reinterpret_cast<char*>(acc) + at);
+  if (rank == 0) *a += v;
+  __syncwarp();
+  uint32_t todo = __ballot_sync(0xffffffffu, rank - 1u < 6u);
+  for (uint32_t k = 1; todo; ++k) {
+    bool now = rank == k;
+    if (k >= 6) now = lane == __ffs(todo) - 1;  // six or more: one lane at a time, in order
+    if (now) *a += v;
+    todo &= ~__ballot_sync(0xffffffffu, now);
+    __syncwarp();
+  }
+}
+
+// ring of row blocks of C filled by one thread of warp kScWin with bulk copies
+struct RowRing {
+  unsigned char* base;
+  uint32_t row_bytes;
+  int stages;
+};
+__device__ __forceinline__ void produce_rows(const ProdJob& J, const RowRing& R, uint64_t* full, uint64_t* empty,
+                                             int64_t ib, int64_t ie, volatile int* abort) {
+  unsigned it = 0, st = 0, ph = 0;
+  bool ok = true;
+  for (int jb = 0; jb < J.blocks && ok; ++jb) {
+    const uint32_t cols = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
+    const uint32_t bytes = ((cols + 1u) & ~1u) * 8u;  // the row stride is even
+    for (int64_t i = ib; i < ie; ++i, ++it) {
+      if (!bar_wait(&empty[st], ph ^ 1u, abort)) { ok = false; break; }
+      bar_expect(&full[st], bytes);
+      bulk_load(R.base + st * R.row_bytes, J.C + i * J.ldc + (int64_t)jb * kScCols, bytes, &full[st]);
+      if (++st == (unsigned)R.stages) { st = 0; ph ^= 1u; }
+    }
+  }
+  if (!ok)  // let the copies in flight land before the CTA ends
+    for (int q = 0; q < R.stages; ++q)
+      for (uint32_t k = 0; k < (1u << 16) && it > (unsigned)q; ++k) {
+        const unsigned z = it - 1 - q;
+        if (bar_test(&full[z % R.stages], (z / R.stages) & 1u)) break;
+        __nanosleep(20);
+      }
+}
+
+// Staged form.  A gather from global memory costs one L1 tag cycle per lane (32
+// a batch), from shared memory about six wavefronts; what pays is that one CTA
+// covers 16 windows, so every staged row serves up to 2^14 buckets.  Warp 16
+// copies the row blocks, warps 0-15 own a window each; the next row's entries
+// are read while a row is added.
+template <int VARIANT>
+__global__ void __launch_bounds__(kScThreads, 1) k_prod_add_staged(const ProdJob* __restrict__ jobs, int gmax,
+                                                                   uint32_t smem, int* __restrict__ timeout) {
+  extern __shared__ __align__(128) unsigned char ssm[];
+  __shared__ uint64_t full[8], empty[8];
+  __shared__ int s_abort;
+  const ProdJob& J = jobs[blockIdx.z / gmax];
+  const int g = blockIdx.z % gmax, t = blockIdx.y;
+  if (J.variant != VARIANT || J.form != kAddStaged || g >= J.G || t >= J.d) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t b = 1u << J.log2b, W = 1u << J.logW, wmask = (W - 1u) * 8u;
+  const uint32_t win0 = blockIdx.x * kScWin, wins = b >> J.logW;
+  if (win0 >= wins) return;
+  const int nw = (int)min((uint32_t)kScWin, wins - win0);
+  double* acc0 = reinterpret_cast<double*>(ssm);
+  const uint32_t acc_bytes = ((uint32_t)kScWin << J.logW) * 8u;
+  RowRing R;
+  R.base = ssm + acc_bytes;
+  R.row_bytes = (((uint32_t)min((int64_t)kScCols, J.n_b) + 15u) & ~15u) * 8u;
+  R.stages = (int)min(8u, (smem - acc_bytes) / R.row_bytes);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], nw); }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  volatile int* abort = &s_abort;
+  const int64_t per = (J.n_a + J.G - 1) / J.G;
+  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
+  if (warp == kScWin) {
+    if (lane == 0) produce_rows(J, R, full, empty, ib, ie, abort);
+  } else if (warp < nw) {
+    const uint32_t m0 = (win0 + warp) << J.logW;
+    double* acc = acc0 + (size_t)warp * W;
+    for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
+    __syncwarp();
+    const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
+    int st = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    for (int jb = 0; jb < J.blocks && ok; ++jb) {
+      const uint32_t cols = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
+      const uint16_t* cum = reinterpret_cast<const uint16_t*>(J.cum) + ((size_t)t * J.blocks + jb) * cum16_stride(J.log2b);
+      const uint32_t* ent = J.ent + 2 * ((size_t)t * J.n_b + (size_t)jb * kScCols);
+      for (int64_t r0 = ib; r0 < ie && ok; r0 += 32) {
+        const RowKeys k = row_keys<VARIANT, 12>(cA, cum, r0 + lane, ie, m0, W, b, cols);
+        const int rows = (int)min((int64_t)32, ie - r0);
+        uint32_t cn = __shfl_sync(0xffffffffu, k.cnt, 0);
+        const uint32_t* en = ent + __shfl_sync(0xffffffffu, k.e0, 0);
+        uint32_t f0 = entry_at(en, cn, lane), f1 = entry_at(en, cn, lane + 32), f2 = entry_at(en, cn, lane + 64);
+        for (int r = 0; r < rows; ++r) {
+          const uint32_t cc = cn, c0 = f0, c1 = f1, c2 = f2;
+          const uint32_t* ec = en;
+          const uint32_t key = __shfl_sync(0xffffffffu, k.key, r), neg1 = __shfl_sync(0xffffffffu, k.neg1, r);
+          if (r + 1 < rows) {
+            cn = __shfl_sync(0xffffffffu, k.cnt, r + 1);
+            en = ent + __shfl_sync(0xffffffffu, k.e0, r + 1);
+            f0 = entry_at(en, cn, lane);
+            f1 = entry_at(en, cn, lane + 32);
+            f2 = entry_at(en, cn, lane + 64);
+          }
+          ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+          if (!ok) break;
+          const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
+          auto take = [&](uint32_t e) {  // (a lane without an entry reads column 0)
+            const double c = *reinterpret_cast<const double*>(row + (e & kColMask<12>));
+            add_batch<VARIANT, 12>(acc, e, signed_value<12>(c, e, neg1), key, wmask, lane);
+          };
+          if (cc > 0) take(c0);
+          if (cc > 32) take(c1);
+          if (cc > 64) take(c2);
+          for (uint32_t at = 96; at < cc; at += 32) take(entry_at(ec, cc, at + lane));
+          __syncwarp();
+          if (lane == 0) bar_arrive(&empty[st]);
+          if (++st == R.stages) { st = 0; ph ^= 1u; }
+        }
+      }
+    }
+    double* out = J.part + ((size_t)g * J.d + t) * b + m0;
+    for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
+  }
+  __syncthreads();
+  if (s_abort && threadIdx.x == 0) {
+    *timeout = 1;
+    *J.flag = 1;
+    __threadfence_system();
+  }
+}
+
+// Lane form: thread = NB buckets (sums in registers); for row i bucket m adds
+// the run of entries of h2 = m - h1(i) (FWHT: m ^ h1(i)).  The sorted columns
+// of the block and the rows are in shared memory.
+template <int VARIANT, int NB>
+__global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* __restrict__ jobs, int gmax,
+                                                                 uint32_t smem, int* __restrict__ timeout) {
+  extern __shared__ __align__(128) unsigned char ssm[];
+  __shared__ uint64_t full[8], empty[8];
+  __shared__ int s_abort;
+  constexpr uint32_t b = 512u * NB;
+  const ProdJob& J = jobs[blockIdx.z / gmax];
+  const int g = blockIdx.z % gmax, t = blockIdx.y;
+  if (J.variant != VARIANT || J.form != kAddLane || (1u << J.log2b) != b || g >= J.G || t >= J.d) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t* es = reinterpret_cast<uint32_t*>(ssm);                         // kScCols entries
+  uint16_t* cs = reinterpret_cast<uint16_t*>(ssm + kScCols * 4);           // b + 8 positions
+  constexpr uint32_t list_bytes = kScCols * 4 + ((b + 8) * 2 + 127) / 128 * 128;
+  RowRing R;
+  R.base = ssm + list_bytes;
+  R.row_bytes = (((uint32_t)min((int64_t)kScCols, J.n_b) + 15u) & ~15u) * 8u;
+  R.stages = (int)min(8u, (smem - list_bytes) / R.row_bytes);
+  if (tid == 0) {
+    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], kScWin); }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  volatile int* abort = &s_abort;
+  const int64_t per = (J.n_a + J.G - 1) / J.G;
+  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
+  if (warp == kScWin) {
+    if (lane == 0) produce_rows(J, R, full, empty, ib, ie, abort);
+  } else {
+    const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
+    double acc[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) acc[q] = 0.0;
+    int st = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    for (int jb = 0; jb < J.blocks; ++jb) {  // (every warp takes every block's barriers)
+      const uint32_t cols = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
+      const uint16_t* cum = reinterpret_cast<const uint16_t*>(J.cum) + ((size_t)t * J.blocks + jb) * cum16_stride(J.log2b);
+      const uint32_t* ent = J.ent + 2 * ((size_t)t * J.n_b + (size_t)jb * kScCols);
+      asm volatile("bar.sync 1, 512;" ::: "memory");  // the previous block's list is no longer read
+      for (uint32_t e = tid; e < cols; e += 512) es[e] = __ldg(ent + e);
+      for (uint32_t e = tid; e <= b; e += 512) cs[e] = __ldg(cum + e);
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      for (int64_t r0 = ib; r0 < ie && ok; r0 += 32) {
+        const uint32_t codes = r0 + lane < ie ? __ldg(cA + r0 + lane) : 0u;
+        const int rows = (int)min((int64_t)32, ie - r0);
+        for (int r = 0; r < rows; ++r) {
+          const uint32_t c1 = __shfl_sync(0xffffffffu, codes, r);
+          const uint32_t h1 = c1 & (b - 1);
+          ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+          if (!ok) break;
+          const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
+#pragma unroll
+          for (int q = 0; q < NB; ++q) {
+            const uint32_t m = q * 512 + tid;
+            const uint32_t h2 = VARIANT == kVariantFFT ? ((m - h1) & (b - 1)) : (m ^ h1);
+            const uint32_t end = cs[h2 + 1];
+            double s = 0.0;
+            for (uint32_t e = cs[h2]; e < end; ++e) {
+              const uint32_t x = es[e];
+              s += signed_value<12>(*reinterpret_cast<const double*>(row + (x & kColMask<12>)), x, 0u);
+            }
+            acc[q] += c1 >> 31 ? s : -s;
+          }
+          __syncwarp();
+          if (lane == 0) bar_arrive(&empty[st]);
+          if (++st == R.stages) { st = 0; ph ^= 1u; }
+        }
+      }
+    }
+    double* out = J.part + ((size_t)g * J.d + t) * b;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) out[q * 512 + tid] = acc[q];
+  }
+  __syncthreads();
+  if (s_abort && tid == 0) {
+    *timeout = 1;
+    *J.flag = 1;
+    __threadfence_system();
+  }
+}
+
+// Gather form: windows as in the staged form, values from L2.  Entries are read
+// two rows ahead and values one row ahead of the additions, so a row's chain
+// of two L2 latencies overlaps the rows before it.
+template <int VARIANT>
+__global__ void __launch_bounds__(kGaWarps * 32) k_prod_add_gather(const ProdJob* __restrict__ jobs, int gmax) {
+  extern __shared__ double sacc[];
+  const ProdJob& J = jobs[blockIdx.z / gmax];
+  const int g = blockIdx.z % gmax, t = blockIdx.y;
+  if (J.variant != VARIANT || J.form != kAddGather || g >= J.G || t >= J.d) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t b = 1u << J.log2b, W = 1u << J.logW, wmask = (W - 1u) * 8u;
+  const uint32_t m0 = (blockIdx.x * kGaWarps + warp) << J.logW;
+  if (m0 >= b) return;
+  double* acc = sacc + (size_t)warp * W;
+  for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
+  __syncwarp();
+  const uint32_t cols = (uint32_t)J.n_b;
+  const uint32_t* cum = reinterpret_cast<const uint32_t*>(J.cum) + (size_t)t * (b + 1);
+  const uint32_t* ent = J.ent + 2 * (size_t)t * cols;
+  const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
+  const int64_t per = (J.n_a + J.G - 1) / J.G;
+  const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
+  const size_t ldc = (size_t)J.ldc * 8;
+  for (int64_t r0 = ib; r0 < ie; r0 += 32) {
+    const RowKeys k = row_keys<VARIANT, 17>(cA, cum, r0 + lane, ie, m0, W, b, cols);
+    const int rows = (int)min((int64_t)32, ie - r0);
+    const char* row = reinterpret_cast<const char*>(J.C) + (size_t)r0 * ldc;  // of row r
+    auto value = [&](const char* at, uint32_t e) {
+      return e != kNoEntry ? __ldg(reinterpret_cast<const double*>(at + (e & kColMask<17>))) : 0.0;
+    };
+    auto entries = [&](int r, uint32_t (&x)[3]) {
+      const uint32_t n = r < rows ? __shfl_sync(0xffffffffu, k.cnt, r) : 0u;
+      const uint32_t* at = ent + __shfl_sync(0xffffffffu, k.e0, r & 31);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) x[q] = entry_at(at, n, lane + 32 * q);
+    };
+    uint32_t e[3], f[3], h[3];  // rows r, r + 1, r + 2
+    double v[3], w[3];          // rows r, r + 1
+    entries(0, e);
+    entries(1, f);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] = value(row, e[q]);
+    for (int r = 0; r < rows; ++r) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) w[q] = value(row + ldc, f[q]);
+      entries(r + 2, h);
+      const uint32_t key = __shfl_sync(0xffffffffu, k.key, r), neg1 = __shfl_sync(0xffffffffu, k.neg1, r);
+      const uint32_t cc = __shfl_sync(0xffffffffu, k.cnt, r);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (cc > 32 * q) add_batch<VARIANT, 17>(acc, e[q], signed_value<17>(v[q], e[q], neg1), key, wmask, lane);
+      if (cc > 96) {
+        const uint32_t* ec = ent + __shfl_sync(0xffffffffu, k.e0, r);
+        for (uint32_t at = 96; at < cc; at += 32) {
+          const uint32_t x = entry_at(ec, cc, at + lane);
+          add_batch<VARIANT, 17>(acc, x, signed_value<17>(value(row, x), x, neg1), key, wmask, lane);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        e[q] = f[q];
+        f[q] = h[q];
+        v[q] = w[q];
+      }
+      row += ldc;
+    }
+  }
+  double* out = J.part + ((size_t)g * J.d + t) * b + m0;
+  for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
+}
+
+// p = sum of the row groups' partial sketches (NaN when the flag is set)
+__global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__ jobs) {
+  const ProdJob& J = jobs[blockIdx.y];
+  const int64_t db = (int64_t)J.d << J.log2b;
+  const bool bad = *J.flag == 1;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < db; e += (int64_t)gridDim.x * 256) {
+    double s = 0.0;
+    for (int g = 0; g < J.G; ++g) s += J.part[(size_t)g * db + e];
+    J.p[e] = bad ? __longlong_as_double(0x7ff8000000000000ll) : s;
+  }
+}
+
+}  // namespace
+
+void plan_product_sketch(ProdJob& J, int sms) {
+  const int64_t b = (int64_t)1 << J.log2b;
+  const int64_t cols = std::max<int64_t>(std::min<int64_t>(J.n_b, kScCols), 1);
+  J.blocks = (int)((J.n_b + kScCols - 1) / kScCols);
+  J.form = J.log2b > 16 ? kAddGather : (cols >= b ? kAddLane : kAddStaged);
+  // windows: 36 to 72 entries of a row, at most 1024 buckets (8 KB of shared memory a warp)
+  const int64_t per_row = J.form == kAddGather ? std::max<int64_t>(J.n_b, 1) : cols;
+  J.logW = 5;
+  while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 72 * b) ++J.logW;
+  J.logW = std::min(J.logW, J.log2b);
+  const int64_t wins = b >> J.logW;
+  if (J.form == kAddGather) {
+    // Row groups of at most 32 MB of C: the CTAs in flight then work on about
+    // two groups, which stay in L2.  (16384 rows of 16384 columns, b = 2^18: 60
+    // ms in 3 groups, whose CTAs drift apart and miss L2.)
+    const int64_t rows = std::max<int64_t>(32, ((int64_t)32 << 20) / (8 * per_row));
+    const int64_t fill = 12 * (int64_t)sms / (J.d * ((wins + kGaWarps - 1) / kGaWarps));
+    J.G = (int)std::max<int64_t>(1, std::min<int64_t>({std::max((J.n_a + rows - 1) / rows, fill), (J.n_a + 31) / 32, 512}));
+    return;
+  }
+  // one CTA per SM
+  const int64_t ctas = J.form == kAddLane ? J.d : J.d * ((wins + kScWin - 1) / kScWin);
+  J.G = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sms / ctas, (J.n_a + 31) / 32, 64}));
+}
+
+size_t prod_cum_bytes(const ProdJob& J) {
+  return J.form == kAddGather ? (size_t)J.d * (((size_t)1 << J.log2b) + 1) * 4
+                              : (size_t)J.d * J.blocks * cum16_stride(J.log2b) * 2;
+}
+
+void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  if (count <= 0) return;
+  int d[2] = {}, blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    int& m = d[hJobs[i].form == kAddGather ? 0 : 1];
+    m = std::max(m, hJobs[i].d);
+    blocks = std::max(blocks, hJobs[i].blocks);
+  }
+  ProfScope prof("plan", s);
+  if (d[0]) {
+    count_launch();
+    k_prod_index<<<dim3((unsigned)d[0], (unsigned)count), kIdxThreads, 0, s>>>(dJobs);
+    CMM_CUDA(cudaGetLastError());
+  }
+  if (d[1]) {
+    count_launch();
+    k_prod_index_blocks<<<dim3((unsigned)d[1], (unsigned)blocks, (unsigned)count), kIdxThreads, 0, s>>>(dJobs);
+    CMM_CUDA(cudaGetLastError());
+  }
+}
+
+namespace {
+
+// the jobs of one kernel: its grid and shared memory
+struct AddGrid {
+  int g = 0, d = 0;
+  int64_t x = 0;
+  size_t smem = 0;
+  void include(const ProdJob& J, int64_t ctas, size_t need) {
+    g = std::max(g, J.G);
+    d = std::max(d, J.d);
+    x = std::max(x, ctas);
+    smem = std::max(smem, need);
+  }
+  dim3 grid(int count) const { return dim3((unsigned)x, (unsigned)d, (unsigned)(g * count)); }
+};
+
+template <typename K, typename... A>
+void launch_add(K kernel, const AddGrid& G, int count, int threads, cudaStream_t s, A... args) {
+  if (!G.g) return;
+  CMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.smem));
+  count_launch();
+  kernel<<<G.grid(count), threads, G.smem, s>>>(args...);
+  CMM_CUDA(cudaGetLastError());
+}
+
+template <int V>
+void launch_adds(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  AddGrid gather, staged, lane[4];  // lane: b = 512 .. 4096
+  for (int i = 0; i < count; ++i) {
+    const ProdJob& J = hJobs[i];
+    if (J.variant != V) continue;
+    const int64_t wins = ((int64_t)1 << J.log2b) >> J.logW;
+    const size_t rows = 8 * ((((size_t)std::min<int64_t>(J.n_b, kScCols) + 15) & ~(size_t)15) * 8);  // a ring of eight
+    if (J.form == kAddGather) gather.include(J, (wins + kGaWarps - 1) / kGaWarps, ((size_t)kGaWarps << J.logW) * 8);
+    else if (J.form == kAddStaged)
+      staged.include(J, (wins + kScWin - 1) / kScWin, std::min(((size_t)kScWin << J.logW) * 8 + rows, kScSmemMax));
+    else lane[J.log2b - 9].include(J, 1, std::min((size_t)kScCols * 4 + (2u << J.log2b) + 128 + rows, kScSmemMax));
+  }
+  int* flag = nullptr;
+  product_timeout_flag(&flag);
+  launch_add(k_prod_add_gather<V>, gather, count, kGaWarps * 32, s, dJobs, gather.g);
+  launch_add(k_prod_add_staged<V>, staged, count, kScThreads, s, dJobs, staged.g, (uint32_t)staged.smem, flag);
+  launch_add(k_prod_add_lane<V, 1>, lane[0], count, kScThreads, s, dJobs, lane[0].g, (uint32_t)lane[0].smem, flag);
+  launch_add(k_prod_add_lane<V, 2>, lane[1], count, kScThreads, s, dJobs, lane[1].g, (uint32_t)lane[1].smem, flag);
+  launch_add(k_prod_add_lane<V, 4>, lane[2], count, kScThreads, s, dJobs, lane[2].g, (uint32_t)lane[2].smem, flag);
+  launch_add(k_prod_add_lane<V, 8>, lane[3], count, kScThreads, s, dJobs, lane[3].g, (uint32_t)lane[3].smem, flag);
+}
+
+}  // namespace
+
+void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+  if (count <= 0) return;
+  ProfScope prof("finalize", s);
+  launch_adds<kVariantFFT>(hJobs, dJobs, count, s);
+  launch_adds<kVariantFWHT>(hJobs, dJobs, count, s);
+  int64_t db = 0;
+  for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
+  count_launch();
+  k_prod_reduce<<<dim3((unsigned)std::min<int64_t>((db + 255) / 256, 2048), (unsigned)count), 256, 0, s>>>(dJobs);
+  CMM_CUDA(cudaGetLastError());
+}
+
+}  // namespace cmm
