@@ -33,6 +33,7 @@
 #include "../../include/compmatmul_b200.h"
 #include "cmm_batch.h"
 #include "cmm_fft_device.cuh"
+#include "cmm_product.h"
 
 namespace cmm {
 namespace {
@@ -758,6 +759,12 @@ struct BatchPlan {
   DevBuf params, codes, scale, partial, work, dprods, ditems, counter, hjobs, sjobs, fjobs;
   int n_fjobs = 0;  // batched finalize jobs (b <= 2^14); other products finalize one by one
   int n_items = 0, ctas = 0, n_scale_jobs = 0;
+  // products that take the product sketch (cmm_product.cu): runs of jobs that
+  // share one work space, each run's jobs longest inner dimension first
+  std::vector<int> by_product;        // per product: 1 if it is one of them
+  std::vector<ProdJob> pjobs;
+  std::vector<std::pair<int, int>> pruns;  // [first, last) jobs
+  DevBuf pmem, plists, pdev, pflags;
   int64_t max_hash_total = 0, max_inner = 0;
   const double2* tw4096 = nullptr;
   cudaGraph_t graph = nullptr;
@@ -851,15 +858,81 @@ void enqueue(BatchPlan& B, cudaStream_t s) {
                             B.tw4096, B.ctas, s);
   }
   batch_launch_finalize(B.fjobs.as<FinJob>(), B.n_fjobs, s);
+  if (!B.pjobs.empty()) CMM_CUDA(cudaMemsetAsync(B.pflags.ptr, 0, B.pflags.bytes, s));
+  for (const auto& run : B.pruns) {
+    const ProdJob* h = B.pjobs.data() + run.first;
+    const ProdJob* d = B.pdev.as<ProdJob>() + run.first;
+    const int n = run.second - run.first;
+    launch_product_planes(h, d, n, B.f32, s);
+    launch_product_gemm(h, d, n, B.f32, s);
+    launch_product_add(h, d, n, s);
+  }
   for (int i = 0; i < B.count; ++i) {
     const cmm_batch_product& q = B.prods[(size_t)i];
-    if (!batch_finalize_fits(B.plans[(size_t)i].log2b))
+    if (!B.by_product[(size_t)i] && !batch_finalize_fits(B.plans[(size_t)i].log2b))
       launch_finalize(B.plans[(size_t)i], B.partial.as<unsigned char>() + B.off_partial[(size_t)i], B.tw[(size_t)i],
                       B.work.ptr, q.p, s);
     if (q.C)
       launch_decompress_dense(q.variant, q.d, q.b, q.n_a, q.n_b, B.codes.as<uint32_t>() + B.off_codesA[(size_t)i],
                               B.codes.as<uint32_t>() + B.off_codesB[(size_t)i], q.p, q.C, s);
   }
+}
+
+// The jobs of the products that take the product sketch, their memory and
+// their sorted columns.  A run's work space takes at most a third of the free
+// device memory or 8 GiB; C is formed in the product's own dense output where
+// there is one.
+void make_product_jobs(BatchPlan& B, cudaStream_t s) {
+  std::vector<int> order;
+  for (int i = 0; i < B.count; ++i)
+    if (B.by_product[(size_t)i]) order.push_back(i);
+  if (order.empty()) return;
+  product_timeout_flag(nullptr);  // set up before any capture
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return B.prods[(size_t)a].n_inner > B.prods[(size_t)b].n_inner; });
+  size_t free_b = 0, total_b = 0;
+  CMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  const size_t budget = std::min<size_t>(free_b / 3, (size_t)8 << 30);
+  size_t lists = 0, work = 0, most = 0;
+  std::vector<size_t> at_work, at_list;
+  int64_t items = 0;
+  for (size_t k = 0; k < order.size(); ++k) {
+    const cmm_batch_product& q = B.prods[(size_t)order[k]];
+    ProdJob J{};
+    product_geometry(J, q.variant, q.d, q.b, q.n_a, q.n_b, q.n_inner, false, num_sms());
+    const size_t need = product_work_bytes(J, B.f32, !product_usable_c(J, q.C));
+    if (B.pruns.empty() || work + need > budget) {
+      B.pruns.push_back({(int)k, (int)k});
+      work = 0;
+      items = 0;
+    }
+    items += (int64_t)J.tiles_a * J.tiles_b * prod_moduli(B.f32);
+    J.item_end = items;
+    J.A = q.AT;
+    J.B = q.B;
+    J.codesA = B.codes.as<uint32_t>() + B.off_codesA[(size_t)order[k]];
+    J.codesB = B.codes.as<uint32_t>() + B.off_codesB[(size_t)order[k]];
+    J.p = q.p;
+    at_work.push_back(work);
+    at_list.push_back(lists);
+    work += need;
+    most = std::max(most, work);
+    lists += product_list_bytes(J);
+    B.pjobs.push_back(J);
+    B.pruns.back().second = (int)k + 1;
+  }
+  B.pmem = DevBuf(most, s);
+  B.plists = DevBuf(lists, s);
+  B.pdev = DevBuf(B.pjobs.size() * sizeof(ProdJob), s);
+  B.pflags = DevBuf(B.pjobs.size() * sizeof(int), s);
+  for (size_t k = 0; k < order.size(); ++k) {
+    ProdJob& J = B.pjobs[k];
+    product_set_work(J, B.pmem.as<uint8_t>() + at_work[k], B.f32, B.prods[(size_t)order[k]].C);
+    product_set_lists(J, B.plists.as<uint8_t>() + at_list[k]);
+    J.flag = B.pflags.as<int>() + k;
+  }
+  CMM_CUDA(cudaMemcpyAsync(B.pdev.ptr, B.pjobs.data(), B.pdev.bytes, cudaMemcpyHostToDevice, s));
+  launch_product_index(B.pjobs.data(), B.pdev.as<ProdJob>(), (int)B.pjobs.size(), s);
 }
 
 // Times the candidate (slab length, radix) pairs of product i on its own
@@ -970,6 +1043,14 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   B->ctas = f32 ? resident_ctas<float>() : resident_ctas<double>();
   B->tw4096 = twiddles(1 << kBFftLog, s);
 
+  // ---- products whose sketch is taken from the product itself
+  B->by_product.assign((size_t)count, 0);
+  for (int i = 0; i < count; ++i) {
+    const cmm_batch_product& q = B->prods[(size_t)i];
+    B->by_product[(size_t)i] = q.n_inner <= kProdMaxK && product_supported(q.b, q.n_a, q.n_inner, q.n_b) &&
+                               product_faster(q.variant, f32, q.d, q.b, q.n_a, q.n_inner, q.n_b, false);
+  }
+
   // ---- validation, hash parameters, buffer offsets
   std::vector<uint8_t> blob;
   std::vector<size_t> off_params((size_t)count), fn_bytes((size_t)count);
@@ -1027,7 +1108,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
     const int log2b = B->plans[(size_t)i].log2b;
     hj.push_back({base, base + 2 * set, B->codes.as<uint32_t>() + B->off_codesA[(size_t)i], q.n_a, q.d, log2b, q.hash_kind});
     hj.push_back({base + set, base + 3 * set, B->codes.as<uint32_t>() + B->off_codesB[(size_t)i], q.n_b, q.d, log2b, q.hash_kind});
-    if (q.variant == kVariantFFT && q.n_inner > 0)
+    if (q.variant == kVariantFFT && q.n_inner > 0 && !B->by_product[(size_t)i])
       sj.push_back({q.AT, q.B, B->scale.as<int>() + B->off_scale[(size_t)i], q.n_a, q.n_inner, q.n_b});
   }
   B->n_scale_jobs = (int)sj.size();
@@ -1042,9 +1123,15 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   launch_hash_codes_jobs(B->hjobs.as<HashJob>(), 2 * count, B->max_hash_total, s);
   enqueue_scale(*B, s);
 
+  make_product_jobs(*B, s);
+
   // ---- per-class configuration (autotuned, cached)
   for (int i = 0; i < count; ++i) {
     const cmm_batch_product& q = B->prods[(size_t)i];
+    if (B->by_product[(size_t)i]) {  // nothing to choose
+      B->tuned[(size_t)i] = tune ? 1 : 0;
+      continue;
+    }
     SketchPlan& P = B->plans[(size_t)i];
     const TuneKey key{q.variant, (int)f32, P.log2b, ilog2c(std::max<int64_t>(q.n_a + q.n_b, 1))};
     TuneVal v{P.logL, 8, 1};
@@ -1071,7 +1158,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   for (int i = 0; i < count; ++i) {
     const cmm_batch_product& q = B->prods[(size_t)i];
     const SketchPlan& P = B->plans[(size_t)i];
-    total += (double)q.n_inner * P.R * q.d * unit_cost(q, P.logL);
+    if (!B->by_product[(size_t)i]) total += (double)q.n_inner * P.R * q.d * unit_cost(q, P.logL);
   }
   const double target = std::max(total / ((double)B->ctas * 6.0), 1.0);
   size_t npart = 0;
@@ -1080,6 +1167,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   for (int i = 0; i < count; ++i) {
     const cmm_batch_product& q = B->prods[(size_t)i];
     SketchPlan& P = B->plans[(size_t)i];
+    if (B->by_product[(size_t)i]) continue;
     const double row = unit_cost(q, P.logL);
     int64_t G = (int64_t)std::ceil((double)q.n_inner * row / target);
     const int64_t gmin = std::max<int64_t>(1, q.n_inner / 8);  // at least 8 rows per item
@@ -1104,11 +1192,16 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   B->partial = DevBuf(std::max<size_t>(npart, 256), s);
   CMM_CUDA(cudaMemsetAsync(B->partial.ptr, 0, std::max<size_t>(npart, 256), s));
   size_t work = 16;
-  for (int i = 0; i < count; ++i) work = std::max(work, 2 * (size_t)B->prods[(size_t)i].d * (size_t)B->prods[(size_t)i].b * 16);
+  for (int i = 0; i < count; ++i)
+    if (!B->by_product[(size_t)i]) work = std::max(work, 2 * (size_t)B->prods[(size_t)i].d * (size_t)B->prods[(size_t)i].b * 16);
   B->work = DevBuf(work, s);
   std::vector<BProd> bp;
   B->splans.resize((size_t)count);
   for (int i = 0; i < count; ++i) {
+    if (B->by_product[(size_t)i]) {
+      bp.push_back(BProd{});  // (items refer to products by their place)
+      continue;
+    }
     B->splans[(size_t)i] = make_sorted(*B, i, B->plans[(size_t)i].logL, s);
     bp.push_back(make_bprod(*B, i, B->partial.as<unsigned char>() + B->off_partial[(size_t)i], B->splans[(size_t)i]));
   }
@@ -1117,7 +1210,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   std::vector<FinJob> fj;
   for (int i = 0; i < count; ++i) {
     const SketchPlan& P = B->plans[(size_t)i];
-    if (!batch_finalize_fits(P.log2b)) continue;
+    if (B->by_product[(size_t)i] || !batch_finalize_fits(P.log2b)) continue;
     for (int t = 0; t < P.d; ++t)
       fj.push_back({B->partial.as<unsigned char>() + B->off_partial[(size_t)i], B->prods[(size_t)i].p, B->tw[(size_t)i],
                     P.G, P.d, t, P.log2b, P.logL, P.variant});
@@ -1136,6 +1229,8 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
 
 void batch_run(BatchPlan* B, cudaStream_t user) {
   if (!B) throw invalid_argument("batch handle is null");
+  if (!B->pjobs.empty() && product_timed_out())
+    throw runtime_error("product sketch: a wait ran out in an earlier launch");
   cudaStream_t s = user ? user : B->stream;
   if (!B->exec) {
     // capture once: the sequence depends only on the plan
@@ -1168,15 +1263,19 @@ void batch_run(BatchPlan* B, cudaStream_t user) {
 
 void batch_info(const BatchPlan* B, int64_t* items, int* ctas, int* launches) {
   if (!B) throw invalid_argument("batch handle is null");
-  if (items) *items = B->n_items;
-  if (ctas) *ctas = B->ctas;
+  int64_t n_prod = 0;
+  for (const auto& run : B->pruns) n_prod += B->pjobs[(size_t)run.second - 1].item_end;
+  if (items) *items = B->n_items + n_prod;
+  if (ctas) *ctas = std::max(B->n_items ? B->ctas : 0, (int)std::min<int64_t>(2 * n_prod, num_sms()));
   if (launches) {
     // kernels per run: scale (if any), sketch (if any), the batched finalize,
-    // 3 per other finalize, 1 per dense C
+    // 3 per other finalize, the product sketches' kernels, 1 per dense C
     int n = (B->n_scale_jobs ? 1 : 0) + (B->n_items ? 1 : 0) + (B->n_fjobs ? 1 : 0);
+    for (const auto& run : B->pruns)
+      n += product_launches(B->pjobs.data() + run.first, run.second - run.first);
     for (size_t i = 0; i < B->prods.size(); ++i) {
       const auto& q = B->prods[i];
-      n += (batch_finalize_fits(B->plans[i].log2b) ? 0 : 3) + (q.C && q.n_a > 0 && q.n_b > 0 ? 1 : 0);
+      n += (B->by_product[i] || batch_finalize_fits(B->plans[i].log2b) ? 0 : 3) + (q.C && q.n_a > 0 && q.n_b > 0 ? 1 : 0);
     }
     *launches = n;
   }

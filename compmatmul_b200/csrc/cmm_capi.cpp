@@ -325,29 +325,17 @@ static int64_t chunk_len(int64_t k0, int64_t kc, int64_t n_inner, const RowFeed*
 }
 
 // The sketch through the product C itself (cmm_product.cu), when that is
-// estimated to be faster than the transforms.  Both estimates are fits to B200
-// times (microseconds), n square, d = 7, transforms / product:
-//   n = 512:  b = 256 119 / 187, 1024 228 / 155, 4096 387 / 157, 2^16 3380 / 236
-//   n = 2048: b = 256 413 / 517, 1024 770 / 593, 4096 1239 / 658, 2^16 12778 / 689
-//   n = 8192, 32 inner indices, b = 256, d = 3: 408 / 3368 (the product pays
-//   d additions per entry of C however few inner indices there are)
-// Where the group kernels apply, products under 2^24 multiply-adds stay with
-// them: both take a few hundred microseconds there, and those kernels' tests,
-// which check that they ran, use such sizes.
+// estimated to be faster.  Where the group kernels apply, products under 2^24
+// multiply-adds stay with them: both take a few hundred microseconds there, and
+// those kernels' tests, which check that they ran, use such sizes.
 static bool product_applicable(int variant, bool f32, const SketchParams& sp, int64_t n_a, int64_t n_inner,
                                int64_t n_b) {
-  if (n_inner <= 0 || n_a <= 0 || n_b <= 0) return false;
-  if (n_a > 0x7fffffff || n_b > 0x7fffffff || n_a * n_b > kProdMaxEntries) return false;
-  if (sp.b < 512 || (sp.b > 65536 && n_b > 131072)) return false;  // the forms of the additions (cmm_product_add.cu)
+  if (!product_supported(sp.b, n_a, n_inner, n_b)) return false;
   if (sketch_kernel_choice() == 3) return true;
   if (sketch_kernel_choice() != 0) return false;
-  const double nn = (double)n_a * (double)n_b, k = (double)n_inner, d = sp.d, b = sp.b;
-  if (sketch_cluster_applicable(variant, f32, sp.b) && nn * k < 16777216.0) return false;
-  const bool small_b = variant == kVariantFFT ? sp.b < 4096 : sp.b < 8192;
-  const double per_b = variant == kVariantFFT && !f32 ? 0.85e-6 : 0.5e-6;
-  const double transforms = (small_b ? 70.0 : 230.0) + d * k * (per_b * b * sp.log2b + 7e-6 * (double)(n_a + n_b));
-  const double product = 110.0 + nn * (d / 1.1e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
-  return product < transforms;
+  if (sketch_cluster_applicable(variant, f32, sp.b) && (double)n_a * (double)n_b * (double)n_inner < 16777216.0)
+    return false;
+  return product_faster(variant, f32, sp.d, sp.b, n_a, n_inner, n_b, true);
 }
 
 // scratch: n_a x n_b doubles for C (the caller's dense output, written
@@ -359,56 +347,27 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   if (product_timed_out()) throw std::runtime_error("product sketch: a wait ran out in an earlier launch");
   const size_t elem = f32 ? 4 : 8;
   ProdJob J{};
-  J.n_a = n_a;
-  J.n_b = n_b;
-  J.tiles_a = prod_tiles(n_a);
-  J.tiles_b = prod_tiles(n_b);
+  product_geometry(J, variant, sp.d, sp.b, n_a, n_b, 1, true, num_sms());
+  // inner indices per chunk: planes within the budget; rows still arriving
+  // from the host: eighths, so that copies and work overlap
   const size_t per_k = (size_t)prod_moduli(f32) * 256 * (size_t)(J.tiles_a + J.tiles_b);
   int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget() / per_k));
-  // rows still arriving from the host: eighths, so that copies and work overlap
   if (feed) kc = std::min<int64_t>(kc, std::max<int64_t>((n_inner + 7) / 8, 512));
   kc = std::max<int64_t>(kc / 128 * 128, 128);
   kc = std::min<int64_t>(kc, n_inner);
   // panels of C whose residues take at most 2 GiB
-  const size_t per_tile = prod_residue_bytes(1, J.tiles_b, f32);
-  const int panel = (int)std::max<int64_t>(1, std::min<int64_t>(J.tiles_a, (int64_t)(((size_t)2 << 30) / per_tile)));
+  const int panel = (int)std::max<int64_t>(1, std::min<int64_t>(J.tiles_a, (int64_t)(((size_t)2 << 30) / prod_residue_row(J, f32))));
+  J.kc = kc;
+  J.tiles_p = panel;
+  const size_t work = product_work_bytes(J, f32, !product_usable_c(J, scratch)), lists = product_list_bytes(J);
+  DevBuf mem(work + lists + sizeof(ProdJob), s);  // one allocation for everything
+  uint8_t* base = mem.as<uint8_t>();
+  product_set_work(J, base, f32, scratch);
+  product_set_lists(J, base + work);
+  ProdJob* dJ = reinterpret_cast<ProdJob*>(base + work + lists);
   J.codesA = codes.a.as<uint32_t>();
   J.codesB = codes.b.as<uint32_t>();
-  J.d = sp.d;
-  J.log2b = sp.log2b;
-  J.variant = variant;
-  plan_product_sketch(J, num_sms());
-  const size_t db = (size_t)sp.d * (size_t)sp.b;
-  // one allocation for everything
-  size_t total = 0;
-  auto take = [&](size_t n) { const size_t o = total; total += (n + 255) & ~(size_t)255; return o; };
-  const size_t nb = (size_t)((kc + 255) / 256);
-  const size_t o_slA = take(prod_plane_bytes(n_a, kc, f32)), o_slB = take(prod_plane_bytes(n_b, kc, f32));
-  const size_t o_res = take(per_tile * panel), o_exp = take((size_t)(n_a + n_b + kc + 1) * 4);
-  const size_t o_csum = take(nb * (size_t)(n_a + n_b) * 8), o_cmax = take(nb * (size_t)(n_a + n_b) * 4);
-  J.ldc = prod_ldc(n_b);
-  if (J.ldc != n_b || reinterpret_cast<uintptr_t>(scratch) % 16) scratch = nullptr;  // rows must be 16-byte aligned
-  const size_t o_C = take(scratch ? 0 : (size_t)n_a * (size_t)J.ldc * 8);
-  const size_t o_cum = take(prod_cum_bytes(J)), o_ent = take(2 * (size_t)sp.d * (size_t)n_b * 4);
-  const size_t o_part = take((size_t)J.G * db * 8), o_job = take(sizeof(ProdJob));
-  DevBuf mem(total, s);
-  uint8_t* base = mem.as<uint8_t>();
-  J.slA = base + o_slA;
-  J.slB = base + o_slB;
-  J.res = reinterpret_cast<uint32_t*>(base + o_res);
-  J.flag = reinterpret_cast<int*>(base + o_exp);
-  J.cexpA = J.flag + 1;
-  J.cexpB = J.cexpA + n_a;
-  J.rexp = J.cexpB + n_b;
-  J.csum = reinterpret_cast<double*>(base + o_csum);
-  J.cmax = reinterpret_cast<int*>(base + o_cmax);
-  J.C = scratch ? scratch : reinterpret_cast<double*>(base + o_C);
-  J.cum = base + o_cum;
-  J.ent = reinterpret_cast<uint32_t*>(base + o_ent);
-  J.part = reinterpret_cast<double*>(base + o_part);
   J.p = dP;
-  ProdJob* dJ = reinterpret_cast<ProdJob*>(base + o_job);
-  auto send = [&] { CMM_CUDA(cudaMemcpyAsync(dJ, &J, sizeof(J), cudaMemcpyHostToDevice, s)); };
   for (int64_t k0 = 0; k0 < n_inner; k0 += kc) {
     J.kc = std::min<int64_t>(kc, n_inner - k0);
     J.A = static_cast<const char*>(dAT) + (size_t)k0 * n_a * elem;
@@ -417,7 +376,7 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
     for (J.tile0 = 0; J.tile0 < J.tiles_a; J.tile0 += panel) {
       J.tiles_p = std::min(panel, J.tiles_a - J.tile0);
       J.item_end = (int64_t)J.tiles_p * J.tiles_b * prod_moduli(f32);
-      send();
+      CMM_CUDA(cudaMemcpyAsync(dJ, &J, sizeof(J), cudaMemcpyHostToDevice, s));
       if (J.tile0 == 0) {
         if (k0 == 0) launch_product_index(&J, dJ, 1, s);
         if (feed) feed->wait(k0, J.kc, s);

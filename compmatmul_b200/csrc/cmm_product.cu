@@ -695,10 +695,30 @@ void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, 
     rows = std::max<int64_t>(rows, (int64_t)hJobs[i].tiles_p * 64);
   }
   count_launch();
-  const dim3 g((unsigned)((n_b + 255) / 256), (unsigned)std::min<int64_t>(rows, 4096), (unsigned)count);
+  const unsigned gx = (unsigned)((n_b + 255) / 256);
+  const int64_t gy = std::max<int64_t>(1, std::min<int64_t>(rows, 32768 / ((int64_t)gx * count)));
+  const dim3 g(gx, (unsigned)gy, (unsigned)count);
   if (f32) k_prod_crt<float><<<g, 256, 0, s>>>(dJobs);
   else k_prod_crt<double><<<g, 256, 0, s>>>(dJobs);
   CMM_CUDA(cudaGetLastError());
+}
+
+// Estimates in microseconds, fitted to B200 times.  Single calls, n square, d =
+// 7, transforms / product:
+//   n = 512:  b = 256 119 / 187, 1024 228 / 155, 4096 387 / 157, 2^16 3380 / 236
+//   n = 2048: b = 256 413 / 517, 1024 770 / 593, 4096 1239 / 658, 2^16 12778 / 689
+//   n = 8192, 32 inner indices, b = 256, d = 3: 408 / 3368 (the product pays
+//   d additions per entry of C however few inner indices there are)
+bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone) {
+  const double nn = (double)n_a * (double)n_b, k = (double)n_inner;
+  const bool small_b = variant == kVariantFFT ? b < 4096 : b < 8192;
+  const double per_b = variant == kVariantFFT && !f32 ? 0.85e-6 : 0.5e-6;
+  double log2b = 0;
+  while ((1 << (int)log2b) < b) ++log2b;
+  const double transforms = (alone ? (small_b ? 70.0 : 230.0) : 0.0) +
+                            d * k * (per_b * b * log2b + 7e-6 * (double)(n_a + n_b));
+  const double product = (alone ? 110.0 : 5.0) + nn * (d / 1.8e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
+  return product < transforms;
 }
 
 }  // namespace cmm

@@ -44,29 +44,40 @@ struct ProdJob {
 };
 
 inline int prod_moduli(bool f32) { return f32 ? 8 : 15; }
-inline int prod_tiles(int64_t n) { return (int)((n + 255) / 256); }
-// residue planes of n columns x kc inner indices; residues of a panel
-inline size_t prod_plane_bytes(int64_t n, int64_t kc, bool f32) {
-  return (size_t)prod_moduli(f32) * 2 * prod_tiles(n) * prod_ksteps(kc) * kProdSlab;
-}
-inline size_t prod_residue_bytes(int tiles_p, int tiles_b, bool f32) {
-  return (size_t)prod_moduli(f32) * 65536 * tiles_p * tiles_b;
-}
-
-// geometry of the additions of a job from its sizes (form, logW, G, blocks)
-void plan_product_sketch(ProdJob& J, int sms);
-size_t prod_cum_bytes(const ProdJob& J);
 // C's row stride: even, so that rows can be copied in 16-byte units
 inline int64_t prod_ldc(int64_t n_b) { return (n_b + 1) & ~(int64_t)1; }
+// bytes of the residues of one output tile row (256 columns of A)
+inline size_t prod_residue_row(const ProdJob& J, bool f32) { return (size_t)prod_moduli(f32) * 65536 * J.tiles_b; }
 // the largest n_a n_b whose product is formed (8 GiB of FP64)
 constexpr int64_t kProdMaxEntries = (int64_t)1 << 30;
 
-// hJobs: the host copy of dJobs.  Sorted columns (also clears the flags);
-// exponents and residue planes; the product; the additions and their sum.
+// Whether the product sketch takes these sizes, and whether it is estimated to
+// be faster than the transforms (alone: with both forms' fixed costs).
+bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b);
+bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone);
+
+// Sizes, tiles and additions of a job of kc inner indices (kc <= kProdMaxK)
+// with all rows of C in one panel.  alone: the job has the device for itself
+// (row groups to fill it); otherwise the row groups follow from the job's
+// sizes only, so that it computes the same among any others.
+void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_t n_b, int64_t kc, bool alone, int sms);
+// Device memory of a job: the sorted columns (they depend on the hash codes
+// only), and the work space for J.kc inner indices and J.tiles_p tiles; with
+// C in it, or in the caller's n_a x n_b doubles where those are usable.
+size_t product_list_bytes(const ProdJob& J);
+void product_set_lists(ProdJob& J, void* base);
+bool product_usable_c(const ProdJob& J, const double* c);
+size_t product_work_bytes(const ProdJob& J, bool f32, bool own_c);
+void product_set_work(ProdJob& J, void* base, bool f32, double* c);
+
+// hJobs: the host copy of dJobs, item_end set.  Sorted columns (also clears
+// the flags); exponents and residue planes; the product; the additions.
 void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
 void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
 void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
 void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
+// kernels of one planes + product + additions sequence
+int product_launches(const ProdJob* hJobs, int count);
 // host-mapped flag set by a wait of these kernels that ran out (*dev: its device address)
 int* product_timeout_flag(int** dev);
 // true (and cleared) when such a wait ran out since the last call

@@ -535,34 +535,111 @@ __global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__
 
 }  // namespace
 
-void plan_product_sketch(ProdJob& J, int sms) {
-  const int64_t b = (int64_t)1 << J.log2b;
-  const int64_t cols = std::max<int64_t>(std::min<int64_t>(J.n_b, kScCols), 1);
-  J.blocks = (int)((J.n_b + kScCols - 1) / kScCols);
+bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
+  return n_inner > 0 && n_a > 0 && n_b > 0 && n_a <= 0x7fffffff && n_b <= 0x7fffffff && n_a * n_b <= kProdMaxEntries &&
+         b >= 512 && (b <= 65536 || n_b <= 131072);  // what the forms of the additions take
+}
+
+void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_t n_b, int64_t kc, bool alone, int sms) {
+  J.variant = variant;
+  J.d = d;
+  J.n_a = n_a;
+  J.n_b = n_b;
+  J.kc = kc;
+  J.ldc = prod_ldc(n_b);
+  J.tiles_a = J.tiles_p = (int)((n_a + 255) / 256);
+  J.tiles_b = (int)((n_b + 255) / 256);
+  J.tile0 = 0;
+  J.accumulate = 0;
+  J.log2b = 0;
+  while ((1 << J.log2b) < b) ++J.log2b;
+  const int64_t cols = std::max<int64_t>(std::min<int64_t>(n_b, kScCols), 1);
+  J.blocks = (int)((n_b + kScCols - 1) / kScCols);
   J.form = J.log2b > 16 ? kAddGather : (cols >= b ? kAddLane : kAddStaged);
   // windows: 36 to 72 entries of a row, at most 1024 buckets (8 KB of shared memory a warp)
-  const int64_t per_row = J.form == kAddGather ? std::max<int64_t>(J.n_b, 1) : cols;
+  const int64_t per_row = J.form == kAddGather ? std::max<int64_t>(n_b, 1) : cols;
   J.logW = 5;
-  while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 72 * b) ++J.logW;
+  while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 72 * (int64_t)b) ++J.logW;
   J.logW = std::min(J.logW, J.log2b);
-  const int64_t wins = b >> J.logW;
+  const int64_t wins = (int64_t)b >> J.logW, most = std::min<int64_t>((n_a + 31) / 32, 512);
+  int64_t G;
   if (J.form == kAddGather) {
     // Row groups of at most 32 MB of C: the CTAs in flight then work on about
     // two groups, which stay in L2.  (16384 rows of 16384 columns, b = 2^18: 60
-    // ms in 3 groups, whose CTAs drift apart and miss L2.)
+    // ms in 3 groups, whose CTAs drift apart and miss L2; 11.6 ms in 64.)
     const int64_t rows = std::max<int64_t>(32, ((int64_t)32 << 20) / (8 * per_row));
-    const int64_t fill = 12 * (int64_t)sms / (J.d * ((wins + kGaWarps - 1) / kGaWarps));
-    J.G = (int)std::max<int64_t>(1, std::min<int64_t>({std::max((J.n_a + rows - 1) / rows, fill), (J.n_a + 31) / 32, 512}));
-    return;
+    const int64_t fill = alone ? 12 * (int64_t)sms / (d * ((wins + kGaWarps - 1) / kGaWarps)) : 0;
+    G = std::max((n_a + rows - 1) / rows, fill);
+  } else {
+    // one CTA per SM; among other jobs 512 rows, which outweigh a CTA's start and end
+    const int64_t ctas = J.form == kAddLane ? d : d * ((wins + kScWin - 1) / kScWin);
+    G = alone ? std::min<int64_t>(sms / ctas, 64) : (n_a + 511) / 512;
   }
-  // one CTA per SM
-  const int64_t ctas = J.form == kAddLane ? J.d : J.d * ((wins + kScWin - 1) / kScWin);
-  J.G = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sms / ctas, (J.n_a + 31) / 32, 64}));
+  J.G = (int)std::max<int64_t>(1, std::min(G, most));
 }
 
-size_t prod_cum_bytes(const ProdJob& J) {
+// --------------------------------------------------------------- device memory
+namespace {
+size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+size_t cum_bytes(const ProdJob& J) {
   return J.form == kAddGather ? (size_t)J.d * (((size_t)1 << J.log2b) + 1) * 4
                               : (size_t)J.d * J.blocks * cum16_stride(J.log2b) * 2;
+}
+// residue planes of n columns (in tiles of 256)
+size_t plane_bytes(int tiles, int64_t kc, bool f32) {
+  return (size_t)prod_moduli(f32) * 2 * tiles * prod_ksteps(kc) * kProdSlab;
+}
+// visits the parts of the work space in order
+template <typename F>
+void work_parts(const ProdJob& J, bool f32, bool own_c, F&& part) {
+  const size_t n = (size_t)(J.n_a + J.n_b), nb = (size_t)((J.kc + 255) / 256);
+  part(0, plane_bytes(J.tiles_a, J.kc, f32));
+  part(1, plane_bytes(J.tiles_b, J.kc, f32));
+  part(2, prod_residue_row(J, f32) * J.tiles_p);
+  part(3, (n + (size_t)J.kc + 1) * 4);
+  part(4, nb * n * 8);
+  part(5, nb * n * 4);
+  part(6, (size_t)J.G * ((size_t)J.d << J.log2b) * 8);
+  if (own_c) part(7, (size_t)J.n_a * (size_t)J.ldc * 8);
+}
+}  // namespace
+
+size_t product_list_bytes(const ProdJob& J) { return up256(cum_bytes(J)) + up256(2 * (size_t)J.d * (size_t)J.n_b * 4); }
+void product_set_lists(ProdJob& J, void* base) {
+  J.cum = base;
+  J.ent = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(base) + up256(cum_bytes(J)));
+}
+// (rows are copied in 16-byte units)
+bool product_usable_c(const ProdJob& J, const double* c) {
+  return c && J.ldc == J.n_b && reinterpret_cast<uintptr_t>(c) % 16 == 0;
+}
+size_t product_work_bytes(const ProdJob& J, bool f32, bool own_c) {
+  size_t total = 0;
+  work_parts(J, f32, own_c, [&](int, size_t n) { total += up256(n); });
+  return total;
+}
+void product_set_work(ProdJob& J, void* base, bool f32, double* c) {
+  const bool own_c = !product_usable_c(J, c);
+  J.C = c;
+  uint8_t* at = static_cast<uint8_t*>(base);
+  work_parts(J, f32, own_c, [&](int i, size_t n) {
+    switch (i) {
+      case 0: J.slA = at; break;
+      case 1: J.slB = at; break;
+      case 2: J.res = reinterpret_cast<uint32_t*>(at); break;
+      case 3:
+        J.flag = reinterpret_cast<int*>(at);
+        J.cexpA = J.flag + 1;
+        J.cexpB = J.cexpA + J.n_a;
+        J.rexp = J.cexpB + J.n_b;
+        break;
+      case 4: J.csum = reinterpret_cast<double*>(at); break;
+      case 5: J.cmax = reinterpret_cast<int*>(at); break;
+      case 6: J.part = reinterpret_cast<double*>(at); break;
+      default: J.C = reinterpret_cast<double*>(at);
+    }
+    at += up256(n);
+  });
 }
 
 void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
@@ -584,6 +661,19 @@ void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count,
     k_prod_index_blocks<<<dim3((unsigned)d[1], (unsigned)blocks, (unsigned)count), kIdxThreads, 0, s>>>(dJobs);
     CMM_CUDA(cudaGetLastError());
   }
+}
+
+int product_launches(const ProdJob* hJobs, int count) {
+  bool used[2][6] = {}, cexp = false;  // additions: [variant][gather, staged, lane of b = 512 .. 4096]
+  for (int i = 0; i < count; ++i) {
+    const ProdJob& J = hJobs[i];
+    used[J.variant][J.form == kAddLane ? J.log2b - 7 : J.form] = true;
+    cexp |= J.kc > 256;
+  }
+  int n = 2 + (cexp ? 1 : 0) + 2 + 2 + 1;  // rows, columns, (their sums), planes, product, residues -> C, sums
+  for (auto& v : used)
+    for (bool u : v) n += u ? 1 : 0;
+  return n;
 }
 
 namespace {
