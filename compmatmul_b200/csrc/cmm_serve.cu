@@ -8,7 +8,9 @@
 // requests that are not yet running -- at most max_wave of them -- form a
 // wave: one persistent k_batch_sketch launch over all of their work items,
 // then each request's k-group reduction + inverse and the copy of its
-// sketch to pinned staging.  Waves on different streams overlap on the
+// sketch to pinned staging.  Requests for which the product sketch is
+// estimated to be faster go through its launches instead, all of a wave's
+// together.  Waves on different streams overlap on the
 // device, so requests that arrive while others run start as soon as memory
 // and a stream free up.  A finished wave releases its requests' memory and
 // copies each sketch to the caller's buffer.
@@ -32,6 +34,7 @@
 #include <vector>
 
 #include "cmm_batch.h"
+#include "cmm_product.h"
 
 namespace cmm {
 namespace {
@@ -69,7 +72,8 @@ class PinnedPool {
 // fixed by those alone, shared read-only by every request that has them
 struct CodePlan {
   DevBuf params, codes_a, codes_b;
-  SlabPlan plan;
+  SlabPlan plan;   // transform kernels
+  DevBuf lists;    // product sketch: sorted columns
   size_t bytes = 0;
 };
 using CodeKey = std::tuple<int, uint64_t, int, int, int64_t, int64_t, int>;
@@ -84,6 +88,8 @@ struct Request {
   std::string error;
   // device state (allocated on the upload stream at admission)
   DevBuf in_a, in_b, scale, partial, p_dev, work;
+  bool product = false;  // takes the product sketch (cmm_product.cu); `work` is its work space
+  ProdJob job{};
   std::shared_ptr<CodePlan> cp;  // codes + plan (cached or this request's own)
   SketchPlan sp{};
   const double2* tw = nullptr;
@@ -145,6 +151,21 @@ namespace {
 void geometry(Request& q, bool f32) {
   const cmm_request& r = q.r;
   q.log2b = ilog2i(r.b);
+  q.product = r.n_inner <= kProdMaxK && product_supported(r.b, r.n_a, r.n_inner, r.n_b) &&
+              product_faster(r.variant, f32, r.d, r.b, r.n_a, r.n_inner, r.n_b, false);
+  if (q.product) {
+    product_geometry(q.job, r.variant, r.d, r.b, r.n_a, r.n_b, r.n_inner, false, num_sms());
+    const size_t esz = f32 ? 4 : 8, d = (size_t)r.d;
+    size_t need = 0;
+    if (!r.inputs_on_device) need += round256(esz * (size_t)r.n_inner * (size_t)r.n_a) + round256(esz * (size_t)r.n_inner * (size_t)r.n_b);
+    need += round256(4 * hash_param_bytes(r.hash_kind) * d);
+    need += round256(4 * d * (size_t)r.n_a) + round256(4 * d * (size_t)r.n_b);
+    need += product_list_bytes(q.job) + round256(sizeof(ProdJob) + 16);
+    need += product_work_bytes(q.job, f32, true) + round256(d * (size_t)r.b * 8);
+    q.logL = -1;  // no slab: tells the cached lists of the two forms apart
+    q.need = need;
+    return;
+  }
   const int lmax = r.variant == kVariantFFT ? kBatchFftLog : kBatchWhtLog;
   int logL = std::min(q.log2b, lmax), radix = 8, tc = 1;
   int tl = 0, tr = 0, tt = 1;
@@ -228,10 +249,22 @@ void prepare(Server& S, Request& q) {
     cp->codes_b = DevBuf(4 * (size_t)r.d * (size_t)std::max<int64_t>(r.n_b, 1), s);
     launch_hash_codes(r.hash_kind, base, base + 2 * set, r.d, q.log2b, r.n_a, cp->codes_a.as<uint32_t>(), s);
     launch_hash_codes(r.hash_kind, base + set, base + 3 * set, r.d, q.log2b, r.n_b, cp->codes_b.as<uint32_t>(), s);
-    cp->plan = make_residue_plan(cp->codes_a.as<uint32_t>(), cp->codes_b.as<uint32_t>(), r.n_a, r.n_b, r.d, r.b,
-                                 q.logL, 0, s);
+    DevBuf job;  // of the sort only
+    if (q.product) {
+      cp->lists = DevBuf(product_list_bytes(q.job), s);
+      job = DevBuf(sizeof(ProdJob) + 16, s);
+      ProdJob J = q.job;
+      J.codesB = cp->codes_b.as<uint32_t>();
+      J.flag = reinterpret_cast<int*>(job.as<uint8_t>() + sizeof(ProdJob));
+      product_set_lists(J, cp->lists.ptr);
+      CMM_CUDA(cudaMemcpyAsync(job.ptr, &J, sizeof(J), cudaMemcpyHostToDevice, s));
+      launch_product_index(&J, job.as<ProdJob>(), 1, s);
+    } else {
+      cp->plan = make_residue_plan(cp->codes_a.as<uint32_t>(), cp->codes_b.as<uint32_t>(), r.n_a, r.n_b, r.d, r.b,
+                                   q.logL, 0, s);
+    }
     cp->bytes = cp->params.bytes + cp->codes_a.bytes + cp->codes_b.bytes + cp->plan.srcA.bytes + cp->plan.srcB.bytes +
-                cp->plan.codeA.bytes + cp->plan.codeB.bytes + cp->plan.countA.bytes + cp->plan.countB.bytes;
+                cp->plan.codeA.bytes + cp->plan.codeB.bytes + cp->plan.countA.bytes + cp->plan.countB.bytes + cp->lists.bytes;
     q.cp = cp;
     {
       std::lock_guard<std::mutex> g(S.mu);
@@ -249,6 +282,18 @@ void prepare(Server& S, Request& q) {
       S.cache_bytes += cp->bytes;
     }
   }
+  q.p_dev = DevBuf((size_t)r.d * (size_t)r.b * 8, s);
+  if (q.product) {
+    q.work = DevBuf(product_work_bytes(q.job, f32, true), s);
+    ProdJob& J = q.job;
+    J.A = AT;
+    J.B = B;
+    J.codesA = q.cp->codes_a.as<uint32_t>();
+    J.codesB = q.cp->codes_b.as<uint32_t>();
+    J.p = q.p_dev.as<double>();
+    product_set_lists(J, q.cp->lists.ptr);
+    product_set_work(J, q.work.ptr, f32, nullptr);
+  } else {
   q.scale = DevBuf(4 * (size_t)std::max<int64_t>(r.n_inner, 1), s);
   if (r.variant == kVariantFFT && r.n_inner > 0) {
     if (f32) launch_row_scale_f32((const float*)AT, (const float*)B, r.n_a, r.n_inner, r.n_b, q.scale.as<int>(), s);
@@ -256,9 +301,9 @@ void prepare(Server& S, Request& q) {
   }
   q.partial = DevBuf((size_t)q.G * r.d * (size_t)r.b * elem, s);
   CMM_CUDA(cudaMemsetAsync(q.partial.ptr, 0, q.partial.bytes, s));  // k-groups without rows stay zero
-  q.p_dev = DevBuf((size_t)r.d * (size_t)r.b * 8, s);
   q.work = DevBuf(2 * (size_t)r.d * (size_t)r.b * 16, s);
   q.tw = twiddles(r.b, s);
+  }
   q.r.AT = AT;  // device inputs from here on
   q.r.B = B;
   CMM_CUDA(cudaEventCreateWithFlags(&q.prepared, cudaEventDisableTiming));
@@ -304,9 +349,15 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   std::vector<BProd> prods;
   struct C { double c; BItem it; };
   std::vector<C> items;
+  std::vector<ProdJob> jobs;  // the requests that take the product sketch
   for (size_t i = 0; i < reqs.size(); ++i) {
     Request& q = *reqs[i];
     CMM_CUDA(cudaStreamWaitEvent(s, q.prepared, 0));
+    if (q.product) {
+      jobs.push_back(q.job);
+      prods.push_back(BProd{});  // (items refer to products by their place)
+      continue;
+    }
     prods.push_back(bprod(q));
     if (q.r.n_inner == 0) continue;
     const int64_t per = (q.r.n_inner + q.G - 1) / q.G;
@@ -321,13 +372,16 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   std::stable_sort(items.begin(), items.end(), [](const C& a, const C& b) { return a.c > b.c; });
   std::vector<FinJob> fin;  // one batched reduction + inverse for the small-b requests
   for (auto& qp : reqs)
-    if (batch_finalize_fits(qp->log2b))
+    if (!qp->product && batch_finalize_fits(qp->log2b))
       for (int t = 0; t < qp->r.d; ++t)
         fin.push_back({qp->partial.ptr, qp->p_dev.as<double>(), qp->tw, qp->G, qp->r.d, t, qp->log2b, qp->logL,
                        qp->r.variant});
   // one pinned staging block and one device table: products | items | finalize jobs
   const size_t pb = prods.size() * sizeof(BProd), ib = items.size() * sizeof(BItem), fb = fin.size() * sizeof(FinJob);
-  const size_t ioff = (pb + 15) & ~(size_t)15, foff = (ioff + ib + 15) & ~(size_t)15, total = foff + fb;
+  const size_t ioff = (pb + 15) & ~(size_t)15, foff = (ioff + ib + 15) & ~(size_t)15;
+  // and the product jobs (longest inner dimension first) with their flags
+  const size_t joff = (foff + fb + 15) & ~(size_t)15, loff = joff + jobs.size() * sizeof(ProdJob);
+  const size_t total = loff + jobs.size() * sizeof(int);
   W->host = S.pinned.get(std::max<size_t>(total, 16), &W->host_cls);
   unsigned char* hb = static_cast<unsigned char*>(W->host);
   std::memcpy(hb, prods.data(), pb);
@@ -335,6 +389,17 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   for (size_t i = 0; i < items.size(); ++i) hi[i] = items[i].it;
   if (fb) std::memcpy(hb + foff, fin.data(), fb);
   W->dprods = DevBuf(std::max<size_t>(total, 16), s);
+  if (!jobs.empty()) {
+    std::stable_sort(jobs.begin(), jobs.end(), [](const ProdJob& a, const ProdJob& b) { return a.kc > b.kc; });
+    int64_t n = 0;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      n += (int64_t)jobs[i].tiles_a * jobs[i].tiles_b * prod_moduli(S.cfg.f32 != 0);
+      jobs[i].item_end = n;
+      jobs[i].flag = reinterpret_cast<int*>(W->dprods.as<unsigned char>() + loff) + i;
+    }
+    std::memcpy(hb + joff, jobs.data(), jobs.size() * sizeof(ProdJob));
+    std::memset(hb + loff, 0, jobs.size() * sizeof(int));
+  }
   W->counter = DevBuf(sizeof(int), s);
   CMM_CUDA(cudaMemcpyAsync(W->dprods.ptr, hb, total, cudaMemcpyHostToDevice, s));
   unsigned char* db = W->dprods.as<unsigned char>();
@@ -342,9 +407,15 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   batch_launch_sketch(S.cfg.f32 != 0, reinterpret_cast<const BProd*>(db), reinterpret_cast<const BItem*>(db + ioff),
                       n_items, W->counter.as<int>(), S.tw4096, std::max(1, std::min(S.ctas, n_items)), s);
   batch_launch_finalize(reinterpret_cast<const FinJob*>(db + foff), (int)fin.size(), s);
+  if (!jobs.empty()) {
+    const ProdJob* dj = reinterpret_cast<const ProdJob*>(db + joff);
+    launch_product_planes(jobs.data(), dj, (int)jobs.size(), S.cfg.f32 != 0, s);
+    launch_product_gemm(jobs.data(), dj, (int)jobs.size(), S.cfg.f32 != 0, s);
+    launch_product_add(jobs.data(), dj, (int)jobs.size(), s);
+  }
   for (auto& qp : reqs) {
     Request& q = *qp;
-    if (!batch_finalize_fits(q.log2b)) launch_finalize(q.sp, q.partial.ptr, q.tw, q.work.ptr, q.p_dev.as<double>(), s);
+    if (!q.product && !batch_finalize_fits(q.log2b)) launch_finalize(q.sp, q.partial.ptr, q.tw, q.work.ptr, q.p_dev.as<double>(), s);
     CMM_CUDA(cudaMemcpyAsync(q.stage, q.p_dev.ptr, q.p_dev.bytes, cudaMemcpyDeviceToHost, s));
   }
   CMM_CUDA(cudaEventCreateWithFlags(&W->done, cudaEventDisableTiming));
@@ -360,6 +431,7 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
 }
 
 void finish_wave(Server& S, std::unique_ptr<Wave>& W) {
+  if (product_timed_out()) throw runtime_error("product sketch: a wait ran out");
   const auto now = Clock::now();
   for (auto& qp : W->reqs) {
     Request& q = *qp;
