@@ -895,7 +895,6 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
   const size_t budget = std::min<size_t>(free_b / 3, (size_t)8 << 30);
   size_t lists = 0, work = 0, most = 0;
   std::vector<size_t> at_work, at_list;
-  int64_t items = 0;
   for (size_t k = 0; k < order.size(); ++k) {
     const cmm_batch_product& q = B.prods[(size_t)order[k]];
     ProdJob J{};
@@ -904,10 +903,7 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
     if (B.pruns.empty() || work + need > budget) {
       B.pruns.push_back({(int)k, (int)k});
       work = 0;
-      items = 0;
     }
-    items += (int64_t)J.tiles_a * J.tiles_b * prod_moduli(B.f32);
-    J.item_end = items;
     J.A = q.AT;
     J.B = q.B;
     J.codesA = B.codes.as<uint32_t>() + B.off_codesA[(size_t)order[k]];
@@ -931,6 +927,7 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
     product_set_lists(J, B.plists.as<uint8_t>() + at_list[k]);
     J.flag = B.pflags.as<int>() + k;
   }
+  for (const auto& run : B.pruns) product_layout(B.pjobs.data() + run.first, run.second - run.first, B.f32);
   CMM_CUDA(cudaMemcpyAsync(B.pdev.ptr, B.pjobs.data(), B.pdev.bytes, cudaMemcpyHostToDevice, s));
   launch_product_index(B.pjobs.data(), B.pdev.as<ProdJob>(), (int)B.pjobs.size(), s);
 }

@@ -375,7 +375,7 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
     J.accumulate = k0 > 0 ? 1 : 0;
     for (J.tile0 = 0; J.tile0 < J.tiles_a; J.tile0 += panel) {
       J.tiles_p = std::min(panel, J.tiles_a - J.tile0);
-      J.item_end = (int64_t)J.tiles_p * J.tiles_b * prod_moduli(f32);
+      product_layout(&J, 1, f32);
       CMM_CUDA(cudaMemcpyAsync(dJ, &J, sizeof(J), cudaMemcpyHostToDevice, s));
       if (J.tile0 == 0) {
         if (k0 == 0) launch_product_index(&J, dJ, 1, s);

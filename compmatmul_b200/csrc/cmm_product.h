@@ -40,6 +40,8 @@ struct ProdJob {
   int d, log2b, variant;
   int form;               // which additions (plan_product_sketch)
   int logW, G;            // window of a warp, row groups
+  int per_sm;             // CTAs of the additions per SM
+  int add_begin, add_x;   // their first CTA in the launch of their kind, CTAs per (t, row group)
   int blocks;             // blocks of columns (staged and lane forms)
 };
 
@@ -70,7 +72,10 @@ bool product_usable_c(const ProdJob& J, const double* c);
 size_t product_work_bytes(const ProdJob& J, bool f32, bool own_c);
 void product_set_work(ProdJob& J, void* base, bool f32, double* c);
 
-// hJobs: the host copy of dJobs, item_end set.  Sorted columns (also clears
+// Places of the jobs of one launch in its work lists (item_end, add_begin).
+void product_layout(ProdJob* jobs, int count, bool f32);
+
+// hJobs: the host copy of dJobs, laid out.  Sorted columns (also clears
 // the flags); exponents and residue planes; the product; the additions.
 void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
 void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);

@@ -27,7 +27,7 @@ constexpr int kIdxThreads = 1024;
 constexpr int kScCols = 4096;  // columns per block of the staged and lane forms (12 bits of an entry)
 constexpr int kScWin = 16;     // windows (warps) per CTA of the staged form
 constexpr int kScThreads = 32 * (kScWin + 1);
-constexpr size_t kScSmemMax = 227 * 1024 - 1024;
+constexpr size_t kScSmemMax = 227 * 1024 - 1024, kScSmemHalf = 112 * 1024;
 constexpr int kGaWarps = 8;    // windows (warps) per CTA of the gather form
 
 // A sorted column, in the order in which the additions take it apart: rank |
@@ -192,6 +192,34 @@ __global__ void __launch_bounds__(kIdxThreads) k_prod_index(const ProdJob* __res
 }
 
 // ----------------------------------------------------------------- additions
+// The kernel of a job's additions: 0 gather, 1 and 2 staged (that many CTAs per
+// SM), 3 .. 6 lane with b = 512 .. 4096
+__host__ __device__ inline int add_class(const ProdJob& J) {
+  return J.form == kAddGather ? 0 : (J.form == kAddStaged ? J.per_sm : J.log2b - 6);
+}
+// Work of a CTA: the job of its class that covers blockIdx.x, and its window
+// group x, repetition t and row group g (x fastest: CTAs that run together
+// share rows).
+struct AddWork {
+  int job, x, t, g;
+};
+__device__ __forceinline__ AddWork add_work(const ProdJob* __restrict__ jobs, int count, int cls) {
+  __shared__ int s_job;
+  const int id = (int)blockIdx.x;
+  for (int j = threadIdx.x; j < count; j += blockDim.x)
+    if (add_class(jobs[j]) == cls && id >= jobs[j].add_begin && id - jobs[j].add_begin < jobs[j].add_x * jobs[j].d * jobs[j].G)
+      s_job = j;
+  __syncthreads();
+  AddWork w;
+  w.job = s_job;
+  const ProdJob& J = jobs[w.job];
+  const int e = id - J.add_begin, xt = J.add_x * J.d;
+  w.g = e / xt;
+  w.t = (e - w.g * xt) / J.add_x;
+  w.x = e - w.g * xt - w.t * J.add_x;
+  return w;
+}
+
 // A warp's look-up of 32 rows (one a lane): first entry, count and key of the
 // window in each row
 struct RowKeys {
@@ -275,18 +303,13 @@ __device__ __forceinline__ void produce_rows(const ProdJob& J, const RowRing& R,
 // copies the row blocks, warps 0-15 own a window each; the next row's entries
 // are read while a row is added.
 template <int VARIANT>
-__global__ void __launch_bounds__(kScThreads, 1) k_prod_add_staged(const ProdJob* __restrict__ jobs, int gmax,
-                                                                   uint32_t smem, int* __restrict__ timeout) {
+__device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, uint32_t smem, int* timeout) {
   extern __shared__ __align__(128) unsigned char ssm[];
   __shared__ uint64_t full[8], empty[8];
   __shared__ int s_abort;
-  const ProdJob& J = jobs[blockIdx.z / gmax];
-  const int g = blockIdx.z % gmax, t = blockIdx.y;
-  if (J.variant != VARIANT || J.form != kAddStaged || g >= J.G || t >= J.d) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t b = 1u << J.log2b, W = 1u << J.logW, wmask = (W - 1u) * 8u;
-  const uint32_t win0 = blockIdx.x * kScWin, wins = b >> J.logW;
-  if (win0 >= wins) return;
+  const uint32_t win0 = x * kScWin, wins = b >> J.logW;
   const int nw = (int)min((uint32_t)kScWin, wins - win0);
   double* acc0 = reinterpret_cast<double*>(ssm);
   const uint32_t acc_bytes = ((uint32_t)kScWin << J.logW) * 8u;
@@ -363,19 +386,24 @@ __global__ void __launch_bounds__(kScThreads, 1) k_prod_add_staged(const ProdJob
   }
 }
 
+template <int PER_SM>
+__global__ void __launch_bounds__(kScThreads, PER_SM) k_prod_add_staged(const ProdJob* __restrict__ jobs, int count,
+                                                                        uint32_t smem, int* __restrict__ timeout) {
+  const AddWork w = add_work(jobs, count, PER_SM);
+  const ProdJob& J = jobs[w.job];
+  if (J.variant == kVariantFFT) add_staged<kVariantFFT>(J, w.x, w.t, w.g, smem, timeout);
+  else add_staged<kVariantFWHT>(J, w.x, w.t, w.g, smem, timeout);
+}
+
 // Lane form: thread = NB buckets (sums in registers); for row i bucket m adds
 // the run of entries of h2 = m - h1(i) (FWHT: m ^ h1(i)).  The sorted columns
 // of the block and the rows are in shared memory.
 template <int VARIANT, int NB>
-__global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* __restrict__ jobs, int gmax,
-                                                                 uint32_t smem, int* __restrict__ timeout) {
+__device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t smem, int* timeout) {
   extern __shared__ __align__(128) unsigned char ssm[];
   __shared__ uint64_t full[8], empty[8];
   __shared__ int s_abort;
   constexpr uint32_t b = 512u * NB;
-  const ProdJob& J = jobs[blockIdx.z / gmax];
-  const int g = blockIdx.z % gmax, t = blockIdx.y;
-  if (J.variant != VARIANT || J.form != kAddLane || (1u << J.log2b) != b || g >= J.G || t >= J.d) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* es = reinterpret_cast<uint32_t*>(ssm);                         // kScCols entries
   uint16_t* cs = reinterpret_cast<uint16_t*>(ssm + kScCols * 4);           // b + 8 positions
@@ -450,18 +478,24 @@ __global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* 
   }
 }
 
+template <int NB>
+__global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* __restrict__ jobs, int count,
+                                                                 uint32_t smem, int* __restrict__ timeout) {
+  const AddWork w = add_work(jobs, count, NB == 1 ? 3 : (NB == 2 ? 4 : (NB == 4 ? 5 : 6)));
+  const ProdJob& J = jobs[w.job];
+  if (J.variant == kVariantFFT) add_lane<kVariantFFT, NB>(J, w.t, w.g, smem, timeout);
+  else add_lane<kVariantFWHT, NB>(J, w.t, w.g, smem, timeout);
+}
+
 // Gather form: windows as in the staged form, values from L2.  Entries are read
 // two rows ahead and values one row ahead of the additions, so a row's chain
 // of two L2 latencies overlaps the rows before it.
 template <int VARIANT>
-__global__ void __launch_bounds__(kGaWarps * 32) k_prod_add_gather(const ProdJob* __restrict__ jobs, int gmax) {
+__device__ __forceinline__ void add_gather(const ProdJob& J, int x, int t, int g) {
   extern __shared__ double sacc[];
-  const ProdJob& J = jobs[blockIdx.z / gmax];
-  const int g = blockIdx.z % gmax, t = blockIdx.y;
-  if (J.variant != VARIANT || J.form != kAddGather || g >= J.G || t >= J.d) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t b = 1u << J.log2b, W = 1u << J.logW, wmask = (W - 1u) * 8u;
-  const uint32_t m0 = (blockIdx.x * kGaWarps + warp) << J.logW;
+  const uint32_t m0 = (x * kGaWarps + warp) << J.logW;
   if (m0 >= b) return;
   double* acc = sacc + (size_t)warp * W;
   for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
@@ -521,6 +555,13 @@ __global__ void __launch_bounds__(kGaWarps * 32) k_prod_add_gather(const ProdJob
   for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
 }
 
+__global__ void __launch_bounds__(kGaWarps * 32) k_prod_add_gather(const ProdJob* __restrict__ jobs, int count) {
+  const AddWork w = add_work(jobs, count, 0);
+  const ProdJob& J = jobs[w.job];
+  if (J.variant == kVariantFFT) add_gather<kVariantFFT>(J, w.x, w.t, w.g);
+  else add_gather<kVariantFWHT>(J, w.x, w.t, w.g);
+}
+
 // p = sum of the row groups' partial sketches (NaN when the flag is set)
 __global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__ jobs) {
   const ProdJob& J = jobs[blockIdx.y];
@@ -538,6 +579,18 @@ __global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__
 bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
   return n_inner > 0 && n_a > 0 && n_b > 0 && n_a <= 0x7fffffff && n_b <= 0x7fffffff && n_a * n_b <= kProdMaxEntries &&
          b >= 512 && (b <= 65536 || n_b <= 131072);  // what the forms of the additions take
+}
+
+// Shared memory of a staged or lane CTA: its windows or lists and a ring of up
+// to eight row blocks; staged, where windows and three row blocks take no more
+// than half an SM, two CTAs share it (1.2 to 1.4 times as fast: 4000 x 2048, b =
+// 8192, d = 7 0.315 -> 0.252 ms).
+static size_t add_fixed(const ProdJob& J) {
+  return J.form == kAddStaged ? ((size_t)kScWin << J.logW) * 8 : (size_t)kScCols * 4 + ((size_t)2 << J.log2b) + 128;
+}
+static size_t add_row(const ProdJob& J) { return (((size_t)std::min<int64_t>(J.n_b, kScCols) + 15) & ~(size_t)15) * 8; }
+static size_t add_smem(const ProdJob& J) {
+  return std::min(add_fixed(J) + 8 * add_row(J), J.per_sm == 2 ? kScSmemHalf : kScSmemMax);
 }
 
 void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_t n_b, int64_t kc, bool alone, int sms) {
@@ -561,6 +614,7 @@ void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_
   J.logW = 5;
   while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 72 * (int64_t)b) ++J.logW;
   J.logW = std::min(J.logW, J.log2b);
+  J.per_sm = J.form == kAddStaged && add_fixed(J) + 3 * add_row(J) <= kScSmemHalf ? 2 : 1;
   const int64_t wins = (int64_t)b >> J.logW, most = std::min<int64_t>((n_a + 31) / 32, 512);
   int64_t G;
   if (J.form == kAddGather) {
@@ -571,9 +625,9 @@ void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_
     const int64_t fill = alone ? 12 * (int64_t)sms / (d * ((wins + kGaWarps - 1) / kGaWarps)) : 0;
     G = std::max((n_a + rows - 1) / rows, fill);
   } else {
-    // one CTA per SM; among other jobs 512 rows, which outweigh a CTA's start and end
+    // the CTAs that fit; among other jobs 512 rows, which outweigh a CTA's start and end
     const int64_t ctas = J.form == kAddLane ? d : d * ((wins + kScWin - 1) / kScWin);
-    G = alone ? std::min<int64_t>(sms / ctas, 64) : (n_a + 511) / 512;
+    G = alone ? std::min<int64_t>(J.per_sm * sms / ctas, 64) : (n_a + 511) / 512;
   }
   J.G = (int)std::max<int64_t>(1, std::min(G, most));
 }
@@ -664,64 +718,40 @@ void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count,
 }
 
 int product_launches(const ProdJob* hJobs, int count) {
-  bool used[2][6] = {}, cexp = false;  // additions: [variant][gather, staged, lane of b = 512 .. 4096]
+  bool used[7] = {}, cexp = false;
   for (int i = 0; i < count; ++i) {
-    const ProdJob& J = hJobs[i];
-    used[J.variant][J.form == kAddLane ? J.log2b - 7 : J.form] = true;
-    cexp |= J.kc > 256;
+    used[add_class(hJobs[i])] = true;
+    cexp |= hJobs[i].kc > 256;
   }
   int n = 2 + (cexp ? 1 : 0) + 2 + 2 + 1;  // rows, columns, (their sums), planes, product, residues -> C, sums
-  for (auto& v : used)
-    for (bool u : v) n += u ? 1 : 0;
+  for (bool u : used) n += u ? 1 : 0;
   return n;
+}
+
+void product_layout(ProdJob* jobs, int count, bool f32) {
+  int64_t items = 0, ctas[7] = {};
+  for (int i = 0; i < count; ++i) {
+    ProdJob& J = jobs[i];
+    items += (int64_t)J.tiles_p * J.tiles_b * prod_moduli(f32);
+    J.item_end = items;
+    const int64_t wins = ((int64_t)1 << J.log2b) >> J.logW;
+    J.add_x = J.form == kAddLane ? 1 : (int)((wins + (J.form == kAddStaged ? kScWin : kGaWarps) - 1) / (J.form == kAddStaged ? kScWin : kGaWarps));
+    int64_t& c = ctas[add_class(J)];
+    J.add_begin = (int)c;
+    c += (int64_t)J.add_x * J.d * J.G;
+    if (c > 0x7fffffff) throw unsupported("product sketch: too many work items");
+  }
 }
 
 namespace {
 
-// the jobs of one kernel: its grid and shared memory
-struct AddGrid {
-  int g = 0, d = 0;
-  int64_t x = 0;
-  size_t smem = 0;
-  void include(const ProdJob& J, int64_t ctas, size_t need) {
-    g = std::max(g, J.G);
-    d = std::max(d, J.d);
-    x = std::max(x, ctas);
-    smem = std::max(smem, need);
-  }
-  dim3 grid(int count) const { return dim3((unsigned)x, (unsigned)d, (unsigned)(g * count)); }
-};
-
 template <typename K, typename... A>
-void launch_add(K kernel, const AddGrid& G, int count, int threads, cudaStream_t s, A... args) {
-  if (!G.g) return;
-  CMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.smem));
+void launch_add(K kernel, int64_t ctas, size_t smem, int threads, cudaStream_t s, A... args) {
+  if (!ctas) return;
+  CMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   count_launch();
-  kernel<<<G.grid(count), threads, G.smem, s>>>(args...);
+  kernel<<<(unsigned)ctas, threads, smem, s>>>(args...);
   CMM_CUDA(cudaGetLastError());
-}
-
-template <int V>
-void launch_adds(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
-  AddGrid gather, staged, lane[4];  // lane: b = 512 .. 4096
-  for (int i = 0; i < count; ++i) {
-    const ProdJob& J = hJobs[i];
-    if (J.variant != V) continue;
-    const int64_t wins = ((int64_t)1 << J.log2b) >> J.logW;
-    const size_t rows = 8 * ((((size_t)std::min<int64_t>(J.n_b, kScCols) + 15) & ~(size_t)15) * 8);  // a ring of eight
-    if (J.form == kAddGather) gather.include(J, (wins + kGaWarps - 1) / kGaWarps, ((size_t)kGaWarps << J.logW) * 8);
-    else if (J.form == kAddStaged)
-      staged.include(J, (wins + kScWin - 1) / kScWin, std::min(((size_t)kScWin << J.logW) * 8 + rows, kScSmemMax));
-    else lane[J.log2b - 9].include(J, 1, std::min((size_t)kScCols * 4 + (2u << J.log2b) + 128 + rows, kScSmemMax));
-  }
-  int* flag = nullptr;
-  product_timeout_flag(&flag);
-  launch_add(k_prod_add_gather<V>, gather, count, kGaWarps * 32, s, dJobs, gather.g);
-  launch_add(k_prod_add_staged<V>, staged, count, kScThreads, s, dJobs, staged.g, (uint32_t)staged.smem, flag);
-  launch_add(k_prod_add_lane<V, 1>, lane[0], count, kScThreads, s, dJobs, lane[0].g, (uint32_t)lane[0].smem, flag);
-  launch_add(k_prod_add_lane<V, 2>, lane[1], count, kScThreads, s, dJobs, lane[1].g, (uint32_t)lane[1].smem, flag);
-  launch_add(k_prod_add_lane<V, 4>, lane[2], count, kScThreads, s, dJobs, lane[2].g, (uint32_t)lane[2].smem, flag);
-  launch_add(k_prod_add_lane<V, 8>, lane[3], count, kScThreads, s, dJobs, lane[3].g, (uint32_t)lane[3].smem, flag);
 }
 
 }  // namespace
@@ -729,8 +759,23 @@ void launch_adds(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStre
 void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
   if (count <= 0) return;
   ProfScope prof("finalize", s);
-  launch_adds<kVariantFFT>(hJobs, dJobs, count, s);
-  launch_adds<kVariantFWHT>(hJobs, dJobs, count, s);
+  int64_t ctas[7] = {};
+  size_t smem[7] = {};
+  for (int i = 0; i < count; ++i) {
+    const ProdJob& J = hJobs[i];
+    const int c = add_class(J);
+    ctas[c] += (int64_t)J.add_x * J.d * J.G;
+    smem[c] = std::max(smem[c], c == 0 ? ((size_t)kGaWarps << J.logW) * 8 : add_smem(J));
+  }
+  int* flag = nullptr;
+  product_timeout_flag(&flag);
+  launch_add(k_prod_add_gather, ctas[0], smem[0], kGaWarps * 32, s, dJobs, count);
+  launch_add(k_prod_add_staged<1>, ctas[1], smem[1], kScThreads, s, dJobs, count, (uint32_t)smem[1], flag);
+  launch_add(k_prod_add_staged<2>, ctas[2], smem[2], kScThreads, s, dJobs, count, (uint32_t)smem[2], flag);
+  launch_add(k_prod_add_lane<1>, ctas[3], smem[3], kScThreads, s, dJobs, count, (uint32_t)smem[3], flag);
+  launch_add(k_prod_add_lane<2>, ctas[4], smem[4], kScThreads, s, dJobs, count, (uint32_t)smem[4], flag);
+  launch_add(k_prod_add_lane<4>, ctas[5], smem[5], kScThreads, s, dJobs, count, (uint32_t)smem[5], flag);
+  launch_add(k_prod_add_lane<8>, ctas[6], smem[6], kScThreads, s, dJobs, count, (uint32_t)smem[6], flag);
   int64_t db = 0;
   for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
   count_launch();

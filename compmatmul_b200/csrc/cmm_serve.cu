@@ -391,12 +391,9 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   W->dprods = DevBuf(std::max<size_t>(total, 16), s);
   if (!jobs.empty()) {
     std::stable_sort(jobs.begin(), jobs.end(), [](const ProdJob& a, const ProdJob& b) { return a.kc > b.kc; });
-    int64_t n = 0;
-    for (size_t i = 0; i < jobs.size(); ++i) {
-      n += (int64_t)jobs[i].tiles_a * jobs[i].tiles_b * prod_moduli(S.cfg.f32 != 0);
-      jobs[i].item_end = n;
+    product_layout(jobs.data(), (int)jobs.size(), S.cfg.f32 != 0);
+    for (size_t i = 0; i < jobs.size(); ++i)
       jobs[i].flag = reinterpret_cast<int*>(W->dprods.as<unsigned char>() + loff) + i;
-    }
     std::memcpy(hb + joff, jobs.data(), jobs.size() * sizeof(ProdJob));
     std::memset(hb + loff, 0, jobs.size() * sizeof(int));
   }
