@@ -1,4 +1,4 @@
-// mbarrier and bulk-copy helpers of the product sketch kernels.
+// mbarrier and bulk-copy helpers of the product sketch and FWHT-of-rows kernels.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -29,12 +29,12 @@ __device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait (about a second of polls); gives up at once when another role
+// bounded wait (2^20 polls of 20 ns and more); gives up at once when another role
 // of the CTA has given up
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
   for (int it = 0; it < 64; ++it)
     if (bar_test(bar, parity)) return true;
-  for (uint32_t it = 0; it < (1u << 22); ++it) {
+  for (uint32_t it = 0; it < (1u << 20); ++it) {
     if (bar_test(bar, parity)) return true;
     if (*abort) return false;
     __nanosleep(20);

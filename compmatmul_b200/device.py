@@ -119,7 +119,7 @@ def wht_rows(x, method="tensor", out=None):
     """Forward natural-order Walsh-Hadamard transform of every row of a
     contiguous 2-D float32 CUDA tensor (rows of 2^11, 2^12 or 2^13), the
     reference's fwht_transformer::forward (transform.hpp:94-144) on FP32.
-    method "tensor": the Hadamard-16 stages as tcgen05 MMAs on BF16
+    method "tensor": a Hadamard-128 stage as tcgen05 MMAs on BF16
     hi/mid/lo splits; "cuda": every stage on CUDA cores.  out may be x
     (in place).  Returns once the rows are transformed."""
     import torch
