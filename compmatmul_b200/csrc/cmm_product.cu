@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) k_prod_rows(const ProdJob* __restrict__ j
 // squares and largest exponents go to csum / cmax (k_prod_cexp adds them up in
 // a fixed order; with one block of rows it is done here).  When the sum of
 // squares leaves the FP64 range, the bound from the largest entry serves.
-constexpr int kColRows = 256;
+constexpr int kColRows = kProdColRows;
 __device__ __forceinline__ int norm_exp(double sum, int mx, int64_t kc) {
   if (mx <= kNoExp) return kNoExp;
   if (sum > 1e-270 && sum < 1e300) {
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(128) k_prod_cols(const ProdJob* __restrict__ j
   const int64_t k1 = k0 + kColRows < J.kc ? k0 + kColRows : J.kc;
   int m = 2 * kNoExp;
   double sum = 0.0;
-#pragma unroll 8
+#pragma unroll 16
   for (int64_t k = k0; k < k1; ++k) {
     const int e = __ldg(J.rexp + k);
     const double v = (double)__ldg(X + k * n);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(128) k_prod_cexp(const ProdJob* __restrict__ j
   const int nb = (int)((J.kc + kColRows - 1) / kColRows);
   double sum = 0.0;
   int m = 2 * kNoExp;
-#pragma unroll 4
+#pragma unroll 16
   for (int r = 0; r < nb; ++r) {
     sum += J.csum[(size_t)r * n + c];
     m = max(m, J.cmax[(size_t)r * n + c]);
@@ -210,43 +210,59 @@ __global__ void __launch_bounds__(128) k_prod_cexp(const ProdJob* __restrict__ j
 // zeros to whole tiles and stages.  The residues of A carry the factor
 // (M / m_i)^-1 mod m_i of the reconstruction.
 //
-// X + 2^58 (2^31) is split into three 20-bit (two 16-bit) parts with fixed
-// residues of their weights; the sum v < 2^30 has the residue v - m floor((v +
-// h) / m) in [-h, m - 1 - h], h = (m - 1) / 2 (128 for m = 256).
-template <typename Real, int SIDE, int I>
-__device__ __forceinline__ int residue(uint32_t x0, uint32_t x1, uint32_t x2) {
-  constexpr int N = Fix<Real>::N, T = Fix<Real>::T, m = modulus(I);
-  constexpr int P = sizeof(Real) == 8 ? 20 : 16;
-  constexpr int f = SIDE == 0 ? crt_inv(I, N) : 1;
-  constexpr int h = m == 256 ? 128 : (m - 1) / 2;
-  constexpr uint32_t c0 = f % m, c1 = powmod2(P, m) * f % m, c2 = powmod2(2 * P, m) * f % m;
-  constexpr uint32_t bias = (uint32_t)((m - powmod2(T, m) * f % m) % m);
-  uint32_t v = x0 * c0 + bias + x1 * c1;
-  if (sizeof(Real) == 8) v += x2 * c2;
-  const uint32_t q = __umulhi(v + h, mod_magic(m)) >> 7;
-  return (int)(v - q * (uint32_t)m);
+// X + 2^T is taken byte by byte: the dot product of its bytes with the balanced
+// residues of 256^i (two dp4a; one for FP32) is an integer below 2^19 with the
+// right residue, and starting the sum at the bits of 1.5 2^23 leaves it in the
+// mantissa of a float.  With q = round(v / m) by the same trick, v - q m is the
+// balanced residue (m odd: v / m stays 1 / 2m = 0.0025 away from a tie, against
+// errors of 1e-4; m = 256: both ends of a tie are the byte 0x80), and its low
+// byte is that of the two bit patterns' difference, because 1.5 2^23's low byte
+// is zero.  Five instructions a residue, bound by issue; with 20-bit parts and
+// an exact division by multiplication it took eight (4096 x 4096 FP64, both
+// sides: 0.28 -> 0.18 ms).
+constexpr int balanced(int r, int m) {  // the residue in [-m / 2, m / 2)
+  return r % m >= (m + 1) / 2 ? r % m - m : r % m;
+}
+// balanced residues of f 256^(4 h + i), i < 4, one a byte
+constexpr uint32_t byte_weights(int f, int h, int m) {
+  uint32_t w = 0;
+  for (int i = 0; i < 4; ++i) w |= (uint32_t)(uint8_t)balanced(powmod2(8 * (4 * h + i), m) * f % m, m) << (8 * i);
+  return w;
+}
+__device__ __forceinline__ uint32_t dp4a_us(uint32_t bytes, uint32_t weights, uint32_t sum) {
+  uint32_t d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(bytes), "r"(weights), "r"(sum));
+  return d;
 }
 template <typename Real, int SIDE, int I>
-__device__ __forceinline__ void plane_store(const uint32_t (&x0)[16], const uint32_t (&x1)[16], const uint32_t (&x2)[16],
-                                            uint8_t* dst, size_t plane) {
+__device__ __forceinline__ uint32_t residue(uint32_t lo, uint32_t hi) {
+  constexpr int N = Fix<Real>::N, T = Fix<Real>::T, m = modulus(I);
+  constexpr int f = SIDE == 0 ? crt_inv(I, N) : 1;
+  constexpr uint32_t kBits = 0x4B400000u;  // 1.5 2^23
+  constexpr uint32_t start = kBits + (uint32_t)balanced(m - powmod2(T, m) * f % m, m);
+  uint32_t v = dp4a_us(lo, byte_weights(f, 0, m), start);
+  if (sizeof(Real) == 8) v = dp4a_us(hi, byte_weights(f, 1, m), v);
+  const float t = fmaf(__uint_as_float(v) - 12582912.f, 1.f / m, 12582912.f);
+  return v - __float_as_uint(t) * (uint32_t)m;  // (the low byte counts)
+}
+template <typename Real, int SIDE, int I>
+__device__ __forceinline__ void plane_store(const uint32_t (&lo)[16], const uint32_t (&hi)[16], uint8_t* dst, size_t plane) {
   constexpr int N = Fix<Real>::N;
   uint32_t w[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    int r[4];
+    uint32_t r[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) r[u] = residue<Real, SIDE, I>(x0[4 * q + u], x1[4 * q + u], x2[4 * q + u]);
-    const uint32_t lo = __byte_perm((uint32_t)r[0], (uint32_t)r[1], 0x0040);
-    const uint32_t hi = __byte_perm((uint32_t)r[2], (uint32_t)r[3], 0x0040);
-    w[q] = __byte_perm(lo, hi, 0x5410);
+    for (int u = 0; u < 4; ++u) r[u] = residue<Real, SIDE, I>(lo[4 * q + u], hi[4 * q + u]);
+    w[q] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
   }
   *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-  if constexpr (I + 1 < N) plane_store<Real, SIDE, I + 1>(x0, x1, x2, dst + plane, plane);
+  if constexpr (I + 1 < N) plane_store<Real, SIDE, I + 1>(lo, hi, dst + plane, plane);
 }
 
 template <typename Real, int SIDE>
 __global__ void __launch_bounds__(128) k_prod_slice(const ProdJob* __restrict__ jobs) {
-  constexpr int T = Fix<Real>::T, P = sizeof(Real) == 8 ? 20 : 16;
+  constexpr int T = Fix<Real>::T;
   const ProdJob& J = jobs[blockIdx.z];
   const int64_t n = SIDE ? J.n_b : J.n_a;
   const int tiles = 2 * (SIDE ? J.tiles_b : J.tiles_a);
@@ -265,17 +281,16 @@ __global__ void __launch_bounds__(128) k_prod_slice(const ProdJob* __restrict__ 
     Real x[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) x[u] = live && k0 + u < J.kc ? __ldg(X + (k0 + u) * n) : (Real)0;
-    uint32_t x0[16], x1[16], x2[16];
+    uint32_t lo[16], hi[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       const int e = k0 + u < J.kc ? __ldg(J.rexp + k0 + u) : kPSkip;
       const double y = e == kPSkip ? 0.0 : (double)x[u] * pow2(SIDE ? e : -e) * g;
       const unsigned long long w = (unsigned long long)__double2ll_rn(y) + (1ull << T);
-      x0[u] = (uint32_t)w & ((1u << P) - 1u);
-      x1[u] = (uint32_t)(w >> P) & ((1u << P) - 1u);
-      x2[u] = sizeof(Real) == 8 ? (uint32_t)(w >> (2 * P)) : 0u;
+      lo[u] = (uint32_t)w;
+      hi[u] = (uint32_t)(w >> 32);
     }
-    plane_store<Real, SIDE, 0>(x0, x1, x2, out + (size_t)(kh >> 1) * kProdSlab + (kh & 1) * (kProdSlab / 2), plane);
+    plane_store<Real, SIDE, 0>(lo, hi, out + (size_t)(kh >> 1) * kProdSlab + (kh & 1) * (kProdSlab / 2), plane);
   }
 }
 

@@ -9,6 +9,7 @@ namespace cmm {
 constexpr int kProdTile = 128;                 // columns per plane tile (two per output tile side)
 constexpr int kProdK = 32;                     // inner indices per int8 MMA
 constexpr int kProdSlab = kProdTile * kProdK;  // bytes of a plane tile per kProdK inner indices
+constexpr int kProdColRows = 64;               // inner indices per partial sum of a column's squares
 constexpr int64_t kProdMaxK = 32768;           // inner indices per launch (int32 accumulators)
 
 // kProdK-index steps of a launch over kc inner indices, in whole stages of 4
@@ -22,7 +23,7 @@ struct ProdJob {
   int* rexp;              // kc: row balance exponents
   int *cexpA, *cexpB;     // column exponents
   double* csum;           // partial sums of squares and largest exponents of the columns:
-  int* cmax;              //   ceil(kc / 256) x (n_a + n_b)
+  int* cmax;              //   ceil(kc / kProdColRows) x (n_a + n_b)
   int* flag;              // 1: a non-finite input or a failed wait
   uint8_t *slA, *slB;     // residue planes
   uint32_t* res;          // residues of the product: modulus x (64 tiles_p) x (256 tiles_b), four rows a word

@@ -646,7 +646,7 @@ size_t plane_bytes(int tiles, int64_t kc, bool f32) {
 // visits the parts of the work space in order
 template <typename F>
 void work_parts(const ProdJob& J, bool f32, bool own_c, F&& part) {
-  const size_t n = (size_t)(J.n_a + J.n_b), nb = (size_t)((J.kc + 255) / 256);
+  const size_t n = (size_t)(J.n_a + J.n_b), nb = (size_t)((J.kc + kProdColRows - 1) / kProdColRows);
   part(0, plane_bytes(J.tiles_a, J.kc, f32));
   part(1, plane_bytes(J.tiles_b, J.kc, f32));
   part(2, prod_residue_row(J, f32) * J.tiles_p);
@@ -721,7 +721,7 @@ int product_launches(const ProdJob* hJobs, int count) {
   bool used[7] = {}, cexp = false;
   for (int i = 0; i < count; ++i) {
     used[add_class(hJobs[i])] = true;
-    cexp |= hJobs[i].kc > 256;
+    cexp |= hJobs[i].kc > kProdColRows;
   }
   int n = 2 + (cexp ? 1 : 0) + 2 + 2 + 1;  // rows, columns, (their sums), planes, product, residues -> C, sums
   for (bool u : used) n += u ? 1 : 0;
