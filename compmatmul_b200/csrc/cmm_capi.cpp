@@ -162,7 +162,8 @@ static void check_sizes(int64_t n_a, int64_t n_inner, int64_t n_b) {
 
 // ------------------------------------------------------------- pipeline
 struct Codes {
-  DevBuf a, b;  // d x n_a, d x n_b
+  DevBuf mem;
+  uint32_t *a = nullptr, *b = nullptr;  // d x n_a, d x n_b, in mem
 };
 
 static DevBuf upload(const void* h, size_t n, cudaStream_t s) {
@@ -254,32 +255,50 @@ class RowFeed {
   std::vector<Piece> pieces_;
 };
 
-// codes of both sides for keys 0..n_a-1 and 0..n_b-1
+// codes of both sides for keys 0..n_a-1 and 0..n_b-1: one allocation, one
+// upload (hash parameters and the two jobs) and one launch
 static Codes make_codes(const SketchParams& sp, int64_t n_a, int64_t n_b, cudaStream_t s) {
-  DevBuf params = upload(sp.blob.data(), sp.blob.size(), s);
-  const size_t set = sp.fn_bytes * (size_t)sp.d;
-  const uint8_t* base = params.as<uint8_t>();
+  auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+  const size_t blob = up(sp.blob.size()), jobs = blob + up(2 * sizeof(HashJob)), a = up((size_t)sp.d * (size_t)n_a * 4);
   Codes c;
-  c.a = DevBuf((size_t)sp.d * (size_t)n_a * 4, s);
-  c.b = DevBuf((size_t)sp.d * (size_t)n_b * 4, s);
-  launch_hash_codes(sp.kind, base, base + 2 * set, sp.d, sp.log2b, n_a, c.a.as<uint32_t>(), s);
-  launch_hash_codes(sp.kind, base + set, base + 3 * set, sp.d, sp.log2b, n_b, c.b.as<uint32_t>(), s);
+  c.mem = DevBuf(jobs + a + (size_t)sp.d * (size_t)n_b * 4, s);
+  uint8_t* base = c.mem.as<uint8_t>();
+  c.a = reinterpret_cast<uint32_t*>(base + jobs);
+  c.b = reinterpret_cast<uint32_t*>(base + jobs + a);
+  const size_t set = sp.fn_bytes * (size_t)sp.d;
+  const HashJob h[2] = {{base, base + 2 * set, c.a, n_a, sp.d, sp.log2b, sp.kind},
+                        {base + set, base + 3 * set, c.b, n_b, sp.d, sp.log2b, sp.kind}};
+  std::vector<uint8_t> host(blob + sizeof(h));
+  std::memcpy(host.data(), sp.blob.data(), sp.blob.size());
+  std::memcpy(host.data() + blob, h, sizeof(h));
+  CMM_CUDA(cudaMemcpyAsync(base, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+  launch_hash_codes_jobs(reinterpret_cast<const HashJob*>(base + blob), 2, (int64_t)sp.d * std::max(n_a, n_b), s);
   return c;
 }
 
-// Budget for the per-chunk materialized rows (d copies of each row pair).
-// Bytes for the materialized rows of one chunk of inner indices: a third of
-// the free device memory, at most 8 GiB, or CMM_MATERIALIZE_BYTES when set
-// (smaller budgets run more chunks).
-static size_t materialize_budget() {
-  size_t free_b = 0, total_b = 0;
-  CMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+// Bytes for what one chunk of inner indices needs (materialized rows or residue
+// planes), at most `need`: a third of the free device memory, at most 8 GiB,
+// or CMM_MATERIALIZE_BYTES when set (smaller budgets run more chunks).  The
+// free memory is asked for only when the stream-ordered pool does not hold
+// enough already: cudaMemGetInfo takes 80 us and more, and waits for the device.
+static size_t materialize_budget(size_t need) {
   size_t cap = (size_t)8 << 30;
   if (const char* e = getenv("CMM_MATERIALIZE_BYTES")) {
     const long long v = atoll(e);
     if (v > 0 && (size_t)v < cap) cap = (size_t)v;
   }
-  return free_b / 3 < cap ? free_b / 3 : cap;
+  if (need > cap) need = cap;
+  int dev = 0;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  CMM_CUDA(cudaGetDevice(&dev));
+  CMM_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+  CMM_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  CMM_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  if (reserved >= used && reserved - used >= need) return need;
+  size_t free_b = 0, total_b = 0;
+  CMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  return std::min(need, free_b / 3);
 }
 
 // The cluster kernels when this device can co-schedule a cluster of them
@@ -311,7 +330,7 @@ static bool try_cluster_plan(int variant, bool f32, const Codes& codes, int64_t 
   } catch (const unsupported&) {
     return false;
   }
-  plan = make_residue_plan(codes.a.as<uint32_t>(), codes.b.as<uint32_t>(), n_a, n_b, sp.d, sp.b,
+  plan = make_residue_plan(codes.a, codes.b, n_a, n_b, sp.d, sp.b,
                            C.logL, C.logR2, s);
   return cluster_smem_fits(variant, f32, C, plan);
 }
@@ -351,7 +370,7 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   // inner indices per chunk: planes within the budget; rows still arriving
   // from the host: eighths, so that copies and work overlap
   const size_t per_k = (size_t)prod_moduli(f32) * 256 * (size_t)(J.tiles_a + J.tiles_b);
-  int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget() / per_k));
+  int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget(per_k * (size_t)((n_inner + 127) / 128 * 128)) / per_k));
   if (feed) kc = std::min<int64_t>(kc, std::max<int64_t>((n_inner + 7) / 8, 512));
   kc = std::max<int64_t>(kc / 128 * 128, 128);
   kc = std::min<int64_t>(kc, n_inner);
@@ -365,8 +384,8 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   product_set_work(J, base, f32, scratch);
   product_set_lists(J, base + work);
   ProdJob* dJ = reinterpret_cast<ProdJob*>(base + work + lists);
-  J.codesA = codes.a.as<uint32_t>();
-  J.codesB = codes.b.as<uint32_t>();
+  J.codesA = codes.a;
+  J.codesB = codes.b;
   J.p = dP;
   for (int64_t k0 = 0; k0 < n_inner; k0 += kc) {
     J.kc = std::min<int64_t>(kc, n_inner - k0);
@@ -414,7 +433,7 @@ static void sketch_device(int variant, const SketchParams& sp, const Codes& code
     set_sketch_kernel("cluster");
     const int64_t SA = plan.slots_a(), SB = plan.slots_b();
     const size_t per_row = (size_t)sp.d * (size_t)(SA + SB) * 8;
-    int64_t kc = (int64_t)(materialize_budget() / per_row);
+    int64_t kc = (int64_t)(materialize_budget(per_row * (size_t)n_inner) / per_row);
     if (kc < 1) kc = 1;
     if (kc > n_inner) kc = n_inner;
     DevBuf matA((size_t)sp.d * kc * SA * 8, s), matB((size_t)sp.d * kc * SB * 8, s);
@@ -434,11 +453,11 @@ static void sketch_device(int variant, const SketchParams& sp, const Codes& code
     // bucket-sorted plan + per-chunk materialized rows + v1 kernels
     set_sketch_kernel("slab");
     const SketchPlan P = plan_sketch_v1(variant, n_a, n_inner, n_b, sp.d, sp.b, num_sms());
-    SlabPlan plan = make_slab_plan(codes.a.as<uint32_t>(), codes.b.as<uint32_t>(), n_a, n_b, sp.d,
+    SlabPlan plan = make_slab_plan(codes.a, codes.b, n_a, n_b, sp.d,
                                    sp.b, P.logL, s);
     const int64_t SA = (int64_t)plan.EA * kPlanThreads, SB = (int64_t)plan.EB * kPlanThreads;
     const size_t per_row = (size_t)sp.d * (size_t)(SA + SB) * 8;
-    int64_t kc = (int64_t)(materialize_budget() / per_row);
+    int64_t kc = (int64_t)(materialize_budget(per_row * (size_t)n_inner) / per_row);
     if (kc < 1) kc = 1;
     if (kc > n_inner) kc = n_inner;
     DevBuf matA((size_t)sp.d * kc * SA * 8, s), matB((size_t)sp.d * kc * SB * 8, s);
@@ -458,7 +477,7 @@ static void sketch_device(int variant, const SketchParams& sp, const Codes& code
   set_sketch_kernel("small-b");
   rows_ready(0, n_inner);
   DevBuf partial((size_t)P.G * sp.d * (size_t)sp.b * elem, s);
-  launch_sketch_accumulate(P, dAT, dB, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
+  launch_sketch_accumulate(P, dAT, dB, codes.a, codes.b,
                            scale.as<int>(), tw, partial.ptr, s);
   DevBuf work(2 * (size_t)sp.d * (size_t)sp.b * 16, s);
   launch_finalize(P, partial.ptr, tw, work.ptr, dP, s);
@@ -498,7 +517,7 @@ static void sketch_device_mixed(int variant, const SketchParams& sp, const Codes
     SlabPlan& plan = cplan;
     const int64_t SA = plan.slots_a(), SB = plan.slots_b();
     const size_t per_row = (size_t)sp.d * (size_t)(SA + SB) * 4;
-    int64_t kc = (int64_t)(materialize_budget() / per_row);
+    int64_t kc = (int64_t)(materialize_budget(per_row * (size_t)n_inner) / per_row);
     if (kc < 1) kc = 1;
     if (kc > n_inner) kc = n_inner;
     DevBuf matA((size_t)sp.d * kc * SA * 4, s), matB((size_t)sp.d * kc * SB * 4, s);
@@ -516,11 +535,11 @@ static void sketch_device_mixed(int variant, const SketchParams& sp, const Codes
   }
   const SketchPlan P = plan_sketch_mixed(variant, n_a, n_inner, n_b, sp.d, sp.b, num_sms());
   set_sketch_kernel("slab-mixed");
-  SlabPlan plan = make_slab_plan(codes.a.as<uint32_t>(), codes.b.as<uint32_t>(), n_a, n_b, sp.d,
+  SlabPlan plan = make_slab_plan(codes.a, codes.b, n_a, n_b, sp.d,
                                  sp.b, P.logL, s);
   const int64_t SA = (int64_t)plan.EA * kPlanThreads, SB = (int64_t)plan.EB * kPlanThreads;
   const size_t per_row = (size_t)sp.d * (size_t)(SA + SB) * 4;
-  int64_t kc = (int64_t)(materialize_budget() / per_row);
+  int64_t kc = (int64_t)(materialize_budget(per_row * (size_t)n_inner) / per_row);
   if (kc < 1) kc = 1;
   if (kc > n_inner) kc = n_inner;
   DevBuf matA((size_t)sp.d * kc * SA * 4, s), matB((size_t)sp.d * kc * SB * 4, s);
@@ -567,11 +586,12 @@ static void decompress_to_host(int variant, int d, int b, int64_t n_a, int64_t n
     }
   } join{s, copy_stream(), {}};
   if (n_a > 0 && n_b > 0) {
-    int64_t rows = (n_a + 7) / 8;
+    // eight blocks, of 4 MB at least: a smaller one's launch and copy cost more than they hide
+    int64_t rows = std::max<int64_t>((n_a + 7) / 8, ((int64_t)4 << 20) / (8 * n_b) + 1);
     rows = (rows + 15) / 16 * 16;
     for (int64_t i0 = 0; i0 < n_a; i0 += rows) {
       const int64_t r = n_a - i0 < rows ? n_a - i0 : rows;
-      launch_decompress_dense_rows(variant, d, b, n_a, n_b, i0, r, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
+      launch_decompress_dense_rows(variant, d, b, n_a, n_b, i0, r, codes.a, codes.b,
                                    dP, dC + i0 * n_b, s);
       cudaEvent_t e;
       CMM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -864,7 +884,7 @@ int cmm_dev_decompress_dense(int variant, int hash_kind, int64_t n_a, int64_t n_
     cudaStream_t s = (cudaStream_t)stream;
     SketchParams sp = make_sketch_params(hash_kind, d, b, seed);
     Codes codes = make_codes(sp, n_a, n_b, s);
-    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
+    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a, codes.b,
                             dP, dC, s);
   });
 }
@@ -880,7 +900,7 @@ int cmm_dev_matmul(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
     sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
-    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
+    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a, codes.b,
                             P.as<double>(), dC, s);
   });
 }
@@ -1010,7 +1030,7 @@ int cmm_dev_matmul_f32(int variant, int hash_kind, int64_t n_a, int64_t n_inner,
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
     sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
-    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a.as<uint32_t>(), codes.b.as<uint32_t>(),
+    launch_decompress_dense(variant, d, b, n_a, n_b, codes.a, codes.b,
                             P.as<double>(), dC, s);
   });
 }

@@ -30,7 +30,7 @@ class CopyPool {
   }
 
   void copy(void* dst, const void* src, size_t n) {
-    constexpr size_t kMinPart = (size_t)4 << 20;
+    constexpr size_t kMinPart = (size_t)512 << 10;  // 50 us of one thread's memcpy, more than a wake-up
     const size_t parts = std::min<size_t>(workers_.size() + 1, (n + kMinPart - 1) / kMinPart);
     if (parts <= 1) {
       std::memcpy(dst, src, n);
