@@ -1266,13 +1266,13 @@ void batch_info(const BatchPlan* B, int64_t* items, int* ctas, int* launches) {
   if (ctas) *ctas = std::max(B->n_items ? B->ctas : 0, (int)std::min<int64_t>(2 * n_prod, num_sms()));
   if (launches) {
     // kernels per run: scale (if any), sketch (if any), the batched finalize,
-    // 3 per other finalize, the product sketches' kernels, 1 per dense C
+    // 2 or 3 per other finalize, the product sketches' kernels, 1 per dense C
     int n = (B->n_scale_jobs ? 1 : 0) + (B->n_items ? 1 : 0) + (B->n_fjobs ? 1 : 0);
     for (const auto& run : B->pruns)
       n += product_launches(B->pjobs.data() + run.first, run.second - run.first);
     for (size_t i = 0; i < B->prods.size(); ++i) {
       const auto& q = B->prods[i];
-      n += (B->by_product[i] || batch_finalize_fits(B->plans[i].log2b) ? 0 : 3) + (q.C && q.n_a > 0 && q.n_b > 0 ? 1 : 0);
+      n += (B->by_product[i] || batch_finalize_fits(B->plans[i].log2b) ? 0 : B->plans[i].logR ? 3 : 2) + (q.C && q.n_a > 0 && q.n_b > 0 ? 1 : 0);
     }
     *launches = n;
   }

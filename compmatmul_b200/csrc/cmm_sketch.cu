@@ -513,6 +513,7 @@ __global__ void k_fft_combine(const double2* partial, int G, int d, int logL, in
     const int rn = (R - r) & (R - 1);
     const int mn = r == 0 ? ((L - m) & (L - 1)) : (L - m - 1);
     double2 Q = make_double2(0.0, 0.0), Qn = make_double2(0.0, 0.0);
+#pragma unroll 8
     for (int g = 0; g < G; ++g) {
       const double2* base = partial + ((size_t)g * d + t) * (size_t)b;
       const double2 u = base[((size_t)r << logL) + m];
@@ -538,6 +539,7 @@ __global__ void k_fft_combine_natural(const double2* partial, int G, int d, int 
     const int64_t f = idx & (b - 1);
     const int64_t fn = (b - f) & (b - 1);
     double2 Q = make_double2(0.0, 0.0), Qn = make_double2(0.0, 0.0);
+#pragma unroll 8
     for (int g = 0; g < G; ++g) {
       const double2* base = partial + ((size_t)g * d + t) * (size_t)b;
       const double2 u = base[f], v = base[fn];
@@ -555,6 +557,7 @@ __global__ void k_sum_partials(const double* partial, int G, int64_t n, double* 
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
        idx += (int64_t)gridDim.x * blockDim.x) {
     double s_ = 0.0;
+#pragma unroll 8
     for (int g = 0; g < G; ++g) s_ += partial[(size_t)g * n + idx];
     out[idx] = s_;
   }
@@ -571,6 +574,7 @@ struct BatchArgs {
   int64_t is1, is2, ie, os1, os2, oe;
   const double2* tw;
   int log2b;
+  int spc;       // sequences per CTA
   int post;      // FFT: 1 = multiply by w_b^{-s2*e} (complex out); 2 = real part * scale out
   double scale;  // WHT: applied to the output
 };
@@ -581,14 +585,24 @@ __device__ __forceinline__ void seq_addr(const BatchArgs& a, int64_t s, int64_t&
   ob = s1 * a.os1 + s2 * a.os2;
 }
 
-constexpr int kBatchThreads = 256;
+constexpr int kBatchThreads = 512;
 constexpr int kBatchFftCap = 8192;  // complex FP64 per CTA (slabs up to L = 8192)
+
+// Sequences per CTA: as few as keep every SM at work (a CTA is bound by the
+// barriers and latencies of its log2 M stages, so a few full CTAs leave the
+// chip idle and each runs long: 5 inverses of length 1024, one a CTA instead of
+// eight: 26 -> 5 us), at most what fits the buffer.
+static int batch_spc(int cap, int logM, int64_t nseq) {
+  const int64_t want = (nseq + num_sms() - 1) / num_sms();
+  const int64_t most = cap >> logM;
+  return (int)(want < 1 ? 1 : want < most ? want : most);
+}
 
 // inverse complex DFT (sign +1), unnormalised
 __global__ void __launch_bounds__(kBatchThreads) k_batch_ifft(BatchArgs a) {
   extern __shared__ double2 sb[];
   const int M = 1 << a.logM;
-  const int spc = kBatchFftCap >> a.logM;  // sequences per CTA
+  const int spc = a.spc;
   const int64_t s0 = (int64_t)blockIdx.x * spc;
   const double2* in = reinterpret_cast<const double2*>(a.in);
   for (int e = threadIdx.x; e < (spc << a.logM); e += kBatchThreads) {
@@ -641,7 +655,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_ifft(BatchArgs a) {
 __global__ void __launch_bounds__(kBatchThreads) k_batch_wht(BatchArgs a) {
   extern __shared__ double sw[];
   const int M = 1 << a.logM;
-  const int spc = kWhtCap >> a.logM;
+  const int spc = a.spc;
   const int64_t s0 = (int64_t)blockIdx.x * spc;
   const double* in = reinterpret_cast<const double*>(a.in);
   for (int e = threadIdx.x; e < (spc << a.logM); e += kBatchThreads) {
@@ -680,19 +694,50 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_wht(BatchArgs a) {
 }
 
 static void run_batch(bool fft, BatchArgs a, cudaStream_t s) {
-  const int cap = fft ? kBatchFftCap : kWhtCap;
-  const int spc = cap >> a.logM;
-  const int64_t blocks = (a.nseq + spc - 1) / spc;
-  const int smem = fft ? kBatchFftCap * (int)sizeof(double2) : kWhtCap * (int)sizeof(double);
+  a.spc = batch_spc(fft ? kBatchFftCap : kWhtCap, a.logM, a.nseq);
+  const int64_t blocks = (a.nseq + a.spc - 1) / a.spc;
+  const int smem = (a.spc << a.logM) * (int)(fft ? sizeof(double2) : sizeof(double));
   count_launch();
   if (fft) {
-    CMM_CUDA(cudaFuncSetAttribute(k_batch_ifft, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CMM_CUDA(cudaFuncSetAttribute(k_batch_ifft, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kBatchFftCap * (int)sizeof(double2)));
     k_batch_ifft<<<(unsigned)blocks, kBatchThreads, smem, s>>>(a);
   } else {
-    CMM_CUDA(cudaFuncSetAttribute(k_batch_wht, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CMM_CUDA(cudaFuncSetAttribute(k_batch_wht, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kWhtCap * (int)sizeof(double)));
     k_batch_wht<<<(unsigned)blocks, kBatchThreads, smem, s>>>(a);
   }
   CMM_CUDA(cudaGetLastError());
+}
+
+// The inverse of [t][r][m] spectra (FWHT: values): length-L sequences, then
+// length-R ones across them, or the first alone when R = 1.  w1 is read, w2 is
+// used in between.
+static void inverse_passes(const SketchPlan& P, const double2* dTw, void* w1, void* w2, double* dP, cudaStream_t s) {
+  const bool fft = P.variant == kVariantFFT;
+  const double inv_b = 1.0 / (double)P.b;
+  // step 1: v_r[n] = sum_m w_L^{-mn} P[t][r][m], times w_b^{-rn}
+  BatchArgs a{};
+  a.in = w1; a.logM = P.logL;
+  a.nseq = (int64_t)P.d * P.R; a.inner = P.R;
+  a.is1 = P.b; a.is2 = P.L; a.ie = 1;
+  a.os1 = P.b; a.os2 = P.L; a.oe = 1;
+  a.tw = dTw; a.log2b = P.log2b;
+  if (P.logR == 0) {
+    a.out = dP; a.post = fft ? 2 : 0; a.scale = inv_b;
+    run_batch(fft, a, s);
+    return;
+  }
+  a.out = w2; a.post = fft ? 1 : 0; a.scale = 1.0;
+  run_batch(fft, a, s);
+  // step 2: p[t][n + qL] = (1/b) Re sum_r w_R^{-rq} v_r[n]
+  BatchArgs c{};
+  c.in = w2; c.out = dP; c.logM = P.logR;
+  c.nseq = (int64_t)P.d * P.L; c.inner = P.L;
+  c.is1 = P.b; c.is2 = 1; c.ie = P.L;
+  c.os1 = P.b; c.os2 = 1; c.oe = P.L;
+  c.tw = dTw; c.log2b = P.log2b; c.post = fft ? 2 : 0; c.scale = inv_b;
+  run_batch(fft, c, s);
 }
 
 // dWork holds 2 * d * b * 16 bytes.
@@ -701,51 +746,20 @@ void launch_finalize(const SketchPlan& P, const void* dPartial, const double2* d
   const int64_t db = (int64_t)P.d * P.b;
   int64_t blocks = (db + 255) / 256;
   if (blocks > 8192) blocks = 8192;
-  const double inv_b = 1.0 / (double)P.b;
   ProfScope prof("finalize", s);
-  count_launch(3);
+  count_launch();
   if (P.variant == kVariantFFT) {
     double2* w1 = reinterpret_cast<double2*>(dWork);
-    double2* w2 = w1 + db;
     k_fft_combine<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const double2*>(dPartial), P.G,
                                                    P.d, P.logL, P.logR, w1);
     CMM_CUDA(cudaGetLastError());
-    // step 1: v_r[n] = sum_m w_L^{-mn} P[t][r][m], times w_b^{-rn}
-    BatchArgs a{};
-    a.in = w1; a.out = w2; a.logM = P.logL;
-    a.nseq = (int64_t)P.d * P.R; a.inner = P.R;
-    a.is1 = P.b; a.is2 = P.L; a.ie = 1;
-    a.os1 = P.b; a.os2 = P.L; a.oe = 1;
-    a.tw = dTw; a.log2b = P.log2b; a.post = 1; a.scale = 1.0;
-    run_batch(true, a, s);
-    // step 2: p[t][n + qL] = (1/b) Re sum_r w_R^{-rq} v_r[n]
-    BatchArgs c{};
-    c.in = w2; c.out = dP; c.logM = P.logR;
-    c.nseq = (int64_t)P.d * P.L; c.inner = P.L;
-    c.is1 = P.b; c.is2 = 1; c.ie = P.L;
-    c.os1 = P.b; c.os2 = 1; c.oe = P.L;
-    c.tw = dTw; c.log2b = P.log2b; c.post = 2; c.scale = inv_b;
-    run_batch(true, c, s);
+    inverse_passes(P, dTw, w1, w1 + db, dP, s);
   } else {
     double* w1 = reinterpret_cast<double*>(dWork);
-    double* w2 = w1 + db;
     k_sum_partials<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const double*>(dPartial), P.G,
                                                     db, w1);
     CMM_CUDA(cudaGetLastError());
-    BatchArgs a{};
-    a.in = w1; a.out = w2; a.logM = P.logL;
-    a.nseq = (int64_t)P.d * P.R; a.inner = P.R;
-    a.is1 = P.b; a.is2 = P.L; a.ie = 1;
-    a.os1 = P.b; a.os2 = P.L; a.oe = 1;
-    a.tw = dTw; a.log2b = P.log2b; a.post = 0; a.scale = 1.0;
-    run_batch(false, a, s);
-    BatchArgs c{};
-    c.in = w2; c.out = dP; c.logM = P.logR;
-    c.nseq = (int64_t)P.d * P.L; c.inner = P.L;
-    c.is1 = P.b; c.is2 = 1; c.ie = P.L;
-    c.os1 = P.b; c.os2 = 1; c.oe = P.L;
-    c.tw = dTw; c.log2b = P.log2b; c.post = 0; c.scale = inv_b;
-    run_batch(false, c, s);
+    inverse_passes(P, dTw, w1, w1 + db, dP, s);
   }
 }
 
@@ -771,26 +785,12 @@ void launch_finalize_natural(int variant, int d, int b, int G, const void* dPart
   int64_t blocks = (db + 255) / 256;
   if (blocks > 8192) blocks = 8192;
   ProfScope prof("finalize", s);
-  count_launch(3);
+  count_launch();
   double2* w1 = reinterpret_cast<double2*>(dWork);
-  double2* w2 = w1 + db;
   k_fft_combine_natural<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const double2*>(dPartial), G, d,
                                                          P.log2b, P.logL, w1);
   CMM_CUDA(cudaGetLastError());
-  BatchArgs a{};
-  a.in = w1; a.out = w2; a.logM = P.logL;
-  a.nseq = (int64_t)P.d * P.R; a.inner = P.R;
-  a.is1 = P.b; a.is2 = P.L; a.ie = 1;
-  a.os1 = P.b; a.os2 = P.L; a.oe = 1;
-  a.tw = dTw; a.log2b = P.log2b; a.post = 1; a.scale = 1.0;
-  run_batch(true, a, s);
-  BatchArgs c{};
-  c.in = w2; c.out = dP; c.logM = P.logR;
-  c.nseq = (int64_t)P.d * P.L; c.inner = P.L;
-  c.is1 = P.b; c.is2 = 1; c.ie = P.L;
-  c.os1 = P.b; c.os2 = 1; c.oe = P.L;
-  c.tw = dTw; c.log2b = P.log2b; c.post = 2; c.scale = 1.0 / (double)P.b;
-  run_batch(true, c, s);
+  inverse_passes(P, dTw, w1, w1 + db, dP, s);
 }
 
 }  // namespace cmm
