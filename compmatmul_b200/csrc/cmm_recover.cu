@@ -273,6 +273,10 @@ __host__ __device__ __forceinline__ int digit_bits(int level) {
   return 64 - kHistBits * level < kHistBits ? 64 - kHistBits * level : kHistBits;
 }
 
+// Passes over the entries keep kTopUnroll loads a thread in flight, eight CTAs
+// of 256 threads per SM (16.8 M entries: one load, four CTAs 71 and 29 us).
+constexpr int kTopUnroll = 4;
+
 // histogram of digit `level` of the keys whose higher bits (the first
 // kHistBits * level) equal `prefix`
 __global__ void k_topk_hist(const double* __restrict__ C, int64_t n, int level, uint64_t prefix,
@@ -284,40 +288,61 @@ __global__ void k_topk_hist(const double* __restrict__ C, int64_t n, int level, 
   const int pbits = kHistBits * level;
   const int shift = 64 - pbits - w;
   const uint64_t dmask = (1ULL << w) - 1ULL;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = okey(__ldg(C + idx));
-    const bool in = level == 0 || (k >> (64 - pbits)) == prefix;
-    // warp-aggregated: one shared atomic per distinct digit in the warp
-    // (values cluster in few digits, plain atomics would serialise)
-    const uint32_t dg = in ? (uint32_t)((k >> shift) & dmask) : 0xffffffffu;
-    const uint32_t active = __activemask();
-    const uint32_t peers = __match_any_sync(active, dg);
-    const int lane = threadIdx.x & 31;
-    if (in && lane == __ffs(peers) - 1) atomicAdd(&sh[dg], (unsigned)__popc(peers));
+  const int lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 - lane < n; i0 += kTopUnroll * step) {
+    double v[kTopUnroll];
+#pragma unroll
+    for (int u = 0; u < kTopUnroll; ++u) v[u] = i0 + u * step < n ? __ldg(C + i0 + u * step) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kTopUnroll; ++u) {
+      const uint64_t k = okey(v[u]);
+      const bool in = i0 + u * step < n && (level == 0 || (k >> (64 - pbits)) == prefix);
+      // warp-aggregated: one shared atomic per distinct digit in the warp
+      // (values cluster in few digits, plain atomics would serialise)
+      const uint32_t dg = in ? (uint32_t)((k >> shift) & dmask) : 0xffffffffu;
+      const uint32_t peers = __match_any_sync(0xffffffffu, dg);
+      if (in && lane == __ffs(peers) - 1) atomicAdd(&sh[dg], (unsigned)__popc(peers));
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x)
     if (sh[i]) atomicAdd(&hist[i], (unsigned long long)sh[i]);
 }
 
-// one thread: walk the histogram from the top and pick the digit where the
-// running count reaches `need`; out = {digit, count_above_in_level, count_in_bin}
-__global__ void k_topk_pick(const unsigned long long* __restrict__ hist, int nbins,
-                            unsigned long long need, unsigned long long* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned long long run = 0;
-  for (int dgt = nbins - 1; dgt >= 0; --dgt) {
-    const unsigned long long c = hist[dgt];
-    if (run + c >= need) {
-      out[0] = (unsigned long long)dgt;
-      out[1] = run;
-      out[2] = c;
-      return;
-    }
-    run += c;
+// The digit, from the top, where the running count reaches `need`: out =
+// {digit, count_above_in_level, count_in_bin}, or {0, total, 0} if none does.
+// One CTA: counts of pairs of bins, then their suffix sums (one thread walking
+// 2048 bins took 54 us).
+constexpr int kPickThreads = kHistBins / 2;
+__global__ void __launch_bounds__(kPickThreads) k_topk_pick(const unsigned long long* __restrict__ hist, int nbins,
+                                                            unsigned long long need,
+                                                            unsigned long long* __restrict__ out) {
+  __shared__ unsigned long long warp_sum[kPickThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // thread x holds digits hi = kHistBins - 1 - 2 x and hi - 1
+  const int hi = kHistBins - 1 - 2 * (int)threadIdx.x;
+  const unsigned long long c0 = hi < nbins ? hist[hi] : 0, c1 = hi - 1 < nbins ? hist[hi - 1] : 0;
+  unsigned long long sum = c0 + c1;  // becomes the count of this thread's and all higher digits
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long x = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += x;
   }
-  out[0] = 0; out[1] = run; out[2] = 0;
+  if (lane == 31) warp_sum[w] = sum;
+  __syncthreads();
+  for (int i = 0; i < w; ++i) sum += warp_sum[i];
+  const unsigned long long above = sum - c0 - c1;
+  if (above < need && above + c0 >= need) {
+    out[0] = (unsigned long long)hi;
+    out[1] = above;
+    out[2] = c0;
+  } else if (above + c0 < need && sum >= need) {
+    out[0] = (unsigned long long)(hi - 1);
+    out[1] = above + c0;
+    out[2] = c1;
+  } else if (threadIdx.x == kPickThreads - 1 && sum < need) {
+    out[0] = 0; out[1] = sum; out[2] = 0;
+  }
 }
 
 // collect entries whose key prefix (top `pbits` bits) is >= pfx (strictly
@@ -326,13 +351,20 @@ __global__ void k_topk_collect(const double* __restrict__ C, int64_t n, int pbit
                                int strict, unsigned long long* __restrict__ keys,
                                unsigned long long* __restrict__ idxs, unsigned int* __restrict__ count,
                                unsigned int cap) {
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = okey(__ldg(C + idx));
-    const uint64_t top = pbits >= 64 ? k : (k >> (64 - pbits));
-    if (strict ? top > pfx : top >= pfx) {
-      const unsigned int slot = atomicAdd(count, 1u);
-      if (slot < cap) { keys[slot] = k; idxs[slot] = (unsigned long long)idx; }
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kTopUnroll * step) {
+    double v[kTopUnroll];
+#pragma unroll
+    for (int u = 0; u < kTopUnroll; ++u) v[u] = i0 + u * step < n ? __ldg(C + i0 + u * step) : 0.0;
+#pragma unroll
+    for (int u = 0; u < kTopUnroll; ++u) {
+      const int64_t idx = i0 + u * step;
+      const uint64_t k = okey(v[u]);
+      const uint64_t top = pbits >= 64 ? k : (k >> (64 - pbits));
+      if (idx < n && (strict ? top > pfx : top >= pfx)) {
+        const unsigned int slot = atomicAdd(count, 1u);
+        if (slot < cap) { keys[slot] = k; idxs[slot] = (unsigned long long)idx; }
+      }
     }
   }
 }
@@ -379,7 +411,8 @@ __global__ void k_topk_tie_write(const double* __restrict__ C, int64_t n, uint64
 }
 
 // single-CTA bitonic sort of up to kCandMax candidates: key descending,
-// index ascending; writes the first K as (i, j, value)
+// index ascending; writes the first K as (i, j, value).  The network is that of
+// the next power of two above the count (4096 always: 67 us).
 __global__ void __launch_bounds__(1024) k_topk_sort(const unsigned long long* __restrict__ keys,
                                                      const unsigned long long* __restrict__ idxs,
                                                      const unsigned int* __restrict__ count,
@@ -389,15 +422,17 @@ __global__ void __launch_bounds__(1024) k_topk_sort(const unsigned long long* __
   unsigned long long* sk = sdyn;
   unsigned long long* si = sdyn + kCandMax;
   const unsigned int n = *count < (unsigned)kCandMax ? *count : (unsigned)kCandMax;
-  for (int e = threadIdx.x; e < kCandMax; e += blockDim.x) {
+  int total = 64;
+  while (total < (int)n) total <<= 1;
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
     if ((unsigned)e < n) { sk[e] = keys[e]; si[e] = idxs[e]; }
     else { sk[e] = 0ULL; si[e] = ~0ULL; }
   }
   __syncthreads();
   // "a before b" := key_a > key_b || (key_a == key_b && idx_a < idx_b)
-  for (int size = 2; size <= kCandMax; size <<= 1) {
+  for (int size = 2; size <= total; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int e = threadIdx.x; e < kCandMax; e += blockDim.x) {
+      for (int e = threadIdx.x; e < total; e += blockDim.x) {
         const int partner = e ^ stride;
         if (partner > e) {
           const bool asc = (e & size) == 0;  // first half of each block: "before" order
@@ -433,7 +468,7 @@ void topk_dense(const double* dC, int64_t n_a, int64_t n_b, int K, uint32_t* dI,
   DevBuf hist((size_t)kHistBins * 8, s), pick(3 * 8, s);
   DevBuf keys((size_t)kCandMax * 8, s), idxs((size_t)kCandMax * 8, s), cnt(8, s);
   int64_t blocks = (n + 255) / 256;
-  if (blocks > 4 * num_sms()) blocks = 4 * num_sms();
+  if (blocks > 8 * num_sms()) blocks = 8 * num_sms();
   uint64_t prefix = 0;              // selected digits so far
   unsigned long long need = (unsigned long long)K;  // still to take at this prefix
   unsigned long long above = 0;     // taken strictly above the prefix (all levels)
@@ -447,7 +482,7 @@ void topk_dense(const double* dC, int64_t n_a, int64_t n_b, int K, uint32_t* dI,
     count_launch(2);
     k_topk_hist<<<(unsigned)blocks, 256, 0, s>>>(dC, n, level, prefix, hist.as<unsigned long long>());
     CMM_CUDA(cudaGetLastError());
-    k_topk_pick<<<1, 32, 0, s>>>(hist.as<unsigned long long>(), 1 << w, need,
+    k_topk_pick<<<1, kPickThreads, 0, s>>>(hist.as<unsigned long long>(), 1 << w, need,
                                  pick.as<unsigned long long>());
     CMM_CUDA(cudaMemcpyAsync(h_pick, pick.ptr, sizeof(h_pick), cudaMemcpyDeviceToHost, s));
     CMM_CUDA(cudaStreamSynchronize(s));
