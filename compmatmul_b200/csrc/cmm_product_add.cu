@@ -7,9 +7,9 @@
 // consecutive in the order of h2 (FFT: h2 in [m - h1(i), + W) mod b; FWHT: the
 // aligned block (m ^ h1(i)) / W), so a warp that owns W buckets reads its
 // entries of the sorted columns coalesced, looks up their C[i][j] and adds.
-// Three forms, chosen by plan_product_sketch:
+// Three forms, chosen by product_geometry:
 //  staged  b <= 2^16: rows of C staged in shared memory, a CTA of 16 windows;
-//  lane    a block of columns holds more columns than there are buckets: lane
+//  lane    a block of columns holds 1.5 times the buckets and more: lane
 //          = bucket, rows and sorted columns in shared memory;
 //  gather  b > 2^16: values gathered from L2.
 // Rows are split into G groups with partial sketches, added up by
@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(kIdxThreads) k_prod_index(const ProdJob* __res
 
 // ----------------------------------------------------------------- additions
 // The kernel of a job's additions: 0 gather, 1 and 2 staged (that many CTAs per
-// SM), 3 .. 6 lane with b = 512 .. 4096
+// SM), 3 .. 5 lane with b = 512 .. 2048
+constexpr int kAddClasses = 6;
 __host__ __device__ inline int add_class(const ProdJob& J) {
   return J.form == kAddGather ? 0 : (J.form == kAddStaged ? J.per_sm : J.log2b - 6);
 }
@@ -248,24 +249,51 @@ template <int JB>
 __device__ __forceinline__ double signed_value(double c, uint32_t e, uint32_t neg1) {
   return __longlong_as_double(__double_as_longlong(c) ^ ((long long)(((e << (28 - JB)) & 0x80000000u) ^ neg1) << 32));
 }
-// Adds a batch (one entry and its signed value a lane) to the warp's window of
-// W = wmask / 8 + 1 buckets.  Entries of one bucket are neighbours and are
-// added one rank after the other.
-template <int VARIANT, int JB>
-__device__ __forceinline__ void add_batch(double* acc, uint32_t e, double v, uint32_t key, uint32_t wmask, int lane) {
-  const uint32_t rank = e & 7u;
-  const uint32_t at = ((VARIANT == kVariantFFT ? e - key : e ^ key) >> (JB + 1)) & wmask;
-  double* a = reinterpret_cast<double*>(reinterpret_cast<char*>(acc) + at);
-  if (rank == 0) *a += v;
-  __syncwarp();
-  uint32_t todo = __ballot_sync(0xffffffffu, rank - 1u < 6u);
-  for (uint32_t k = 1; todo; ++k) {
-    bool now = rank == k;
-    if (k >= 6) now = lane == __ffs(todo) - 1;  // six or more: one lane at a time, in order
-    if (now) *a += v;
-    todo &= ~__ballot_sync(0xffffffffu, now);
-    __syncwarp();
+__device__ __forceinline__ void load_if(double& v, uint32_t at, bool p) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.f64 %0, [%1];\n\t}" : "+d"(v) : "r"(at), "r"((uint32_t)p) : "memory");
+}
+__device__ __forceinline__ void store_if(uint32_t at, double v, bool p) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f64 [%0], %1;\n\t}" ::"r"(at), "d"(v), "r"((uint32_t)p) : "memory");
+}
+// Adds Q batches of a row (an entry and its value a lane and batch) to the warp's
+// window of W = wmask / 8 + 1 buckets.  Entries of one bucket are neighbours and
+// are added one rank after the other; the entries of one rank are in different
+// buckets, so the batches' loads, sums and stores overlap.  Bound by latency and
+// issue (0.6 of the slots, a third of the shared memory cycles): with a batch at
+// a time 4096 x 4096, b = 65536, d = 9 took 0.675 ms, now 0.57; b = 16384 products of
+// a batch 4.5 -> 3.4 ms.  (Reading the next row's values before this row's
+// additions took 0.83 ms: the ring holds three rows.)
+template <int VARIANT, int JB, int Q>
+__device__ __forceinline__ void add_row(uint32_t acc, const uint32_t (&e)[Q], const double (&c)[Q], uint32_t key, uint32_t neg1,
+                                        uint32_t wmask, int lane) {
+  double v[Q], s[Q];
+  uint32_t at[Q], rank[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    rank[q] = e[q] & 7u;
+    v[q] = signed_value<JB>(c[q], e[q], neg1);
+    at[q] = acc + (((VARIANT == kVariantFFT ? e[q] - key : e[q] ^ key) >> (JB + 1)) & wmask);
+    s[q] = 0.0;
   }
+  for (uint32_t k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) load_if(s[q], at[q], rank[q] == k);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) store_if(at[q], s[q] + v[q], rank[q] == k);
+    __syncwarp();
+    bool more = false;  // an entry of a higher rank
+#pragma unroll
+    for (int q = 0; q < Q; ++q) more |= rank[q] - (k + 1) < 6u - k;
+    if (!__any_sync(0xffffffffu, more)) return;
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q)  // six or more: one lane at a time, in order
+    for (uint32_t todo = __ballot_sync(0xffffffffu, rank[q] == 6u); todo; todo &= todo - 1u) {
+      const bool now = lane == __ffs(todo) - 1;
+      load_if(s[q], at[q], now);
+      store_if(at[q], s[q] + v[q], now);
+      __syncwarp();
+    }
 }
 
 // ring of row blocks of C filled by one thread of warp kScWin with bulk copies
@@ -333,6 +361,7 @@ __device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, u
     double* acc = acc0 + (size_t)warp * W;
     for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
     __syncwarp();
+    const uint32_t acc_at = smem_u32(acc);
     const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
     int st = 0;
     unsigned ph = 0;
@@ -341,37 +370,52 @@ __device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, u
       const uint32_t cols = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
       const uint16_t* cum = reinterpret_cast<const uint16_t*>(J.cum) + ((size_t)t * J.blocks + jb) * cum16_stride(J.log2b);
       const uint32_t* ent = J.ent + 2 * ((size_t)t * J.n_b + (size_t)jb * kScCols);
+      const char* C = reinterpret_cast<const char*>(J.C + (size_t)jb * kScCols);
+      auto entries = [&](const RowKeys& k, int r, uint32_t (&x)[3]) {
+        const uint32_t n = __shfl_sync(0xffffffffu, k.cnt, r);
+        const uint32_t* at = ent + __shfl_sync(0xffffffffu, k.e0, r);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) x[q] = entry_at(at, n, lane + 32 * q);
+        return n;
+      };
+      auto values = [&](const uint32_t (&x)[3], uint32_t n, double (&y)[3]) {  // (a lane without an entry reads column 0)
+        ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+        if (!ok) return;
+        const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          y[q] = 0.0;
+          if (n > 32 * q) y[q] = *reinterpret_cast<const double*>(row + (x[q] & kColMask<12>));
+        }
+      };
+      auto release = [&] {
+        __syncwarp();
+        if (lane == 0) bar_arrive(&empty[st]);
+        if (++st == R.stages) { st = 0; ph ^= 1u; }
+      };
+      auto rest = [&](uint32_t e0, uint32_t n, int64_t i, uint32_t key, uint32_t neg1) {  // entries from the 97th on
+        for (uint32_t at = 96; at < n; at += 32) {
+          const uint32_t x[1] = {entry_at(ent + e0, n, at + lane)};
+          const double y[1] = {__ldg(reinterpret_cast<const double*>(C + i * J.ldc * 8 + (x[0] & kColMask<12>)))};
+          add_row<VARIANT, 12>(acc_at, x, y, key, neg1, wmask, lane);
+        }
+      };
       for (int64_t r0 = ib; r0 < ie && ok; r0 += 32) {
         const RowKeys k = row_keys<VARIANT, 12>(cA, cum, r0 + lane, ie, m0, W, b, cols);
         const int rows = (int)min((int64_t)32, ie - r0);
-        uint32_t cn = __shfl_sync(0xffffffffu, k.cnt, 0);
-        const uint32_t* en = ent + __shfl_sync(0xffffffffu, k.e0, 0);
-        uint32_t f0 = entry_at(en, cn, lane), f1 = entry_at(en, cn, lane + 32), f2 = entry_at(en, cn, lane + 64);
+        uint32_t f[3];
+        uint32_t nf = entries(k, 0, f);
         for (int r = 0; r < rows; ++r) {
-          const uint32_t cc = cn, c0 = f0, c1 = f1, c2 = f2;
-          const uint32_t* ec = en;
+          const uint32_t e[3] = {f[0], f[1], f[2]}, ne = nf;
+          if (r + 1 < rows) nf = entries(k, r + 1, f);
           const uint32_t key = __shfl_sync(0xffffffffu, k.key, r), neg1 = __shfl_sync(0xffffffffu, k.neg1, r);
-          if (r + 1 < rows) {
-            cn = __shfl_sync(0xffffffffu, k.cnt, r + 1);
-            en = ent + __shfl_sync(0xffffffffu, k.e0, r + 1);
-            f0 = entry_at(en, cn, lane);
-            f1 = entry_at(en, cn, lane + 32);
-            f2 = entry_at(en, cn, lane + 64);
-          }
-          ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+          double v[3];
+          values(e, ne, v);
           if (!ok) break;
-          const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
-          auto take = [&](uint32_t e) {  // (a lane without an entry reads column 0)
-            const double c = *reinterpret_cast<const double*>(row + (e & kColMask<12>));
-            add_batch<VARIANT, 12>(acc, e, signed_value<12>(c, e, neg1), key, wmask, lane);
-          };
-          if (cc > 0) take(c0);
-          if (cc > 32) take(c1);
-          if (cc > 64) take(c2);
-          for (uint32_t at = 96; at < cc; at += 32) take(entry_at(ec, cc, at + lane));
-          __syncwarp();
-          if (lane == 0) bar_arrive(&empty[st]);
-          if (++st == R.stages) { st = 0; ph ^= 1u; }
+          if (ne > 64) add_row<VARIANT, 12, 3>(acc_at, e, v, key, neg1, wmask, lane);
+          else add_row<VARIANT, 12, 2>(acc_at, {e[0], e[1]}, {v[0], v[1]}, key, neg1, wmask, lane);
+          if (ne > 96) rest(__shfl_sync(0xffffffffu, k.e0, r), ne, r0 + r, key, neg1);
+          release();
         }
       }
     }
@@ -481,7 +525,7 @@ __device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t s
 template <int NB>
 __global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* __restrict__ jobs, int count,
                                                                  uint32_t smem, int* __restrict__ timeout) {
-  const AddWork w = add_work(jobs, count, NB == 1 ? 3 : (NB == 2 ? 4 : (NB == 4 ? 5 : 6)));
+  const AddWork w = add_work(jobs, count, NB == 1 ? 3 : (NB == 2 ? 4 : 5));
   const ProdJob& J = jobs[w.job];
   if (J.variant == kVariantFFT) add_lane<kVariantFFT, NB>(J, w.t, w.g, smem, timeout);
   else add_lane<kVariantFWHT, NB>(J, w.t, w.g, smem, timeout);
@@ -500,6 +544,7 @@ __device__ __forceinline__ void add_gather(const ProdJob& J, int x, int t, int g
   double* acc = sacc + (size_t)warp * W;
   for (uint32_t e = lane; e < W; e += 32) acc[e] = 0.0;
   __syncwarp();
+  const uint32_t acc_at = smem_u32(acc);
   const uint32_t cols = (uint32_t)J.n_b;
   const uint32_t* cum = reinterpret_cast<const uint32_t*>(J.cum) + (size_t)t * (b + 1);
   const uint32_t* ent = J.ent + 2 * (size_t)t * cols;
@@ -532,14 +577,14 @@ __device__ __forceinline__ void add_gather(const ProdJob& J, int x, int t, int g
       entries(r + 2, h);
       const uint32_t key = __shfl_sync(0xffffffffu, k.key, r), neg1 = __shfl_sync(0xffffffffu, k.neg1, r);
       const uint32_t cc = __shfl_sync(0xffffffffu, k.cnt, r);
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        if (cc > 32 * q) add_batch<VARIANT, 17>(acc, e[q], signed_value<17>(v[q], e[q], neg1), key, wmask, lane);
+      if (cc > 64) add_row<VARIANT, 17, 3>(acc_at, e, v, key, neg1, wmask, lane);
+      else add_row<VARIANT, 17, 2>(acc_at, {e[0], e[1]}, {v[0], v[1]}, key, neg1, wmask, lane);
       if (cc > 96) {
         const uint32_t* ec = ent + __shfl_sync(0xffffffffu, k.e0, r);
         for (uint32_t at = 96; at < cc; at += 32) {
-          const uint32_t x = entry_at(ec, cc, at + lane);
-          add_batch<VARIANT, 17>(acc, x, signed_value<17>(value(row, x), x, neg1), key, wmask, lane);
+          const uint32_t x[1] = {entry_at(ec, cc, at + lane)};
+          const double y[1] = {value(row, x[0])};
+          add_row<VARIANT, 17>(acc_at, x, y, key, neg1, wmask, lane);
         }
       }
 #pragma unroll
@@ -608,13 +653,25 @@ void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_
   while ((1 << J.log2b) < b) ++J.log2b;
   const int64_t cols = std::max<int64_t>(std::min<int64_t>(n_b, kScCols), 1);
   J.blocks = (int)((n_b + kScCols - 1) / kScCols);
-  J.form = J.log2b > 16 ? kAddGather : (cols >= b ? kAddLane : kAddStaged);
-  // windows: 36 to 72 entries of a row, at most 1024 buckets (8 KB of shared memory a warp)
+  // Lane where the columns of a block are 1.5 times the buckets and more (4000 x
+  // 4000, b = 2048, d = 9: lane 0.46 ms, staged 0.64; 8000 x 8000, b = 4096, d = 7:
+  // 2.39 and 2.11); among other jobs 2.5 times, since a launch of its own for a
+  // few long CTAs costs more (64 uneven products: 12.55 ms a run at 1.5, 12.26).
+  J.form = J.log2b > 16 ? kAddGather : (2 * cols >= (alone ? 3 : 5) * (int64_t)b ? kAddLane : kAddStaged);
+  // Windows: 48 to 96 entries of a row (two or three batches a warp; 4000 x 1385, b =
+  // 8192: 36 to 72 227 G/s, 48 to 96 275), at most 1024 buckets (8 KB of shared
+  // memory a warp).  Half as many where that lets two CTAs share an SM and
+  // leaves 36 (batches of b = 16384 products: 3.5 -> 3.4 ms).
   const int64_t per_row = J.form == kAddGather ? std::max<int64_t>(n_b, 1) : cols;
   J.logW = 5;
-  while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 72 * (int64_t)b) ++J.logW;
+  while (J.logW < 10 && ((int64_t)2 << J.logW) * per_row <= 96 * (int64_t)b) ++J.logW;
   J.logW = std::min(J.logW, J.log2b);
-  J.per_sm = J.form == kAddStaged && add_fixed(J) + 3 * add_row(J) <= kScSmemHalf ? 2 : 1;
+  auto two = [&] { return J.form == kAddStaged && add_fixed(J) + 3 * add_row(J) <= kScSmemHalf; };
+  if (J.form == kAddStaged && !two() && J.logW > 5 && ((int64_t)1 << J.logW) * per_row > 72 * (int64_t)b) {
+    --J.logW;
+    if (!two()) ++J.logW;
+  }
+  J.per_sm = two() ? 2 : 1;
   const int64_t wins = (int64_t)b >> J.logW, most = std::min<int64_t>((n_a + 31) / 32, 512);
   int64_t G;
   if (J.form == kAddGather) {
@@ -625,9 +682,17 @@ void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_
     const int64_t fill = alone ? 12 * (int64_t)sms / (d * ((wins + kGaWarps - 1) / kGaWarps)) : 0;
     G = std::max((n_a + rows - 1) / rows, fill);
   } else {
-    // the CTAs that fit; among other jobs 512 rows, which outweigh a CTA's start and end
+    // The CTAs that fit, and up to three times as many where they keep 512 rows,
+    // since some SMs are faster than others (16384 rows, b = 65536: 9.45 -> 8.7
+    // ms).  Among other jobs 256 rows, which outweigh a CTA's start and end (64
+    // uneven products: 512 rows 13.4 ms a run, 256 12.3, 128 12.3).
     const int64_t ctas = J.form == kAddLane ? d : d * ((wins + kScWin - 1) / kScWin);
-    G = alone ? std::min<int64_t>(J.per_sm * sms / ctas, 64) : (n_a + 511) / 512;
+    if (alone) {
+      G = std::min<int64_t>(J.per_sm * sms / ctas, 64);
+      if (J.form == kAddStaged) G = std::max(G, std::min(3 * G, n_a / 512));
+    } else {
+      G = (n_a + 255) / 256;
+    }
   }
   J.G = (int)std::max<int64_t>(1, std::min(G, most));
 }
@@ -718,7 +783,7 @@ void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count,
 }
 
 int product_launches(const ProdJob* hJobs, int count) {
-  bool used[7] = {}, cexp = false;
+  bool used[kAddClasses] = {}, cexp = false;
   for (int i = 0; i < count; ++i) {
     used[add_class(hJobs[i])] = true;
     cexp |= hJobs[i].kc > kProdColRows;
@@ -729,7 +794,7 @@ int product_launches(const ProdJob* hJobs, int count) {
 }
 
 void product_layout(ProdJob* jobs, int count, bool f32) {
-  int64_t items = 0, ctas[7] = {};
+  int64_t items = 0, ctas[kAddClasses] = {};
   for (int i = 0; i < count; ++i) {
     ProdJob& J = jobs[i];
     items += (int64_t)J.tiles_p * J.tiles_b * prod_moduli(f32);
@@ -748,7 +813,8 @@ namespace {
 template <typename K, typename... A>
 void launch_add(K kernel, int64_t ctas, size_t smem, int threads, cudaStream_t s, A... args) {
   if (!ctas) return;
-  CMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the same for every launch: threads launch these kernels at the same time)
+  CMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScSmemMax));
   count_launch();
   kernel<<<(unsigned)ctas, threads, smem, s>>>(args...);
   CMM_CUDA(cudaGetLastError());
@@ -759,8 +825,8 @@ void launch_add(K kernel, int64_t ctas, size_t smem, int threads, cudaStream_t s
 void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
   if (count <= 0) return;
   ProfScope prof("finalize", s);
-  int64_t ctas[7] = {};
-  size_t smem[7] = {};
+  int64_t ctas[kAddClasses] = {};
+  size_t smem[kAddClasses] = {};
   for (int i = 0; i < count; ++i) {
     const ProdJob& J = hJobs[i];
     const int c = add_class(J);
@@ -775,7 +841,6 @@ void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, c
   launch_add(k_prod_add_lane<1>, ctas[3], smem[3], kScThreads, s, dJobs, count, (uint32_t)smem[3], flag);
   launch_add(k_prod_add_lane<2>, ctas[4], smem[4], kScThreads, s, dJobs, count, (uint32_t)smem[4], flag);
   launch_add(k_prod_add_lane<4>, ctas[5], smem[5], kScThreads, s, dJobs, count, (uint32_t)smem[5], flag);
-  launch_add(k_prod_add_lane<8>, ctas[6], smem[6], kScThreads, s, dJobs, count, (uint32_t)smem[6], flag);
   int64_t db = 0;
   for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
   count_launch();
