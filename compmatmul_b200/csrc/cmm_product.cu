@@ -534,13 +534,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
   if (s_abort) {  // a wait ran out: report, and let this CTA's MMAs and copies end before it does
     if (rank == 0 && warp == 9 && lane == 0) {
       mma_commit(&drain);
-      for (uint32_t it = 0; it < (1u << 20) && !bar_test(&drain, 0); ++it) __nanosleep(20);
+      bar_drain(&drain, 0);
     }
     if (tid == 0) {
       *timeout = 1;
       __threadfence_system();
       for (unsigned b = s_issued > kStages ? s_issued - kStages : 0; b < s_issued; ++b)
-        for (uint32_t it = 0; it < (1u << 20) && !bar_test(&full[b % kStages], (b / kStages) & 1u); ++it) __nanosleep(20);
+        bar_drain(&full[b % kStages], (b / kStages) & 1u);
       int job = 0;
       for (int64_t idx = pair; idx < items; idx += pairs) {
         job = prod_item(jobs, idx, job, NMOD).job;

@@ -317,12 +317,8 @@ __device__ __forceinline__ void produce_rows(const ProdJob& J, const RowRing& R,
     }
   }
   if (!ok)  // let the copies in flight land before the CTA ends
-    for (int q = 0; q < R.stages; ++q)
-      for (uint32_t k = 0; k < (1u << 16) && it > (unsigned)q; ++k) {
-        const unsigned z = it - 1 - q;
-        if (bar_test(&full[z % R.stages], (z / R.stages) & 1u)) break;
-        __nanosleep(20);
-      }
+    for (unsigned z = it > (unsigned)R.stages ? it - R.stages : 0; z < it; ++z)
+      bar_drain(&full[z % R.stages], (z / R.stages) & 1u);
 }
 
 // Staged form.  A gather from global memory costs one L1 tag cycle per lane (32

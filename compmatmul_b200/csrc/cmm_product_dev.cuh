@@ -29,18 +29,31 @@ __device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait (2^20 polls of 20 ns and more); gives up at once when another role
-// of the CTA has given up
+// bounded wait: two seconds on the device's clock (a count of polls would not
+// do, try_wait itself may suspend the thread for as long as it likes); gives up
+// at once when another role of the CTA has given up
+constexpr uint64_t kWaitNs = 2000000000ull;
+__device__ __forceinline__ uint64_t clock_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
   for (int it = 0; it < 64; ++it)
     if (bar_test(bar, parity)) return true;
-  for (uint32_t it = 0; it < (1u << 20); ++it) {
+  const uint64_t t0 = clock_ns();
+  do {
     if (bar_test(bar, parity)) return true;
     if (*abort) return false;
     __nanosleep(20);
-  }
+  } while (clock_ns() - t0 < kWaitNs);
   *abort = 1;
   return false;
+}
+// the same for what is in flight when a CTA gives up
+__device__ __forceinline__ void bar_drain(uint64_t* bar, uint32_t parity) {
+  const uint64_t t0 = clock_ns();
+  while (!bar_test(bar, parity) && clock_ns() - t0 < kWaitNs) __nanosleep(20);
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

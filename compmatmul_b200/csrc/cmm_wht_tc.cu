@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
   if (s_abort && tid == kLoaders + 128) {  // the MMAs this CTA issued, before their columns are freed
     atomicExch(timeout, 1);
     mma_commit(&drain);
-    for (uint32_t it = 0; it < (1u << 20) && !bar_test(&drain, 0); ++it) __nanosleep(20);
+    bar_drain(&drain, 0);
   }
   tc_fence_before();
   __syncthreads();
