@@ -93,50 +93,85 @@ struct Fix<float> {
 // when a row is zero.  A row pair with a non-finite value makes the whole
 // sketch NaN, as the transforms would (flag[0] = 1; the FFT form skips row
 // pairs with a zero row first, as its transform kernels do).
+//
+// Bound by latency: a CTA of four warps per row pair keeps four loads a thread
+// in flight and takes several rows, and the largest magnitude is that of the
+// bit patterns, one integer maximum a value (256 threads, one load, FP64
+// maxima: 56 us at 4096 x 4096, 52 now; 64 uneven FP32 products 510 -> 197 us).
+constexpr int kRowThreads = 128, kRowUnroll = 4;
+// largest magnitude's bits (FP64: of the high word, and whether any value is not zero)
+struct RowMax {
+  uint32_t hi = 0, any = 0;
+};
+__device__ __forceinline__ void row_take(RowMax& m, double v) {
+  const uint32_t h = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+  m.hi = max(m.hi, h);
+  m.any |= h | (uint32_t)__double2loint(v);
+}
+__device__ __forceinline__ void row_take(RowMax& m, float v) { m.hi = max(m.hi, __float_as_uint(v) & 0x7fffffffu); }
 template <typename Real>
-__global__ void __launch_bounds__(256) k_prod_rows(const ProdJob* __restrict__ jobs) {
+__device__ __forceinline__ RowMax row_max(const Real* __restrict__ x, int64_t n) {
+  RowMax m;
+  for (int64_t i = threadIdx.x; i < n; i += kRowUnroll * kRowThreads) {
+    Real v[kRowUnroll];
+#pragma unroll
+    for (int u = 0; u < kRowUnroll; ++u) v[u] = i + u * kRowThreads < n ? __ldg(x + i + u * kRowThreads) : (Real)0;
+#pragma unroll
+    for (int u = 0; u < kRowUnroll; ++u) row_take(m, v[u]);
+  }
+  m.hi = __reduce_max_sync(0xffffffffu, m.hi);
+  m.any = sizeof(Real) == 8 ? __reduce_or_sync(0xffffffffu, m.any) : m.hi;
+  return m;
+}
+template <typename Real>
+__global__ void __launch_bounds__(kRowThreads) k_prod_rows(const ProdJob* __restrict__ jobs) {
   const ProdJob& J = jobs[blockIdx.y];
-  __shared__ double sa[8], sb[8];
-  __shared__ int sbad;
-  for (int64_t k = blockIdx.x; k < J.kc; k += gridDim.x) {
-    const Real* ra = reinterpret_cast<const Real*>(J.A) + k * J.n_a;
-    const Real* rb = reinterpret_cast<const Real*>(J.B) + k * J.n_b;
-    if (threadIdx.x == 0) sbad = 0;
-    __syncthreads();
-    double ma = 0.0, mb = 0.0;
-    bool bad = false;
-    for (int64_t i = threadIdx.x; i < J.n_a; i += 256) {
-      const double v = fabs((double)__ldg(ra + i));
-      bad |= !(v <= DBL_MAX);
-      ma = fmax(ma, v);
+  constexpr int kWarps = kRowThreads / 32;
+  __shared__ uint32_t part[2][kWarps][4];  // (two rows: one barrier a row)
+  const int w = threadIdx.x >> 5;
+  int buf = 0;
+  for (int64_t k = blockIdx.x; k < J.kc; k += gridDim.x, buf ^= 1) {
+    const RowMax a = row_max(reinterpret_cast<const Real*>(J.A) + k * J.n_a, J.n_a);
+    const RowMax b = row_max(reinterpret_cast<const Real*>(J.B) + k * J.n_b, J.n_b);
+    if ((threadIdx.x & 31) == 0) {
+      part[buf][w][0] = a.hi;
+      part[buf][w][1] = a.any;
+      part[buf][w][2] = b.hi;
+      part[buf][w][3] = b.any;
     }
-    for (int64_t j = threadIdx.x; j < J.n_b; j += 256) {
-      const double v = fabs((double)__ldg(rb + j));
-      bad |= !(v <= DBL_MAX);
-      mb = fmax(mb, v);
+    constexpr uint32_t kInf = sizeof(Real) == 8 ? 0x7ff00000u : 0x7f800000u;
+    const bool bad = __syncthreads_or(a.hi >= kInf || b.hi >= kInf);
+    bool some = true;
+    if (bad) {  // a row counts as zero when all its numbers are, whatever NaNs it has
+      bool sa = false, sb = false;
+      for (int64_t i = threadIdx.x; i < J.n_a; i += kRowThreads) sa |= fabs((double)reinterpret_cast<const Real*>(J.A)[k * J.n_a + i]) > 0.0;
+      for (int64_t j = threadIdx.x; j < J.n_b; j += kRowThreads) sb |= fabs((double)reinterpret_cast<const Real*>(J.B)[k * J.n_b + j]) > 0.0;
+      sa = __syncthreads_or(sa);
+      some = __syncthreads_or(sb) && sa;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      ma = fmax(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-      mb = fmax(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { sa[w] = ma; sb[w] = mb; }
-    if (bad) sbad = 1;
-    __syncthreads();
     if (threadIdx.x == 0) {
-      for (int i = 1; i < 8; ++i) { ma = fmax(ma, sa[i]); mb = fmax(mb, sb[i]); }
+      uint32_t ha = 0, na = 0, hb = 0, nb = 0;
+      for (int i = 0; i < kWarps; ++i) {
+        ha = max(ha, part[buf][i][0]);
+        na |= part[buf][i][1];
+        hb = max(hb, part[buf][i][2]);
+        nb |= part[buf][i][3];
+      }
+      // exponent of the largest magnitude (-1023: an FP64 subnormal)
+      auto ex = [](uint32_t h) {
+        if (sizeof(Real) == 4) h = (uint32_t)__double2hiint((double)__uint_as_float(h));
+        return (int)(h >> 20) - 1023;
+      };
       int e;
-      if (!(ma > 0.0) || !(mb > 0.0)) {
+      if (na == 0 || nb == 0 || !some) {
         e = kPSkip;
       } else {
-        auto ex = [](double m) { return (int)((__double_as_longlong(m) >> 52) & 0x7ff) - 1023; };
-        e = (ex(ma) - ex(mb)) / 2;
+        e = (ex(ha) - ex(hb)) / 2;
         e = e > 1000 ? 1000 : (e < -1000 ? -1000 : e);
       }
       J.rexp[k] = e;
-      if (sbad && (e != kPSkip || J.variant != kVariantFFT)) *J.flag = 1;
+      if (bad && (e != kPSkip || J.variant != kVariantFFT)) *J.flag = 1;
     }
-    __syncthreads();
   }
 }
 
@@ -161,29 +196,30 @@ __global__ void __launch_bounds__(128) k_prod_cols(const ProdJob* __restrict__ j
   const int side = blockIdx.z & 1;
   const int64_t n = side ? J.n_b : J.n_a;
   const int64_t c = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  const int64_t k0 = (int64_t)blockIdx.y * kColRows;
-  if (c >= n || k0 >= J.kc) return;
+  if (c >= n) return;
   const Real* X = reinterpret_cast<const Real*>(side ? J.B : J.A) + c;
-  const int64_t k1 = k0 + kColRows < J.kc ? k0 + kColRows : J.kc;
-  int m = 2 * kNoExp;
-  double sum = 0.0;
+  for (int64_t r = blockIdx.y; r * kColRows < J.kc; r += gridDim.y) {
+    const int64_t k0 = r * kColRows, k1 = k0 + kColRows < J.kc ? k0 + kColRows : J.kc;
+    int m = 2 * kNoExp;
+    double sum = 0.0;
 #pragma unroll 16
-  for (int64_t k = k0; k < k1; ++k) {
-    const int e = __ldg(J.rexp + k);
-    const double v = (double)__ldg(X + k * n);
-    if (e != kPSkip && v != 0.0) {
-      const int hi = __double2hiint(v) & 0x7fffffff;
-      m = max(m, max((hi >> 20) - 1023, -1023) + (side ? e : -e));
-      const double w = v * pow2(side ? e : -e);
-      sum = fma(w, w, sum);
+    for (int64_t k = k0; k < k1; ++k) {
+      const int e = __ldg(J.rexp + k);
+      const double v = (double)__ldg(X + k * n);
+      if (e != kPSkip && v != 0.0) {
+        const int hi = __double2hiint(v) & 0x7fffffff;
+        m = max(m, max((hi >> 20) - 1023, -1023) + (side ? e : -e));
+        const double w = v * pow2(side ? e : -e);
+        sum = fma(w, w, sum);
+      }
     }
-  }
-  if (J.kc <= kColRows) {
-    (side ? J.cexpB : J.cexpA)[c] = norm_exp(sum, m, J.kc);
-  } else {
-    const size_t at = (size_t)blockIdx.y * (J.n_a + J.n_b) + (side ? J.n_a : 0) + c;
-    J.csum[at] = sum;
-    J.cmax[at] = m;
+    if (J.kc <= kColRows) {
+      (side ? J.cexpB : J.cexpA)[c] = norm_exp(sum, m, J.kc);
+    } else {
+      const size_t at = (size_t)r * (J.n_a + J.n_b) + (side ? J.n_a : 0) + c;
+      J.csum[at] = sum;
+      J.cmax[at] = m;
+    }
   }
 }
 __global__ void __launch_bounds__(128) k_prod_cexp(const ProdJob* __restrict__ jobs) {
@@ -658,6 +694,13 @@ bool product_timed_out() {
   return t;
 }
 
+// CTAs along a dimension that kernels stride over, of `want` useful ones, next to
+// `others` in the other dimensions: the grid is sized for the largest job, so
+// among many jobs most CTAs find nothing to do, and 250,000 of them take 0.1 ms.
+static unsigned spread(int64_t want, int64_t others) {
+  return (unsigned)std::max<int64_t>(1, std::min(want, std::max<int64_t>(8, 32768 / others)));
+}
+
 void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s) {
   if (count <= 0) return;
   int64_t kc = 0, n = 0, nn = 0;
@@ -672,14 +715,15 @@ void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count
   }
   {
     ProfScope prof("scale", s);
-    const dim3 gr((unsigned)std::min<int64_t>(kc, 4096), (unsigned)count);
-    const dim3 gc((unsigned)((n + 127) / 128), (unsigned)((kc + kColRows - 1) / kColRows), (unsigned)(2 * count));
+    const dim3 gr(spread(kc, count), (unsigned)count);
+    const unsigned cx = (unsigned)((n + 127) / 128);
+    const dim3 gc(cx, spread((kc + kColRows - 1) / kColRows, 2 * (int64_t)cx * count), (unsigned)(2 * count));
     count_launch(kc > kColRows ? 3 : 2);
     if (f32) {
-      k_prod_rows<float><<<gr, 256, 0, s>>>(dJobs);
+      k_prod_rows<float><<<gr, kRowThreads, 0, s>>>(dJobs);
       k_prod_cols<float><<<gc, 128, 0, s>>>(dJobs);
     } else {
-      k_prod_rows<double><<<gr, 256, 0, s>>>(dJobs);
+      k_prod_rows<double><<<gr, kRowThreads, 0, s>>>(dJobs);
       k_prod_cols<double><<<gc, 128, 0, s>>>(dJobs);
     }
     if (kc > kColRows) k_prod_cexp<<<dim3((unsigned)((nn + 127) / 128), (unsigned)count), 128, 0, s>>>(dJobs);
@@ -687,7 +731,7 @@ void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count
   }
   ProfScope prof("materialize", s);
   count_launch(2);
-  const unsigned ky = (unsigned)std::min(2 * prod_ksteps(kc), 64);
+  const unsigned ky = spread(2 * prod_ksteps(kc), 2 * (int64_t)std::max(ta, tb) * count);
   const dim3 ga((unsigned)(2 * ta), ky, (unsigned)count), gb((unsigned)(2 * tb), ky, (unsigned)count);
   if (f32) {
     k_prod_slice<float, 0><<<ga, 128, 0, s>>>(dJobs);
