@@ -181,11 +181,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // H128[n][k] at unit k / 8, row n
-  for (int e = tid; e < 128 * 128; e += kTcThreads) {
-    const int n = e >> 7, k = e & 127;
-    *reinterpret_cast<__nv_bfloat16*>(As + (k >> 3) * kUnitA + n * 16 + (k & 7) * 2) =
-        __float2bfloat16_rn((__popc(n & k) & 1) ? -1.f : 1.f);
+  // H128[n][k] at unit k / 8, row n, eight elements of K a store
+  for (int e = tid; e < 128 * 16; e += kTcThreads) {
+    const int n = e & 127, u = e >> 7;
+    const uint32_t row = __popc(n & (8 * u)) & 1 ? 0xbf80bf80u : 0x3f803f80u;
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      w[q] = row ^ ((__popc(n & (2 * q)) & 1) << 15) ^ ((uint32_t)(__popc(n & (2 * q + 1)) & 1) << 31);
+    *reinterpret_cast<uint4*>(As + u * kUnitA + n * 16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
