@@ -344,15 +344,16 @@ static int64_t chunk_len(int64_t k0, int64_t kc, int64_t n_inner, const RowFeed*
 }
 
 // The sketch through the product C itself (cmm_product.cu), when that is
-// estimated to be faster.  Where the group kernels apply, products under 2^24
-// multiply-adds stay with them: both take a few hundred microseconds there, and
-// those kernels' tests, which check that they ran, use such sizes.
+// estimated to be faster.  Where the group kernels apply, products under 10^7
+// multiply-adds stay with them, though the product sketch would take 0.1 ms
+// where they take 0.3 to 1: their tests, which check that they ran, use such
+// sizes.
 static bool product_applicable(int variant, bool f32, const SketchParams& sp, int64_t n_a, int64_t n_inner,
                                int64_t n_b) {
   if (!product_supported(sp.b, n_a, n_inner, n_b)) return false;
   if (sketch_kernel_choice() == 3) return true;
   if (sketch_kernel_choice() != 0) return false;
-  if (sketch_cluster_applicable(variant, f32, sp.b) && (double)n_a * (double)n_b * (double)n_inner < 16777216.0)
+  if (sketch_cluster_applicable(variant, f32, sp.b) && (double)n_a * (double)n_b * (double)n_inner < 1e7)
     return false;
   return product_faster(variant, f32, sp.d, sp.b, n_a, n_inner, n_b, true);
 }

@@ -764,19 +764,21 @@ void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, 
 
 // Estimates in microseconds, fitted to B200 times.  Single calls, n square, d =
 // 7, transforms / product:
-//   n = 512:  b = 256 119 / 187, 1024 228 / 155, 4096 387 / 157, 2^16 3380 / 236
-//   n = 2048: b = 256 413 / 517, 1024 770 / 593, 4096 1239 / 658, 2^16 12778 / 689
+//   n = 96:   FFT b = 512 49 / 97, 1024 64 / 93, 2048 107 / 92; FWHT b = 2048 66 / 92, 4096 96 / 90
+//   n = 512:  FFT b = 512 115 / 105, 4096 384 / 102, 2^16 3380 / 144; FWHT b = 512 93 / 104, 1024 116 / 105
+//   n = 2048: FFT b = 512 511 / 393, 1024 776 / 390, 4096 1221 / 407, 2^16 13190 / 501
 //   n = 8192, 32 inner indices, b = 256, d = 3: 408 / 3368 (the product pays
 //   d additions per entry of C however few inner indices there are)
 bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone) {
   const double nn = (double)n_a * (double)n_b, k = (double)n_inner;
-  const bool small_b = variant == kVariantFFT ? b < 4096 : b < 8192;
-  const double per_b = variant == kVariantFFT && !f32 ? 0.85e-6 : 0.5e-6;
+  const bool fft = variant == kVariantFFT, small_b = fft ? b < 4096 : b < 8192;
+  const double per_b = fft && !f32 ? 0.85e-6 : 0.5e-6;
   double log2b = 0;
   while ((1 << (int)log2b) < b) ++log2b;
-  const double transforms = (alone ? (small_b ? 70.0 : 230.0) : 0.0) +
-                            d * k * (per_b * b * log2b + 7e-6 * (double)(n_a + n_b));
-  const double product = (alone ? 110.0 : 5.0) + nn * (d / 1.8e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
+  // launches and the chain of one transform; small b: the stages of the longest chain
+  const double fixed = !alone ? 0.0 : small_b ? (fft ? 40.0 + 0.033 * b : 38.0 + 0.014 * b) : 230.0;
+  const double transforms = fixed + (alone && small_b ? 1.3 : 1.0) * d * k * (per_b * b * log2b + 7e-6 * (double)(n_a + n_b));
+  const double product = (alone ? 92.0 : 5.0) + nn * (d / 1.8e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
   return product < transforms;
 }
 
