@@ -14,7 +14,7 @@ The default single-GPU run also measures the other workloads as short legs,
 reported as extra keys of the same JSON line ("legs"): config 2 FWHT at
 n = 16384, config 1 (n = 512, FFT), config 2 at n = 4096 (both variants),
 config 3 (mixed precision, FFT and FWHT, against the FP64 path on the same
-inputs), the FP32 FWHT with its Hadamard-16 stages on the tensor cores
+inputs), the FP32 FWHT with a Hadamard-128 stage on the tensor cores
 (tcgen05) against CUDA cores on the same rows, config 4 (256 uneven
 products in one batch plan) and a bounded config 5 serving run.
 Each leg states its steps, its clocks and its result check.
@@ -152,6 +152,16 @@ def fft_flops(n_a, n_inner, n_b, d, b):
 def fwht_ops(n_a, n_inner, n_b, d, b):
     lb = np.log2(b)
     return n_inner * d * (2 * b * lb + 2 * b + 2 * (n_a + n_b)) + d * b * lb
+
+
+def int8_peak():
+    """(TOP/s, source): twice the measured sustained bf16 rate."""
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            bf16 = json.load(f)["bf16_tflops_sustained"]
+        return 2.0 * bf16, "twice bf16_tflops_sustained of MEASURED_PEAKS.json (int8 MMAs run at twice the bf16 rate)"
+    except (OSError, KeyError, ValueError):
+        return 2.0 * 1400.0, "twice 1400 TFLOP/s of bf16, an earlier measurement (MEASURED_PEAKS.json absent)"
 
 
 def fma_peak(L, fp64):
@@ -398,17 +408,21 @@ def run_batch(args, reps, warm, steps, compare_fp64, e2e_steps):
                "api": "BatchPlan.run with pinned host inputs copied in and dense estimates copied out"}
         del hin, hout
 
-    peak_tf = fma_peak(L, fp64=False)
+    # most of these products take the product sketch: its int8 work, 8 moduli
+    peak_tf, peak_src = int8_peak()
+    int8_total = sum(2.0 * s["m"] * s["n"] * s["p"] * 8 for s in shapes)
     alg_bytes = sum(4.0 * s["n"] * (s["m"] + s["p"]) for s in shapes)
     peak, peak_kind = measured_peaks()
-    achieved_tf = flops_total / (batch_ms / 1e3) / 1e12
+    achieved_tf = int8_total / (batch_ms / 1e3) / 1e12
     out = {
         "value": value, "ms_per_step": ms_per_step, "steps": steps, "warmup": warm,
-        "roofline": {"bound": "fp32", "achieved": achieved_tf, "peak": peak_tf, "unit": "TFLOP/s",
+        "roofline": {"bound": "int8 tensor", "achieved": achieved_tf, "peak": peak_tf, "unit": "TOP/s",
                      "frac": achieved_tf / peak_tf if peak_tf else None, "traffic": None,
-                     "peak_source": "measured now on this GPU by the library's FMA loop (cmm_probe_fma_tflops)",
-                     "kernel": "batch graph (persistent k_batch_sketch + finalize + dense decompress)",
-                     "launch_ms": batch_ms, "flops_per_launch": flops_total,
+                     "peak_source": peak_src,
+                     "kernel": "batch graph (product sketches, persistent k_batch_sketch + finalize for the "
+                               "others, dense decompress); the additions and the gathers of the estimates "
+                               "bound it, not the tensor cores",
+                     "launch_ms": batch_ms, "flops_per_launch": int8_total,
                      "hbm": {"achieved": alg_bytes / (batch_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                              "frac": alg_bytes / (batch_ms / 1e3) / 1e9 / peak, "peak_source": peak_kind,
                              "algorithmic_bytes_per_launch": alg_bytes}},
@@ -666,7 +680,7 @@ def leg_mixed_vs_fp64(workload, variant, warm=2, steps=3, warm64=1, steps64=2):
 
 
 def leg_wht_rows(rows=16384, log2n=13, warm=3, steps=1000):
-    """The FWHT's Hadamard-16 stages on the tensor cores (tcgen05 MMAs on
+    """The FWHT with a Hadamard-128 stage on the tensor cores (tcgen05 MMAs on
     BF16 hi/mid/lo splits, FP32 accumulators in tensor memory) against the
     same batched transform on CUDA cores: rows of 2^13 FP32 values (the
     mixed FWHT's slab length), 512 MB in and out per call (over L2).  Each
@@ -687,8 +701,8 @@ def leg_wht_rows(rows=16384, log2n=13, warm=3, steps=1000):
         results[method] = y.clone()
         out[method] = {"ms_per_call": ms, "clocks": clocks, "hbm_gbs": bytes_per_call / ms / 1e6,
                        "hbm_frac": bytes_per_call / ms / 1e6 / peak}
-    # tensor work of the two Hadamard-16 stages: 3 MMAs of 128 x 16 x 16 per 128-row tile
-    tflop = 2 * 3 * 2 * 16 * (rows * (1 << log2n)) / 1e12
+    # tensor work of the Hadamard-128 stage: 3 products of 128 multiply-adds per value
+    tflop = 3 * 2 * 128 * (rows * (1 << log2n)) / 1e12
     out["tensor"]["tensor_tflops"] = tflop / (out["tensor"]["ms_per_call"] * 1e-3)
     out["tensor_vs_cuda"] = out["cuda"]["ms_per_call"] / out["tensor"]["ms_per_call"]
     ref = results["cuda"]
@@ -939,26 +953,37 @@ def main():
         fp64_ms, _ = time_events(step64, 1, args.compare_fp64)
         del dAT64, dB64
 
-    # Roofline of the dominant kernel (the sketch kernel).  Its binding bound
-    # is arithmetic (FP64 for the plain path, FP32 for the mixed one): the
-    # transform work of the launch's share of the product, over its event
-    # time, against this GPU's FMA peak measured now.  The HBM view counts
-    # the algorithmic bytes of the inputs read once (8 n_inner (n_a + n_b)
-    # per product, split evenly over the product's sketch launches).
+    # Roofline of the dominant kernel.  Product sketch: the int8 tensor work of
+    # the residue products (15 moduli for FP64 inputs, 8 for FP32) over the time
+    # of the product kernels and the reconstruction, against twice the measured
+    # bf16 rate (int8 MMAs run at twice the bf16 rate).  Transform kernels:
+    # their binding bound is arithmetic (FP64 for the plain path, FP32 for the
+    # mixed one), the transform work of the launch's share of the product
+    # against this GPU's FMA peak measured now.  The HBM view counts the
+    # algorithmic bytes of the inputs read once (8 n_inner (n_a + n_b) per
+    # product, split evenly over the product's sketch launches).
     sk_ms, sk_n = fam["sketch"]
     sk_launch_ms = sk_ms / max(1, sk_n)
     launches_per_product = max(1, sk_n // max(1, args.steps))
-    flops = (fft_flops(n, n_inner, n, d, b) if variant == "fft" else fwht_ops(n, n_inner, n, d, b))
+    by_product = sketch_kernel == "product"
+    if by_product:
+        flops = 2.0 * n * n_inner * n * (8 if mixed else 15)
+        bound, unit = "int8 tensor", "TOP/s"
+        peak_tf, peak_src = int8_peak()
+    else:
+        flops = (fft_flops(n, n_inner, n, d, b) if variant == "fft" else fwht_ops(n, n_inner, n, d, b))
+        bound, unit = "fp32" if mixed else "fp64", "TFLOP/s"
+        peak_tf = fma_peak(L, fp64=not mixed)
+        peak_src = ("measured now on this GPU by the library's FMA loop (cmm_probe_fma_tflops); "
+                    "MEASURED_PEAKS.json has no FP64/FP32 CUDA-core entry")
     flops /= launches_per_product
     alg_bytes = esz * n_inner * (n + n) / launches_per_product
-    peak_tf = fma_peak(L, fp64=not mixed)
     hbm_peak, hbm_kind = measured_peaks()
     achieved_tf = flops / (sk_launch_ms / 1e3) / 1e12
     achieved_gb = alg_bytes / (sk_launch_ms / 1e3) / 1e9
-    roofline = {"bound": "fp32" if mixed else "fp64", "achieved": achieved_tf, "peak": peak_tf, "unit": "TFLOP/s",
+    roofline = {"bound": bound, "achieved": achieved_tf, "peak": peak_tf, "unit": unit,
                 "frac": achieved_tf / peak_tf if peak_tf else None, "traffic": None,
-                "peak_source": "measured now on this GPU by the library's FMA loop (cmm_probe_fma_tflops); "
-                               "MEASURED_PEAKS.json has no FP64/FP32 CUDA-core entry",
+                "peak_source": peak_src,
                 "kernel": f"sketch ({sketch_kernel})", "launch_ms": sk_launch_ms,
                 "launches_per_product": launches_per_product, "flops_per_launch": flops,
                 "hbm": {"achieved": achieved_gb, "peak": hbm_peak, "unit": "GB/s", "frac": achieved_gb / hbm_peak,

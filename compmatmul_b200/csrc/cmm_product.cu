@@ -595,22 +595,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
 
 // ------------------------------------------------------------ reconstruction
 // C[i][j] (+)= the integer with the N residues, in (-M / 2, M / 2), times
-// 2^(E_i + E_j - 2T).  sum r_i (M / m_i) - t M with t = round(sum r_i / m_i)
-// (24-bit fixed point: |entry| <= 2^2T < 0.34 M keeps it away from a tie) is
-// evaluated modulo 2^128 (2^64).  Thread = column j, four rows i at a time.
+// 2^(E_i + E_j - 2T).  S = sum r_i (M / m_i) in 32-bit limbs, minus t M with t =
+// round(S / M) from S's top limb (in FP32, off by less than 2^-11; |entry| <=
+// 2^2T < 0.34 M keeps S / M 0.16 away from a tie), modulo 2^128 (2^64).  The
+// top limb of 15 moduli needs 32 bits only.  Thread = column j, four rows i at a
+// time.  Bound by the multiply-adds of the limbs (4096 x 4096, 15 moduli: 168
+// us with a fixed-point sum for t and 64-bit top limbs, @C now).
 template <int N, int I>
-__device__ __forceinline__ void crt_terms(const uint32_t (&w)[16], int sh, unsigned long long (&s)[4], uint32_t& t) {
+__device__ __forceinline__ void crt_terms(const uint32_t (&w)[16], uint32_t pick, unsigned long long (&s)[3], uint32_t& top) {
   constexpr U128 P = mod_product(N, I);
-  const uint32_t r = (w[I] >> sh) & 0xffu;
-  t += r * (uint32_t)((16777216 + modulus(I) / 2) / modulus(I));
+  const uint32_t r = __byte_perm(w[I], 0, pick);
   s[0] += (unsigned long long)r * (uint32_t)P.lo;
   s[1] += (unsigned long long)r * (uint32_t)(P.lo >> 32);
   if (N > 8) {
     s[2] += (unsigned long long)r * (uint32_t)P.hi;
-    s[3] += (unsigned long long)r * (uint32_t)(P.hi >> 32);
+    top += r * (uint32_t)(P.hi >> 32);
   }
-  if constexpr (I + 1 < N) crt_terms<N, I + 1>(w, sh, s, t);
+  if constexpr (I + 1 < N) crt_terms<N, I + 1>(w, pick, s, top);
 }
+constexpr double two_to(int e) { return e <= 0 ? 1.0 : 2.0 * two_to(e - 1); }
 template <typename Real>
 __global__ void __launch_bounds__(256) k_prod_crt(const ProdJob* __restrict__ jobs) {
   constexpr int N = Fix<Real>::N, T = Fix<Real>::T;
@@ -629,20 +632,23 @@ __global__ void __launch_bounds__(256) k_prod_crt(const ProdJob* __restrict__ jo
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (i + u >= J.n_a) break;
-      unsigned long long s[4] = {0, 0, 0, 0};
-      uint32_t t = 1u << 23;
-      crt_terms<N, 0>(w, 8 * u, s, t);
-      t >>= 24;
+      unsigned long long s[3] = {0, 0, 0};
+      uint32_t top = 0;
+      crt_terms<N, 0>(w, 0x4440u + u, s, top);
       double v;
       if (N > 8) {
+        constexpr float inv = (float)(two_to(96) / ((double)M.hi * two_to(64)));
+        const uint32_t t = (uint32_t)__float2int_rn((float)(top + (uint32_t)(s[2] >> 32)) * inv);
         unsigned __int128 x = (unsigned __int128)s[0] + ((unsigned __int128)s[1] << 32) + ((unsigned __int128)s[2] << 64) +
-                              ((unsigned __int128)s[3] << 96);
+                              ((unsigned __int128)top << 96);
         x -= (((unsigned __int128)M.hi << 64) | M.lo) * t;
         const bool neg = (__int128)x < 0;
         if (neg) x = -x;
         v = fma((double)(unsigned long long)(x >> 64), 18446744073709551616.0, (double)(unsigned long long)x);
         if (neg) v = -v;
       } else {
+        constexpr float inv = (float)(two_to(36) / (double)M.lo);
+        const uint32_t t = (uint32_t)__float2int_rn((float)(uint32_t)(s[1] >> 4) * inv);
         v = (double)(long long)(s[0] + (s[1] << 32) - M.lo * t);
       }
       const int e = min(max(__ldg(J.cexpA + i + u), kMinExp) + eB, 2046), h = e >> 1;

@@ -204,10 +204,12 @@ int cmm_dev_gemm(int64_t n_a, int64_t n_inner, int64_t n_b, double* dC, const do
 
 /* ---------------------------------------------------------------------
  * Mixed precision (no reference twin: the reference binding accepts FP64
- * only, compmatmul.cpp:22-30).  FP32 inputs; sketches and transforms in
- * FP32 with two-sum compensated accumulation over k; FWHT Hadamard-16
- * factors on the tensor cores (BF16 hi/lo split, FP32 accumulation); the
- * reduction of the d spectra, the inverse transform, p and C in FP64.
+ * only, compmatmul.cpp:22-30).  FP32 inputs.  Where the product sketch is
+ * the faster form, the product of the inputs (each column scaled and rounded
+ * to 2^-31 of its norm) is formed exactly by int8 residue products on the
+ * tensor cores and added up in FP64.  Else sketches and transforms are FP32
+ * with two-sum compensated accumulation over k; the reduction of the d
+ * spectra, the inverse transform, p and C are FP64 in both.
  * ------------------------------------------------------------------- */
 int cmm_dev_compressed_product_f32(int variant, int hash_kind, int64_t n_a, int64_t n_inner,
                                    int64_t n_b, const float* dAT, const float* dB, int d, int b,
@@ -244,6 +246,10 @@ int cmm_dev_wht_rows_f32(const float* x, float* y, int64_t rows, int log2n, int 
  *   items (product, repetition t, frequency slab, k-group) from a device
  *   queue ordered longest first, then each product's k-group reduction +
  *   inverse and (when C != NULL) dense median decompression.
+ * Products for which the product sketch is estimated to be faster take it
+ * instead: its launches (residue planes, int8 products, reconstruction,
+ * additions) are shared by all of them, and the autotuner has nothing to
+ * choose there.
  * The whole sequence is captured in a CUDA graph on the first run and
  * replayed afterwards.  Per product class (variant, precision, b, sizes) an
  * autotuner times the candidate slab lengths and transform radices on the
@@ -289,7 +295,8 @@ int cmm_batch_destroy(void* handle);
  * (inputs when copied in, hash codes, sorted plans, row balance, k-group
  * partials, the sketch), prepares each on an upload stream, groups the
  * prepared ones into waves -- each wave is one persistent sketch launch over
- * all of its products' work items plus their reduction + inverse -- and runs
+ * all of its products' work items plus their reduction + inverse, and the
+ * shared launches of those that take the product sketch -- and runs
  * waves on several streams at once, so requests that arrive while others
  * run are admitted as memory frees up and their work overlaps on the device.
  * The sketch p of each request is copied back to the caller's host buffer.
@@ -350,7 +357,7 @@ int cmm_profile_read(const char* family, double* total_ms, int64_t* launches);
 /* Kernels launched by this library since load (always counted). */
 int64_t cmm_launch_count(void);
 /* Name of the sketch kernel family the last compressed product on this host
- * thread ran ("cluster", "slab", "slab-mixed", "small-b"); "" before any. */
+ * thread ran ("product", "cluster", "slab", "slab-mixed", "small-b"); "" before any. */
 const char* cmm_last_sketch_kernel(void);
 /* Measured FMA throughput of the current device in TFLOP/s (2 flops per
  * FMA; FP64 if fp64 != 0, else FP32), from a register-resident FMA loop
