@@ -355,7 +355,9 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
       "h"((uint16_t)3)
       : "memory");
 }
-__device__ __forceinline__ void cluster_sync() {
+// every thread of both CTAs, whole warps at a time
+__device__ __forceinline__ void pair_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -470,12 +472,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x & 1;
   const int64_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
   if (tid == 0) {
     // CTA 0's stage is full when both CTAs' halves are there
     for (int s = 0; s < kStages; ++s) { bar_init(&full[s], rank == 0 ? 2 : 1); bar_init(&empty[s], 1); }
@@ -485,9 +481,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
     s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pair_sync();  // both CTAs run
+  if (warp == 0)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                 "r"(512u)
+                 : "memory");
   fence_before();
-  __syncthreads();
-  cluster_sync();
+  pair_sync();
   fence_after();
   const uint32_t tbase = tmem_base;
   volatile int* abort = &s_abort;
@@ -514,6 +514,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
         }
       }
       s_issued = it;
+      // the last arrivals on this CTA's empty barriers come from the other CTA's MMAs
+      for (unsigned z = it > kStages ? it - kStages : 0; ok && z < it; ++z)
+        ok = bar_wait(&empty[z % kStages], (z / kStages) & 1u, abort);
     }
   } else if (warp == 9) {
     if (lane == 0) {
@@ -566,6 +569,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
       if (lane == 0) bar_arrive_lead(&accempty[ab]);
     }
   }
+  __syncwarp();
   __syncthreads();
   if (s_abort) {  // a wait ran out: report, and let this CTA's MMAs and copies end before it does
     if (rank == 0 && warp == 9 && lane == 0) {
@@ -585,12 +589,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
     }
     __syncthreads();
   }
-  // the pair ends together: CTA 0's MMAs read CTA 1's shared memory
+  // Allocating and freeing pairs of CTAs' tensor memory are operations of one
+  // warp of each CTA together, and CTA 0's MMAs read CTA 1's shared memory: the
+  // pair starts them together, and neither CTA leaves before both are through.
+  // (Left to end on their own, CTAs that shared their SMs with other streams'
+  // kernels did now and then not end at all.)
   fence_before();
-  cluster_sync();
+  pair_sync();
   fence_after();
-  if (warp == 0)
+  if (warp == 0) {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(512u) : "memory");
+  }
+  pair_sync();
 }
 
 // ------------------------------------------------------------ reconstruction
