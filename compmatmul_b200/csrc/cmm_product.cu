@@ -27,6 +27,7 @@
 // rows of a pair equally large, so this is normwise the error of FP64 (FP32)
 // transforms or smaller.
 #include <cfloat>
+#include <cmath>
 #include <mutex>
 
 #include "cmm_internal.h"
@@ -779,24 +780,71 @@ void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, 
   CMM_CUDA(cudaGetLastError());
 }
 
-// Estimates in microseconds, fitted to B200 times.  Single calls, n square, d =
-// 7, transforms / product:
-//   n = 96:   FFT b = 512 49 / 97, 1024 64 / 93, 2048 107 / 92; FWHT b = 2048 66 / 92, 4096 96 / 90
-//   n = 512:  FFT b = 512 115 / 105, 4096 384 / 102, 2^16 3380 / 144; FWHT b = 512 93 / 104, 1024 116 / 105
-//   n = 2048: FFT b = 512 511 / 393, 1024 776 / 390, 4096 1221 / 407, 2^16 13190 / 501
-//   n = 8192, 32 inner indices, b = 256, d = 3: 408 / 3368 (the product pays
-//   d additions per entry of C however few inner indices there are)
-bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone) {
-  const double nn = (double)n_a * (double)n_b, k = (double)n_inner;
-  const bool fft = variant == kVariantFFT, small_b = fft ? b < 4096 : b < 8192;
-  const double per_b = fft && !f32 ? 0.85e-6 : 0.5e-6;
+// ------------------------------------------------------------------- dispatch
+// Estimates in microseconds, fitted to single calls on B200 (random shapes, n 1 to
+// 20,000, b 2^9 to 2^23, both routes timed: the product within 10 % rms, the
+// transforms within 5 to 20).  Of 640 shapes 6 take the route that is slower by
+// more than a tenth; with the formula before, which counted the entries of C
+// only, 61 did (8953 x 32 x 6096, b = 2^21, d = 5: 13.7 ms, transforms 3.0).
+namespace {
+
+// Additions: a warp's step over one row and window costs the same with one entry
+// or twenty, so sparse rows (few columns, many buckets) pay per step.
+double additions_us(const ProdJob& J, bool alone, int sms) {
+  const double db = (double)J.d * (double)(1u << J.log2b), wins = (double)((1u << J.log2b) >> J.logW);
+  const double cols = (double)std::min<int64_t>(J.n_b, 4096);
+  double t = (double)J.G * db * 8.0 * 1.5 / 6.5e6;  // partial sketches, written and read
+  if (J.form == kAddGather)
+    return t + 7e-6 * db + (double)J.n_a * J.d * (wins * 1.09e-4 + (double)J.n_b * 2.0e-6);
+  const double ctas = J.d * (J.form == kAddLane ? 1.0 : std::ceil(wins / 16.0));
+  const double load = ctas * (double)J.G / ((double)J.per_sm * sms);  // CTAs per slot
+  const double row = J.form == kAddLane ? 0.3 + 2.1e-4 * cols
+                     : J.per_sm == 1   ? 0.43 + 1.5e-3 * cols / wins
+                                       : 0.5 + 3.6e-3 * cols / wins;
+  return t + (alone ? std::max(1.0, load) : load) * (double)J.n_a / J.G * J.blocks * row;
+}
+
+double product_us(const ProdJob& J, bool f32, int64_t n_inner, bool alone, int sms) {
+  const double na = (double)J.n_a, nb = (double)J.n_b, k = (double)n_inner;
+  const double gemm = 65536.0 * J.tiles_a * J.tiles_b * std::ceil(k / 128.0) * 128.0 * 2.0 * prod_moduli(f32) / 3.0e9;
+  const double planes = k * (na + nb), entries = na * nb;
+  // among other jobs there are no launches to wait for, and every kernel fills the device
+  if (!alone) return 5.0 + gemm + planes * (f32 ? 5e-6 : 8e-6) + entries * (f32 ? 4e-6 : 9e-6) + additions_us(J, alone, sms);
+  return 85.0 + gemm + planes * 9.3e-6 + entries * (f32 ? 1e-5 : 2e-5) + additions_us(J, alone, sms);
+}
+
+// The transform kernels that would run: launches and plan, the inverse per d b
+// log b, the work per d k b log b (FP64, FP32) and per d k (n_a + n_b).
+struct TransformCost {
+  double fixed, inverse, work, work32, rows;
+};
+double transforms_us(int variant, bool f32, int d, int b, double k, double n, bool alone) {
+  const bool fft = variant == kVariantFFT;
   double log2b = 0;
   while ((1 << (int)log2b) < b) ++log2b;
-  // launches and the chain of one transform; small b: the stages of the longest chain
-  const double fixed = !alone ? 0.0 : small_b ? (fft ? 40.0 + 0.033 * b : 38.0 + 0.014 * b) : 230.0;
-  const double transforms = fixed + (alone && small_b ? 1.3 : 1.0) * d * k * (per_b * b * log2b + 7e-6 * (double)(n_a + n_b));
-  const double product = (alone ? 92.0 : 5.0) + nn * (d / 1.8e5 + k * 2.0 * prod_moduli(f32) / 2.4e9);
-  return product < transforms;
+  const double blog = (double)b * log2b;
+  if (!alone) return d * k * ((fft && !f32 ? 0.85e-6 : 0.5e-6) * blog + 7e-6 * n);  // the batch kernel
+  static const TransformCost kSmall[2] = {{55, 0, 2.6e-6, 2.4e-6, 4.5e-6}, {52, 0, 2.2e-6, 2.1e-6, 7.5e-6}};
+  static const TransformCost kSlab[2] = {{135, 7e-6, 7.2e-7, 4.2e-7, 8e-6}, {138, 2e-6, 3.6e-7, 4.4e-7, 6e-6}};
+  static const TransformCost kGroup[2] = {{135, 7.6e-6, 8e-7, 4.2e-7, 8e-6}, {132, 4e-6, 4.5e-7, 3.1e-7, 1.3e-5}};
+  static const TransformCost kSlabBig[2] = {{140, 5.1e-6, 4.5e-7, 2.7e-7, 7e-4}, {150, 1.4e-6, 2.3e-7, 2.9e-7, 3.3e-4}};
+  static const TransformCost kBig[2] = {{170, 4.7e-6, 1.7e-6, 1.7e-6, 7e-3}, {130, 1.3e-6, 8.5e-7, 8.2e-7, 2.5e-3}};
+  const bool mixed = f32 && sketch_mixed_applicable(variant, b), slab = mixed || sketch_v1_applicable(variant, b, 0, 0);
+  const bool small_b = !slab && b <= 65536;
+  const TransformCost& c = (sketch_cluster_applicable(variant, f32, b) ? kGroup
+                            : slab ? (b < (1 << 20) ? kSlab : kSlabBig)
+                            : small_b ? kSmall : kBig)[fft ? 0 : 1];
+  return c.fixed + (small_b && fft ? 0.005 * b : 0.0) + c.inverse * d * blog +
+         d * k * ((f32 && (mixed || !slab) ? c.work32 : c.work) * blog + c.rows * n);
+}
+
+}  // namespace
+
+bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone) {
+  ProdJob J{};
+  product_geometry(J, variant, d, b, n_a, n_b, std::min(n_inner, kProdMaxK), alone, num_sms());
+  return product_us(J, f32, n_inner, alone, num_sms()) <
+         transforms_us(variant, f32, d, b, (double)n_inner, (double)(n_a + n_b), alone);
 }
 
 }  // namespace cmm
