@@ -762,6 +762,7 @@ struct BatchPlan {
   // products that take the product sketch (cmm_product.cu): runs of jobs that
   // share one work space, each run's jobs longest inner dimension first
   std::vector<int> by_product;        // per product: 1 if it is one of them
+  std::vector<char> shared_c;         // per product: its dense output overlaps another output
   std::vector<ProdJob> pjobs;
   std::vector<std::pair<int, int>> pruns;  // [first, last) jobs
   DevBuf pmem, plists, pdev, pflags;
@@ -878,6 +879,41 @@ void enqueue(BatchPlan& B, cudaStream_t s) {
   }
 }
 
+// Which dense outputs share memory with another output (shared_c), and whether
+// any output shares memory with an input.  Ranges in ascending order; of those
+// seen, the one that reaches farthest is enough: whatever else covers a point
+// below its end was found to overlap it.
+bool outputs_meet_inputs(BatchPlan& B) {
+  struct Range {
+    uintptr_t begin, end;
+    int product;
+    bool input;
+  };
+  std::vector<Range> r;
+  auto add = [&](const void* p, int64_t rows, int64_t cols, size_t elem, int i, bool input) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    if (p && rows > 0 && cols > 0) r.push_back({at, at + (size_t)rows * (size_t)cols * elem, i, input});
+  };
+  for (int i = 0; i < B.count; ++i) {
+    const cmm_batch_product& q = B.prods[(size_t)i];
+    const size_t elem = B.f32 ? 4 : 8;
+    add(q.AT, q.n_inner, q.n_a, elem, i, true);
+    add(q.B, q.n_inner, q.n_b, elem, i, true);
+    add(q.p, q.d, q.b, 8, i, false);
+    add(q.C, q.n_a, q.n_b, 8, i, false);
+  }
+  std::sort(r.begin(), r.end(), [](const Range& x, const Range& y) { return x.begin < y.begin; });
+  bool meet = false;
+  Range far_in{}, far_out{};
+  for (const Range& x : r) {
+    meet |= x.begin < (x.input ? far_out : far_in).end;
+    if (!x.input && x.begin < far_out.end) B.shared_c[(size_t)x.product] = B.shared_c[(size_t)far_out.product] = 1;
+    Range& f = x.input ? far_in : far_out;
+    if (x.end > f.end) f = x;
+  }
+  return meet;
+}
+
 // The jobs of the products that take the product sketch, their memory and
 // their sorted columns.  A run's work space takes at most a third of the free
 // device memory or 8 GiB; C is formed in the product's own dense output where
@@ -899,7 +935,8 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
     const cmm_batch_product& q = B.prods[(size_t)order[k]];
     ProdJob J{};
     product_geometry(J, q.variant, q.d, q.b, q.n_a, q.n_b, q.n_inner, false, num_sms());
-    const size_t need = product_work_bytes(J, B.f32, !product_usable_c(J, q.C));
+    double* room = B.shared_c[(size_t)order[k]] ? nullptr : q.C;
+    const size_t need = product_work_bytes(J, B.f32, !product_usable_c(J, room));
     if (B.pruns.empty() || work + need > budget) {
       B.pruns.push_back({(int)k, (int)k});
       work = 0;
@@ -923,7 +960,8 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
   B.pflags = DevBuf(B.pjobs.size() * sizeof(int), s);
   for (size_t k = 0; k < order.size(); ++k) {
     ProdJob& J = B.pjobs[k];
-    product_set_work(J, B.pmem.as<uint8_t>() + at_work[k], B.f32, B.prods[(size_t)order[k]].C);
+    product_set_work(J, B.pmem.as<uint8_t>() + at_work[k], B.f32,
+                     B.shared_c[(size_t)order[k]] ? nullptr : B.prods[(size_t)order[k]].C);
     product_set_lists(J, B.plists.as<uint8_t>() + at_list[k]);
     J.flag = B.pflags.as<int>() + k;
   }
@@ -1041,8 +1079,12 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   B->tw4096 = twiddles(1 << kBFftLog, s);
 
   // ---- products whose sketch is taken from the product itself
+  // (they write sketches and dense outputs while other products' inputs are still
+  // to be read, so none where those share memory)
   B->by_product.assign((size_t)count, 0);
-  for (int i = 0; i < count; ++i) {
+  B->shared_c.assign((size_t)count, 0);
+  const bool apart = !outputs_meet_inputs(*B);
+  for (int i = 0; i < count && apart; ++i) {
     const cmm_batch_product& q = B->prods[(size_t)i];
     B->by_product[(size_t)i] = q.n_inner <= kProdMaxK && product_supported(q.b, q.n_a, q.n_inner, q.n_b) &&
                                product_faster(q.variant, f32, q.d, q.b, q.n_a, q.n_inner, q.n_b, false);

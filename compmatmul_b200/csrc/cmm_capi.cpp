@@ -358,8 +358,19 @@ static bool product_applicable(int variant, bool f32, const SketchParams& sp, in
   return product_faster(variant, f32, sp.d, sp.b, n_a, n_inner, n_b, true);
 }
 
-// scratch: n_a x n_b doubles for C (the caller's dense output, written
-// later), or nullptr.
+// The caller's dense output as room for C, which it holds until the estimate is
+// written; nullptr where an input shares memory with it (later chunks of the
+// inner index are read after C's first entries are there).
+static double* product_room(double* dC, int64_t n_a, int64_t n_b, const void* dAT, const void* dB, int64_t n_inner,
+                            size_t elem) {
+  const size_t bytes = (size_t)n_a * (size_t)n_b * 8;
+  if (overlap(dC, bytes, dAT, (size_t)n_inner * (size_t)n_a * elem) ||
+      overlap(dC, bytes, dB, (size_t)n_inner * (size_t)n_b * elem))
+    return nullptr;
+  return dC;
+}
+
+// scratch: n_a x n_b doubles for C that no input overlaps, or nullptr.
 static void sketch_product(int variant, bool f32, const SketchParams& sp, const Codes& codes, int64_t n_a,
                            int64_t n_inner, int64_t n_b, const void* dAT, const void* dB, double* dP, double* scratch,
                            cudaStream_t s, RowFeed* feed) {
@@ -900,7 +911,8 @@ int cmm_dev_matmul(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int
     SketchParams sp = make_sketch_params(hash_kind, d, b, seed);
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
-    sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
+    sketch_device(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr,
+                  product_room(dC, n_a, n_b, dAT, dB, n_inner, 8));
     launch_decompress_dense(variant, d, b, n_a, n_b, codes.a, codes.b,
                             P.as<double>(), dC, s);
   });
@@ -1030,7 +1042,8 @@ int cmm_dev_matmul_f32(int variant, int hash_kind, int64_t n_a, int64_t n_inner,
     SketchParams sp = make_sketch_params(hash_kind, d, b, seed);
     Codes codes = make_codes(sp, n_a, n_b, s);
     DevBuf P((size_t)d * (size_t)b * 8, s);
-    sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr, dC);
+    sketch_device_mixed(variant, sp, codes, n_a, n_inner, n_b, dAT, dB, P.as<double>(), s, nullptr,
+                        product_room(dC, n_a, n_b, dAT, dB, n_inner, 4));
     launch_decompress_dense(variant, d, b, n_a, n_b, codes.a, codes.b,
                             P.as<double>(), dC, s);
   });

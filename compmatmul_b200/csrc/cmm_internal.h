@@ -259,6 +259,11 @@ void topk_dense(const double* dC, int64_t n_a, int64_t n_b, int K, uint32_t* dI,
 
 int num_sms();
 
+inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return na > 0 && nb > 0 && x < y + nb && y < x + na;
+}
+
 // ------------------------------------------------------- instrumentation
 // Event timing of kernel families (cmm_profile_*) and the launch counter.
 void prof_begin(const char* family, cudaStream_t s);
