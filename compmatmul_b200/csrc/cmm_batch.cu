@@ -766,6 +766,7 @@ struct BatchPlan {
   std::vector<ProdJob> pjobs;
   std::vector<std::pair<int, int>> pruns;  // [first, last) jobs
   DevBuf pmem, plists, pdev, pflags;
+  std::unique_ptr<WaitFlag> waits;
   int64_t max_hash_total = 0, max_inner = 0;
   const double2* tw4096 = nullptr;
   cudaGraph_t graph = nullptr;
@@ -865,8 +866,8 @@ void enqueue(BatchPlan& B, cudaStream_t s) {
     const ProdJob* d = B.pdev.as<ProdJob>() + run.first;
     const int n = run.second - run.first;
     launch_product_planes(h, d, n, B.f32, s);
-    launch_product_gemm(h, d, n, B.f32, s);
-    launch_product_add(h, d, n, s);
+    launch_product_gemm(h, d, n, B.f32, B.waits->dev(), s);
+    launch_product_add(h, d, n, B.waits->dev(), s);
   }
   for (int i = 0; i < B.count; ++i) {
     const cmm_batch_product& q = B.prods[(size_t)i];
@@ -923,7 +924,7 @@ void make_product_jobs(BatchPlan& B, cudaStream_t s) {
   for (int i = 0; i < B.count; ++i)
     if (B.by_product[(size_t)i]) order.push_back(i);
   if (order.empty()) return;
-  product_timeout_flag(nullptr);  // set up before any capture
+  B.waits.reset(new WaitFlag());
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return B.prods[(size_t)a].n_inner > B.prods[(size_t)b].n_inner; });
   size_t free_b = 0, total_b = 0;
@@ -1268,8 +1269,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
 
 void batch_run(BatchPlan* B, cudaStream_t user) {
   if (!B) throw invalid_argument("batch handle is null");
-  if (!B->pjobs.empty() && product_timed_out())
-    throw runtime_error("product sketch: a wait ran out in an earlier launch");
+  if (B->waits && B->waits->take()) throw runtime_error("product sketch: a wait ran out in an earlier run of this plan");
   cudaStream_t s = user ? user : B->stream;
   if (!B->exec) {
     // capture once: the sequence depends only on the plan
@@ -1297,7 +1297,9 @@ void batch_run(BatchPlan* B, cudaStream_t user) {
     CMM_CUDA(cudaGraphLaunch(B->exec, s));
   }
   count_launch((int)B->launches_per_run);
-  if (!user) CMM_CUDA(cudaStreamSynchronize(s));
+  if (user) return;
+  CMM_CUDA(cudaStreamSynchronize(s));
+  if (B->waits && B->waits->take()) throw runtime_error("product sketch: a wait ran out; its sketches are invalid");
 }
 
 void batch_info(const BatchPlan* B, int64_t* items, int* ctas, int* launches) {

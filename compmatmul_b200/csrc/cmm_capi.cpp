@@ -375,7 +375,8 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
                            int64_t n_inner, int64_t n_b, const void* dAT, const void* dB, double* dP, double* scratch,
                            cudaStream_t s, RowFeed* feed) {
   set_sketch_kernel("product");
-  if (product_timed_out()) throw std::runtime_error("product sketch: a wait ran out in an earlier launch");
+  WaitFlag& flag = thread_wait_flag();
+  if (flag.take()) throw std::runtime_error("product sketch: a wait ran out in an earlier launch of this thread");
   const size_t elem = f32 ? 4 : 8;
   ProdJob J{};
   product_geometry(J, variant, sp.d, sp.b, n_a, n_b, 1, true, num_sms());
@@ -413,10 +414,10 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
         if (feed) feed->wait(k0, J.kc, s);
         launch_product_planes(&J, dJ, 1, f32, s);
       }
-      launch_product_gemm(&J, dJ, 1, f32, s);
+      launch_product_gemm(&J, dJ, 1, f32, flag.dev(), s);
     }
   }
-  launch_product_add(&J, dJ, 1, s);
+  launch_product_add(&J, dJ, 1, flag.dev(), s);
 }
 
 // feed != nullptr: the rows of dAT / dB are still arriving from the host;
@@ -579,7 +580,7 @@ static uint64_t pick_seed(int has_seed, uint64_t seed) { return has_seed ? seed 
 static void check_group_waits() {
   if (sketch_group_timed_out())
     throw std::runtime_error("cluster sketch: a group barrier wait ran out; the sketch is invalid");
-  if (product_timed_out()) throw std::runtime_error("product sketch: a wait ran out; the sketch is invalid");
+  if (thread_wait_flag().take()) throw std::runtime_error("product sketch: a wait ran out; the sketch is invalid");
 }
 
 static void decompress_to_host(int variant, int d, int b, int64_t n_a, int64_t n_b, const Codes& codes,

@@ -26,9 +26,12 @@
 // per entry, in the norms of the balanced columns.  Balancing makes the two
 // rows of a pair equally large, so this is normwise the error of FP64 (FP32)
 // transforms or smaller.
-#include <cfloat>
 #include <cmath>
+#include <cstdlib>
+#include <cstring>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "cmm_internal.h"
 #include "cmm_product.h"
@@ -463,22 +466,23 @@ __device__ __forceinline__ void prod_epilogue(const ProdJob& J, const ProdItem& 
 
 template <int NMOD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
-    k_prod_gemm(const ProdJob* __restrict__ jobs, int64_t items, int* __restrict__ timeout) {
+    k_prod_gemm(const ProdJob* __restrict__ jobs, int64_t items, const ProdWaits waits) {
   extern __shared__ __align__(1024) unsigned char psm[];
   unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)psm + 127) & ~(uintptr_t)127);
   __shared__ uint64_t full[kStages], empty[kStages], accfull[2], accempty[2], drain;
   __shared__ uint32_t tmem_base;
-  __shared__ int s_abort;
+  __shared__ int s_wait[2];
   __shared__ unsigned s_issued;  // stages whose copies were issued
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x & 1;
   const int64_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (tid == 0) {
     // CTA 0's stage is full when both CTAs' halves are there
-    for (int s = 0; s < kStages; ++s) { bar_init(&full[s], rank == 0 ? 2 : 1); bar_init(&empty[s], 1); }
+    for (int s = 0; s < kStages; ++s) { bar_init(&full[s], (rank == 0 ? 2 : 1) + waits.extra); bar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { bar_init(&accfull[s], 1); bar_init(&accempty[s], 16); }
     bar_init(&drain, 1);
-    s_abort = 0;
+    s_wait[0] = 0;
+    s_wait[1] = waits.limit_us;
     s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -491,7 +495,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
   pair_sync();
   fence_after();
   const uint32_t tbase = tmem_base;
-  volatile int* abort = &s_abort;
+  volatile int* wait = s_wait;
 
   if (warp == 8) {
     if (lane == 0) {
@@ -507,7 +511,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
         const uint8_t* gn = J.slA + ((size_t)p.mod * 2 * J.tiles_a + 2 * (J.tile0 + p.nt) + rank) * KS * kProdSlab;
         for (int ks = 0; ks < KS; ks += kStageK, ++it) {
           const unsigned st = it % kStages;
-          if (!bar_wait(&empty[st], ((it / kStages) & 1u) ^ 1u, abort)) { ok = false; break; }
+          if (!bar_wait(&empty[st], ((it / kStages) & 1u) ^ 1u, wait)) { ok = false; break; }
           unsigned char* dst = ring + st * kStageBytes;
           bar_expect(&full[st], kStageBytes);
           bulk_load(dst, gm + (size_t)ks * kProdSlab, kStageBytes / 2, &full[st]);
@@ -517,7 +521,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
       s_issued = it;
       // the last arrivals on this CTA's empty barriers come from the other CTA's MMAs
       for (unsigned z = it > kStages ? it - kStages : 0; ok && z < it; ++z)
-        ok = bar_wait(&empty[z % kStages], (z / kStages) & 1u, abort);
+        ok = bar_wait(&empty[z % kStages], (z / kStages) & 1u, wait);
     }
   } else if (warp == 9) {
     if (lane == 0) {
@@ -529,12 +533,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
         const int KS = prod_ksteps(jobs[job].kc);
         const unsigned ab = acc & 1u;
         if (rank == 0) {
-          if (!bar_wait(&accempty[ab], ((acc >> 1) & 1u) ^ 1u, abort)) break;
+          if (!bar_wait(&accempty[ab], ((acc >> 1) & 1u) ^ 1u, wait)) break;
           fence_after();
         }
         for (int ks = 0; ks < KS; ks += kStageK, ++it) {
           const unsigned st = it % kStages;
-          if (!bar_wait(&full[st], (it / kStages) & 1u, abort)) { ok = false; break; }
+          if (!bar_wait(&full[st], (it / kStages) & 1u, wait)) { ok = false; break; }
           if (rank == 1) {
             bar_arrive_lead(&full[st]);
             continue;
@@ -558,7 +562,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
       const ProdItem p = prod_item(jobs, idx, job, NMOD);
       job = p.job;
       const unsigned ab = acc & 1u;
-      int got = lane == 0 ? (bar_wait(&accfull[ab], (acc >> 1) & 1u, abort) ? 1 : 0) : 0;
+      int got = lane == 0 ? (bar_wait(&accfull[ab], (acc >> 1) & 1u, wait) ? 1 : 0) : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) break;
       bar_test(&accfull[ab], (acc >> 1) & 1u);  // every lane observes the phase before it reads tensor memory
@@ -572,16 +576,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
   }
   __syncwarp();
   __syncthreads();
-  if (s_abort) {  // a wait ran out: report, and let this CTA's MMAs and copies end before it does
+  if (s_wait[0]) {  // a wait ran out: report, and let this CTA's MMAs and copies end before it does
     if (rank == 0 && warp == 9 && lane == 0) {
       mma_commit(&drain);
-      bar_drain(&drain, 0);
+      bar_drain(&drain, 0, wait);
     }
     if (tid == 0) {
-      *timeout = 1;
+      *waits.flag = 1;
       __threadfence_system();
       for (unsigned b = s_issued > kStages ? s_issued - kStages : 0; b < s_issued; ++b)
-        bar_drain(&full[b % kStages], (b / kStages) & 1u);
+        bar_drain(&full[b % kStages], (b / kStages) & 1u, wait);
       int job = 0;
       for (int64_t idx = pair; idx < items; idx += pairs) {
         job = prod_item(jobs, idx, job, NMOD).job;
@@ -671,46 +675,63 @@ __global__ void __launch_bounds__(256) k_prod_crt(const ProdJob* __restrict__ jo
   }
 }
 
-// host-mapped flag set by a wait of the product kernel that ran out
 }  // namespace
 
-int* product_timeout_flag(int** dev) {
-  static int* host = nullptr;
-  static int* mapped = nullptr;
-  static std::mutex mu;
-  std::lock_guard<std::mutex> g(mu);
-  if (!host) {
-    int* h = nullptr;
-    CMM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h), sizeof(int), cudaHostAllocMapped));
-    *h = 0;
-    CMM_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), h, 0));
-    host = h;
+// Flags come from pages of host-mapped memory that stay for the process.
+namespace {
+std::mutex g_flag_mu;
+std::vector<std::pair<int*, int*>> g_flags;  // free ones: host and device address
+}  // namespace
+
+WaitFlag::WaitFlag() {
+  constexpr int kPage = 256;
+  std::lock_guard<std::mutex> g(g_flag_mu);
+  if (g_flags.empty()) {
+    int *host = nullptr, *dev = nullptr;
+    CMM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host), kPage * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    CMM_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev), host, 0));
+    for (int i = 0; i < kPage; ++i) g_flags.emplace_back(host + i, dev + i);
   }
-  if (dev) *dev = mapped;
-  return host;
+  host_ = g_flags.back().first;
+  dev_ = g_flags.back().second;
+  g_flags.pop_back();
+  __atomic_store_n(host_, 0, __ATOMIC_RELEASE);
+}
+WaitFlag::~WaitFlag() {
+  std::lock_guard<std::mutex> g(g_flag_mu);
+  g_flags.emplace_back(host_, dev_);
+}
+bool WaitFlag::take() { return __atomic_exchange_n(host_, 0, __ATOMIC_ACQ_REL) != 0; }
+
+// (never given back: kernels of an ended thread may still run)
+WaitFlag& thread_wait_flag() {
+  static thread_local WaitFlag* f = nullptr;
+  if (!f) f = new WaitFlag();
+  return *f;
+}
+
+ProdWaits product_waits(int* flag, const char* kernel) {
+  ProdWaits w{flag, kWaitUs, 0};
+  const char* e = getenv("CMM_TEST_PRODUCT_WAIT");  // test hook: waits that cannot complete
+  if (e && !strcmp(e, kernel)) {
+    w.limit_us = 1000;
+    w.extra = 1;
+  }
+  return w;
 }
 
 namespace {
 
 template <int NMOD>
-void launch_gemm(const ProdJob* dJobs, int64_t items, cudaStream_t s) {
-  int* flag = nullptr;
-  product_timeout_flag(&flag);
+void launch_gemm(const ProdJob* dJobs, int64_t items, int* flag, cudaStream_t s) {
   CMM_CUDA(cudaFuncSetAttribute(k_prod_gemm<NMOD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProdSmem));
   const int grid = 2 * (int)std::min<int64_t>(items, num_sms() / 2);
   count_launch();
-  k_prod_gemm<NMOD><<<grid, kProdThreads, kProdSmem, s>>>(dJobs, items, flag);
+  k_prod_gemm<NMOD><<<grid, kProdThreads, kProdSmem, s>>>(dJobs, items, product_waits(flag, "product"));
   CMM_CUDA(cudaGetLastError());
 }
 
 }  // namespace
-
-bool product_timed_out() {
-  volatile int* h = product_timeout_flag(nullptr);
-  const bool t = *h != 0;
-  *h = 0;
-  return t;
-}
 
 // CTAs along a dimension that kernels stride over, of `want` useful ones, next to
 // `others` in the other dimensions: the grid is sized for the largest job, so
@@ -761,11 +782,11 @@ void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count
   CMM_CUDA(cudaGetLastError());
 }
 
-void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s) {
+void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, int* flag, cudaStream_t s) {
   if (count <= 0) return;
   ProfScope prof("sketch", s);
-  if (f32) launch_gemm<Fix<float>::N>(dJobs, hJobs[count - 1].item_end, s);
-  else launch_gemm<Fix<double>::N>(dJobs, hJobs[count - 1].item_end, s);
+  if (f32) launch_gemm<Fix<float>::N>(dJobs, hJobs[count - 1].item_end, flag, s);
+  else launch_gemm<Fix<double>::N>(dJobs, hJobs[count - 1].item_end, flag, s);
   int64_t n_b = 0, rows = 0;
   for (int i = 0; i < count; ++i) {
     n_b = std::max(n_b, hJobs[i].n_b);

@@ -80,13 +80,34 @@ void product_layout(ProdJob* jobs, int count, bool f32);
 // the flags); exponents and residue planes; the product; the additions.
 void launch_product_index(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
 void launch_product_planes(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
-void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, cudaStream_t s);
-void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s);
+// (flag: device address of the caller's WaitFlag)
+void launch_product_gemm(const ProdJob* hJobs, const ProdJob* dJobs, int count, bool f32, int* flag, cudaStream_t s);
+void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, int* flag, cudaStream_t s);
 // kernels of one planes + product + additions sequence
 int product_launches(const ProdJob* hJobs, int count);
-// host-mapped flag set by a wait of these kernels that ran out (*dev: its device address)
-int* product_timeout_flag(int** dev);
-// true (and cleared) when such a wait ran out since the last call
-bool product_timed_out();
+
+// Set by a wait of these kernels that ran out; its sketch is NaN.  One for each
+// caller that reports on its own: a host thread's single calls, a batch plan, a
+// stream of a server.  Kernels that may set it have ended when it is destroyed.
+class WaitFlag {
+ public:
+  WaitFlag();
+  ~WaitFlag();
+  WaitFlag(const WaitFlag&) = delete;
+  WaitFlag& operator=(const WaitFlag&) = delete;
+  int* dev() const { return dev_; }
+  bool take();  // true (and cleared) when a wait ran out since the last call
+
+ private:
+  int *host_ = nullptr, *dev_ = nullptr;
+};
+WaitFlag& thread_wait_flag();
+// How a kernel's waits end: the flag, the limit, and arrivals that its barriers
+// wait for and do not get (the test hook CMM_TEST_PRODUCT_WAIT = product | add)
+struct ProdWaits {
+  int* flag;
+  int limit_us, extra;
+};
+ProdWaits product_waits(int* flag, const char* kernel);
 
 }  // namespace cmm

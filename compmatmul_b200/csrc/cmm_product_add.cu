@@ -332,23 +332,31 @@ struct RowRing {
   uint32_t row_bytes;
   int stages;
 };
-__device__ __forceinline__ void produce_rows(const ProdJob& J, const RowRing& R, uint64_t* full, uint64_t* empty,
-                                             int64_t ib, int64_t ie, volatile int* abort) {
+// (returns the row blocks that it issued)
+__device__ __forceinline__ unsigned produce_rows(const ProdJob& J, const RowRing& R, uint64_t* full, uint64_t* empty,
+                                                 int64_t ib, int64_t ie, volatile int* wait) {
   unsigned it = 0, st = 0, ph = 0;
   bool ok = true;
   for (int jb = 0; jb < J.blocks && ok; ++jb) {
     const uint32_t cols = (uint32_t)min((int64_t)kScCols, J.n_b - (int64_t)jb * kScCols);
     const uint32_t bytes = ((cols + 1u) & ~1u) * 8u;  // the row stride is even
     for (int64_t i = ib; i < ie; ++i, ++it) {
-      if (!bar_wait(&empty[st], ph ^ 1u, abort)) { ok = false; break; }
+      if (!bar_wait(&empty[st], ph ^ 1u, wait)) { ok = false; break; }
       bar_expect(&full[st], bytes);
       bulk_load(R.base + st * R.row_bytes, J.C + i * J.ldc + (int64_t)jb * kScCols, bytes, &full[st]);
       if (++st == (unsigned)R.stages) { st = 0; ph ^= 1u; }
     }
   }
-  if (!ok)  // let the copies in flight land before the CTA ends
-    for (unsigned z = it > (unsigned)R.stages ? it - R.stages : 0; z < it; ++z)
-      bar_drain(&full[z % R.stages], (z / R.stages) & 1u);
+  return it;
+}
+// a wait ran out: report, and let the copies in flight land before the CTA ends
+__device__ __forceinline__ void give_up(const ProdJob& J, const RowRing& R, uint64_t* full, unsigned issued,
+                                        const ProdWaits& waits, volatile int* wait) {
+  *waits.flag = 1;
+  *J.flag = 1;
+  __threadfence_system();
+  for (unsigned z = issued > (unsigned)R.stages ? issued - R.stages : 0; z < issued; ++z)
+    bar_drain(&full[z % R.stages], (z / R.stages) & 1u, wait);
 }
 
 // Staged form.  A gather from global memory costs one L1 tag cycle per lane (32
@@ -357,10 +365,11 @@ __device__ __forceinline__ void produce_rows(const ProdJob& J, const RowRing& R,
 // copies the row blocks, warps 0-15 own a window each; the next row's entries
 // are read while a row is added.
 template <int VARIANT>
-__device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, uint32_t smem, int* timeout) {
+__device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, uint32_t smem, const ProdWaits& waits) {
   extern __shared__ __align__(128) unsigned char ssm[];
   __shared__ uint64_t full[8], empty[8];
-  __shared__ int s_abort;
+  __shared__ int s_wait[2];
+  __shared__ unsigned s_issued;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t b = 1u << J.log2b, W = 1u << J.logW, wmask = (W - 1u) * 8u;
   const uint32_t win0 = x * kScWin, wins = b >> J.logW;
@@ -372,16 +381,18 @@ __device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, u
   R.row_bytes = (((uint32_t)min((int64_t)kScCols, J.n_b) + 15u) & ~15u) * 8u;
   R.stages = (int)min(8u, (smem - acc_bytes) / R.row_bytes);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], nw); }
-    s_abort = 0;
+    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1 + waits.extra); bar_init(&empty[s], nw); }
+    s_wait[0] = 0;
+    s_wait[1] = waits.limit_us;
+    s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  volatile int* abort = &s_abort;
+  volatile int* wait = s_wait;
   const int64_t per = (J.n_a + J.G - 1) / J.G;
   const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
   if (warp == kScWin) {
-    if (lane == 0) produce_rows(J, R, full, empty, ib, ie, abort);
+    if (lane == 0) s_issued = produce_rows(J, R, full, empty, ib, ie, wait);
   } else if (warp < nw) {
     const uint32_t m0 = (win0 + warp) << J.logW;
     double* acc = acc0 + (size_t)warp * W;
@@ -405,7 +416,7 @@ __device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, u
         return n;
       };
       auto values = [&](const uint32_t (&x)[3], uint32_t n, double (&y)[3]) {  // (a lane without an entry reads column 0)
-        ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+        ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, wait));
         if (!ok) return;
         const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
 #pragma unroll
@@ -449,30 +460,27 @@ __device__ __noinline__ void add_staged(const ProdJob& J, int x, int t, int g, u
     for (uint32_t e = lane; e < W; e += 32) out[e] = acc[e];
   }
   __syncthreads();
-  if (s_abort && threadIdx.x == 0) {
-    *timeout = 1;
-    *J.flag = 1;
-    __threadfence_system();
-  }
+  if (s_wait[0] && threadIdx.x == 0) give_up(J, R, full, s_issued, waits, wait);
 }
 
 template <int PER_SM>
 __global__ void __launch_bounds__(kScThreads, PER_SM) k_prod_add_staged(const ProdJob* __restrict__ jobs, int count,
-                                                                        uint32_t smem, int* __restrict__ timeout) {
+                                                                        uint32_t smem, const __grid_constant__ ProdWaits waits) {
   const AddWork w = add_work(jobs, count, PER_SM);
   const ProdJob& J = jobs[w.job];
-  if (J.variant == kVariantFFT) add_staged<kVariantFFT>(J, w.x, w.t, w.g, smem, timeout);
-  else add_staged<kVariantFWHT>(J, w.x, w.t, w.g, smem, timeout);
+  if (J.variant == kVariantFFT) add_staged<kVariantFFT>(J, w.x, w.t, w.g, smem, waits);
+  else add_staged<kVariantFWHT>(J, w.x, w.t, w.g, smem, waits);
 }
 
 // Lane form: thread = NB buckets (sums in registers); for row i bucket m adds
 // the run of entries of h2 = m - h1(i) (FWHT: m ^ h1(i)).  The sorted columns
 // of the block and the rows are in shared memory.
 template <int VARIANT, int NB>
-__device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t smem, int* timeout) {
+__device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t smem, const ProdWaits& waits) {
   extern __shared__ __align__(128) unsigned char ssm[];
   __shared__ uint64_t full[8], empty[8];
-  __shared__ int s_abort;
+  __shared__ int s_wait[2];
+  __shared__ unsigned s_issued;
   constexpr uint32_t b = 512u * NB;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* es = reinterpret_cast<uint32_t*>(ssm);                         // kScCols entries
@@ -483,16 +491,18 @@ __device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t s
   R.row_bytes = (((uint32_t)min((int64_t)kScCols, J.n_b) + 15u) & ~15u) * 8u;
   R.stages = (int)min(8u, (smem - list_bytes) / R.row_bytes);
   if (tid == 0) {
-    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], kScWin); }
-    s_abort = 0;
+    for (int s = 0; s < R.stages; ++s) { bar_init(&full[s], 1 + waits.extra); bar_init(&empty[s], kScWin); }
+    s_wait[0] = 0;
+    s_wait[1] = waits.limit_us;
+    s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  volatile int* abort = &s_abort;
+  volatile int* wait = s_wait;
   const int64_t per = (J.n_a + J.G - 1) / J.G;
   const int64_t ib = (int64_t)g * per, ie = min(ib + per, J.n_a);
   if (warp == kScWin) {
-    if (lane == 0) produce_rows(J, R, full, empty, ib, ie, abort);
+    if (lane == 0) s_issued = produce_rows(J, R, full, empty, ib, ie, wait);
   } else {
     const uint32_t* cA = J.codesA + (size_t)t * J.n_a;
     double acc[NB];
@@ -515,7 +525,7 @@ __device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t s
         for (int r = 0; r < rows; ++r) {
           const uint32_t c1 = __shfl_sync(0xffffffffu, codes, r);
           const uint32_t h1 = c1 & (b - 1);
-          ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, abort));
+          ok = __all_sync(0xffffffffu, bar_wait(&full[st], ph, wait));
           if (!ok) break;
           const char* row = reinterpret_cast<const char*>(R.base) + st * R.row_bytes;
 #pragma unroll
@@ -541,20 +551,16 @@ __device__ __noinline__ void add_lane(const ProdJob& J, int t, int g, uint32_t s
     for (int q = 0; q < NB; ++q) out[q * 512 + tid] = acc[q];
   }
   __syncthreads();
-  if (s_abort && tid == 0) {
-    *timeout = 1;
-    *J.flag = 1;
-    __threadfence_system();
-  }
+  if (s_wait[0] && tid == 0) give_up(J, R, full, s_issued, waits, wait);
 }
 
 template <int NB>
 __global__ void __launch_bounds__(kScThreads, 1) k_prod_add_lane(const ProdJob* __restrict__ jobs, int count,
-                                                                 uint32_t smem, int* __restrict__ timeout) {
+                                                                 uint32_t smem, const __grid_constant__ ProdWaits waits) {
   const AddWork w = add_work(jobs, count, NB == 1 ? 3 : (NB == 2 ? 4 : 5));
   const ProdJob& J = jobs[w.job];
-  if (J.variant == kVariantFFT) add_lane<kVariantFFT, NB>(J, w.t, w.g, smem, timeout);
-  else add_lane<kVariantFWHT, NB>(J, w.t, w.g, smem, timeout);
+  if (J.variant == kVariantFFT) add_lane<kVariantFFT, NB>(J, w.t, w.g, smem, waits);
+  else add_lane<kVariantFWHT, NB>(J, w.t, w.g, smem, waits);
 }
 
 // Gather form: windows as in the staged form, values from L2.  Entries are read
@@ -850,7 +856,7 @@ void launch_add(K kernel, int64_t ctas, size_t smem, int threads, cudaStream_t s
 
 }  // namespace
 
-void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, cudaStream_t s) {
+void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, int* flag, cudaStream_t s) {
   if (count <= 0) return;
   ProfScope prof("finalize", s);
   int64_t ctas[kAddClasses] = {};
@@ -861,14 +867,13 @@ void launch_product_add(const ProdJob* hJobs, const ProdJob* dJobs, int count, c
     ctas[c] += (int64_t)J.add_x * J.d * J.G;
     smem[c] = std::max(smem[c], c == 0 ? ((size_t)kGaWarps << J.logW) * 8 : add_smem(J));
   }
-  int* flag = nullptr;
-  product_timeout_flag(&flag);
+  const ProdWaits waits = product_waits(flag, "add");
   launch_add(k_prod_add_gather, ctas[0], smem[0], kGaWarps * 32, s, dJobs, count);
-  launch_add(k_prod_add_staged<1>, ctas[1], smem[1], kScThreads, s, dJobs, count, (uint32_t)smem[1], flag);
-  launch_add(k_prod_add_staged<2>, ctas[2], smem[2], kScThreads, s, dJobs, count, (uint32_t)smem[2], flag);
-  launch_add(k_prod_add_lane<1>, ctas[3], smem[3], kScThreads, s, dJobs, count, (uint32_t)smem[3], flag);
-  launch_add(k_prod_add_lane<2>, ctas[4], smem[4], kScThreads, s, dJobs, count, (uint32_t)smem[4], flag);
-  launch_add(k_prod_add_lane<4>, ctas[5], smem[5], kScThreads, s, dJobs, count, (uint32_t)smem[5], flag);
+  launch_add(k_prod_add_staged<1>, ctas[1], smem[1], kScThreads, s, dJobs, count, (uint32_t)smem[1], waits);
+  launch_add(k_prod_add_staged<2>, ctas[2], smem[2], kScThreads, s, dJobs, count, (uint32_t)smem[2], waits);
+  launch_add(k_prod_add_lane<1>, ctas[3], smem[3], kScThreads, s, dJobs, count, (uint32_t)smem[3], waits);
+  launch_add(k_prod_add_lane<2>, ctas[4], smem[4], kScThreads, s, dJobs, count, (uint32_t)smem[4], waits);
+  launch_add(k_prod_add_lane<4>, ctas[5], smem[5], kScThreads, s, dJobs, count, (uint32_t)smem[5], waits);
   int64_t db = 0;
   for (int i = 0; i < count; ++i) db = std::max<int64_t>(db, (int64_t)hJobs[i].d << hJobs[i].log2b);
   count_launch();

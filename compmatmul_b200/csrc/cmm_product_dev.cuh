@@ -29,31 +29,31 @@ __device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait: two seconds on the device's clock (a count of polls would not
-// do, try_wait itself may suspend the thread for as long as it likes); gives up
-// at once when another role of the CTA has given up
-constexpr uint64_t kWaitNs = 2000000000ull;
+// Bounded wait, by the device's clock (a count of polls would not do, try_wait
+// itself may suspend the thread for as long as it likes).  state: [0] a role of
+// the CTA has given up, upon which the others do at once; [1] limit in us.
+constexpr int kWaitUs = 2000000;
 __device__ __forceinline__ uint64_t clock_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* state) {
   for (int it = 0; it < 64; ++it)
     if (bar_test(bar, parity)) return true;
-  const uint64_t t0 = clock_ns();
+  const uint64_t t0 = clock_ns(), limit = 1000ull * (unsigned)state[1];
   do {
     if (bar_test(bar, parity)) return true;
-    if (*abort) return false;
+    if (state[0]) return false;
     __nanosleep(20);
-  } while (clock_ns() - t0 < kWaitNs);
-  *abort = 1;
+  } while (clock_ns() - t0 < limit);
+  state[0] = 1;
   return false;
 }
 // the same for what is in flight when a CTA gives up
-__device__ __forceinline__ void bar_drain(uint64_t* bar, uint32_t parity) {
-  const uint64_t t0 = clock_ns();
-  while (!bar_test(bar, parity) && clock_ns() - t0 < kWaitNs) __nanosleep(20);
+__device__ __forceinline__ void bar_drain(uint64_t* bar, uint32_t parity, volatile int* state) {
+  const uint64_t t0 = clock_ns(), limit = 1000ull * (unsigned)state[1];
+  while (!bar_test(bar, parity) && clock_ns() - t0 < limit) __nanosleep(20);
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

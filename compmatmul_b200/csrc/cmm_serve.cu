@@ -132,6 +132,7 @@ struct Server {
   std::vector<std::shared_ptr<Request>> ready;  // admitted, not yet in a wave
   std::vector<std::unique_ptr<Wave>> waves;
   std::vector<cudaStream_t> streams;
+  std::vector<std::unique_ptr<WaitFlag>> waits;  // of the wave on each stream
   std::vector<bool> busy;
   cudaStream_t up = nullptr;
   int ctas = 0;
@@ -407,8 +408,8 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
   if (!jobs.empty()) {
     const ProdJob* dj = reinterpret_cast<const ProdJob*>(db + joff);
     launch_product_planes(jobs.data(), dj, (int)jobs.size(), S.cfg.f32 != 0, s);
-    launch_product_gemm(jobs.data(), dj, (int)jobs.size(), S.cfg.f32 != 0, s);
-    launch_product_add(jobs.data(), dj, (int)jobs.size(), s);
+    launch_product_gemm(jobs.data(), dj, (int)jobs.size(), S.cfg.f32 != 0, S.waits[(size_t)si]->dev(), s);
+    launch_product_add(jobs.data(), dj, (int)jobs.size(), S.waits[(size_t)si]->dev(), s);
   }
   for (auto& qp : reqs) {
     Request& q = *qp;
@@ -428,11 +429,12 @@ void launch_wave(Server& S, std::vector<std::shared_ptr<Request>> reqs, int si) 
 }
 
 void finish_wave(Server& S, std::unique_ptr<Wave>& W) {
-  if (product_timed_out()) throw runtime_error("product sketch: a wait ran out");
+  const bool ran_out = S.waits[(size_t)W->stream]->take();  // of this wave's product sketches
   const auto now = Clock::now();
   for (auto& qp : W->reqs) {
     Request& q = *qp;
-    std::memcpy(q.r.p, q.stage, (size_t)q.r.d * (size_t)q.r.b * 8);
+    if (ran_out && q.product) q.error = "product sketch: a wait ran out";
+    else std::memcpy(q.r.p, q.stage, (size_t)q.r.d * (size_t)q.r.b * 8);
     S.pinned.put(q.stage, q.stage_cls);
     q.stage = nullptr;
     cudaEventDestroy(q.prepared);
@@ -549,6 +551,7 @@ Server* server_create(const cmm_server_config* cfg) {
     cudaStream_t s;
     CMM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     S->streams.push_back(s);
+    S->waits.emplace_back(new WaitFlag());
     S->busy.push_back(false);
   }
   S->ctas = batch_resident_ctas(cfg->f32 != 0);
@@ -653,10 +656,12 @@ void server_destroy(Server* S) {
     S->cache.clear();
   }
   cudaStreamSynchronize(S->up);
-  for (cudaStream_t s : S->streams) {
-    cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-  }
+  for (cudaStream_t s : S->streams) cudaStreamSynchronize(s);
+  // what a server that failed still holds is released on its streams
+  S->waves.clear();
+  S->ready.clear();
+  S->incoming.clear();
+  for (cudaStream_t s : S->streams) cudaStreamDestroy(s);
   cudaStream_t up = S->up;
   delete S;  // pinned pool and remaining buffers
   cudaStreamSynchronize(up);

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
   unsigned char* Bs = As + 16 * kUnitA;
   __shared__ uint64_t full[kBufs], empty[kBufs], accfull[2], accempty[2], drain;
   __shared__ uint32_t tmem_base;
-  __shared__ int s_abort;
+  __shared__ int s_wait[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // H128[n][k] at unit k / 8, row n, eight elements of K a store
   for (int e = tid; e < 128 * 16; e += kTcThreads) {
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     for (int s = 0; s < kBufs; ++s) { bar_init(&full[s], 128); bar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { bar_init(&accfull[s], 1); bar_init(&accempty[s], 4); }
     bar_init(&drain, 1);
-    s_abort = 0;
+    s_wait[0] = 0;
+    s_wait[1] = kWaitUs;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // H128 -> visible to the tensor core
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = tmem_base;
-  volatile int* abort = &s_abort;
+  volatile int* wait = s_wait;
   const int64_t step = (int64_t)gridDim.x * kTile;
 
   if (tid < kLoaders) {
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
       load_column(x + e0, c, elements - e0, v);
       block_transform<LOGL>(v);
       const unsigned buf = it % kBufs;
-      if (!__all_sync(0xffffffffu, bar_wait(&empty[buf], ((it / kBufs) & 1u) ^ 1u, abort))) break;
+      if (!__all_sync(0xffffffffu, bar_wait(&empty[buf], ((it / kBufs) & 1u) ^ 1u, wait))) break;
       // neighbouring lanes trade, so that each holds the pair (c, c + 1) of
       // half of the blocks: 4-byte stores, eight lanes 32 contiguous bytes
       unsigned char* dst = Bs + buf * kBufBytes + (c >> 3) * kUnitB + (c & 1) * 16 + ((c & 7) >> 1) * 4;
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     unsigned it = 0;
     for (int64_t e0 = (int64_t)blockIdx.x * kTile; e0 < elements; e0 += step, ++it) {
       const unsigned ab = it & 1u;
-      const bool ok = __all_sync(0xffffffffu, bar_wait(&accfull[ab], (it >> 1) & 1u, abort));
+      const bool ok = __all_sync(0xffffffffu, bar_wait(&accfull[ab], (it >> 1) & 1u, wait));
       if (!ok) break;
       tc_fence_after();
       const int64_t left = elements - e0;
@@ -269,8 +270,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     const uint64_t da = kmajor_desc(smem_u32(As), kUnitA);
     for (int64_t e0 = (int64_t)blockIdx.x * kTile; e0 < elements; e0 += step, ++it) {
       const unsigned buf = it % kBufs, ab = it & 1u;
-      if (!bar_wait(&accempty[ab], ((it >> 1) & 1u) ^ 1u, abort)) break;
-      if (!bar_wait(&full[buf], (it / kBufs) & 1u, abort)) break;
+      if (!bar_wait(&accempty[ab], ((it >> 1) & 1u) ^ 1u, wait)) break;
+      if (!bar_wait(&full[buf], (it / kBufs) & 1u, wait)) break;
       tc_fence_after();
       const uint64_t db = kmajor_desc(smem_u32(Bs + buf * kBufBytes), kUnitB);
 #pragma unroll
@@ -288,10 +289,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     }
   }
   __syncthreads();
-  if (s_abort && tid == kLoaders + 128) {  // the MMAs this CTA issued, before their columns are freed
+  if (s_wait[0] && tid == kLoaders + 128) {  // the MMAs this CTA issued, before their columns are freed
     atomicExch(timeout, 1);
     mma_commit(&drain);
-    bar_drain(&drain, 0);
+    bar_drain(&drain, 0, wait);
   }
   tc_fence_before();
   __syncthreads();
