@@ -276,17 +276,22 @@ static Codes make_codes(const SketchParams& sp, int64_t n_a, int64_t n_b, cudaSt
   return c;
 }
 
-// Bytes for what one chunk of inner indices needs (materialized rows or residue
-// planes), at most `need`: a third of the free device memory, at most 8 GiB,
-// or CMM_MATERIALIZE_BYTES when set (smaller budgets run more chunks).  The
-// free memory is asked for only when the stream-ordered pool does not hold
-// enough already: cudaMemGetInfo takes 80 us and more, and waits for the device.
-static size_t materialize_budget(size_t need) {
+size_t scratch_cap() {
   size_t cap = (size_t)8 << 30;
   if (const char* e = getenv("CMM_MATERIALIZE_BYTES")) {
     const long long v = atoll(e);
     if (v > 0 && (size_t)v < cap) cap = (size_t)v;
   }
+  return cap;
+}
+
+// Bytes for what one chunk of inner indices needs (materialized rows or residue
+// planes), at most `need`: a third of the free device memory and scratch_cap()
+// (smaller budgets run more chunks).  The
+// free memory is asked for only when the stream-ordered pool does not hold
+// enough already: cudaMemGetInfo takes 80 us and more, and waits for the device.
+static size_t materialize_budget(size_t need) {
+  const size_t cap = scratch_cap();
   if (need > cap) need = cap;
   int dev = 0;
   cudaMemPool_t pool;
@@ -350,7 +355,9 @@ static int64_t chunk_len(int64_t k0, int64_t kc, int64_t n_inner, const RowFeed*
 // sizes.
 static bool product_applicable(int variant, bool f32, const SketchParams& sp, int64_t n_a, int64_t n_inner,
                                int64_t n_b) {
-  if (!product_supported(sp.b, n_a, n_inner, n_b)) return false;
+  if (!product_supported(sp.b, n_a, n_inner, n_b) ||
+      prod_plane_bytes(f32, n_a, n_b, std::min<int64_t>(n_inner, 128)) > kProdMaxBytes)
+    return false;
   if (sketch_kernel_choice() == 3) return true;
   if (sketch_kernel_choice() != 0) return false;
   if (sketch_cluster_applicable(variant, f32, sp.b) && (double)n_a * (double)n_b * (double)n_inner < 1e7)
@@ -370,11 +377,12 @@ static double* product_room(double* dC, int64_t n_a, int64_t n_b, const void* dA
   return dC;
 }
 
-// scratch: n_a x n_b doubles for C that no input overlaps, or nullptr.
-static void sketch_product(int variant, bool f32, const SketchParams& sp, const Codes& codes, int64_t n_a,
+// scratch: n_a x n_b doubles for C that no input overlaps, or nullptr.  False,
+// with nothing done, where the device has no memory for C, its planes, residues
+// and partial sketches: the transforms take less.
+static bool sketch_product(int variant, bool f32, const SketchParams& sp, const Codes& codes, int64_t n_a,
                            int64_t n_inner, int64_t n_b, const void* dAT, const void* dB, double* dP, double* scratch,
                            cudaStream_t s, RowFeed* feed) {
-  set_sketch_kernel("product");
   WaitFlag& flag = thread_wait_flag();
   if (flag.take()) throw std::runtime_error("product sketch: a wait ran out in an earlier launch of this thread");
   const size_t elem = f32 ? 4 : 8;
@@ -382,17 +390,25 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
   product_geometry(J, variant, sp.d, sp.b, n_a, n_b, 1, true, num_sms());
   // inner indices per chunk: planes within the budget; rows still arriving
   // from the host: eighths, so that copies and work overlap
-  const size_t per_k = (size_t)prod_moduli(f32) * 256 * (size_t)(J.tiles_a + J.tiles_b);
-  int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget(per_k * (size_t)((n_inner + 127) / 128 * 128)) / per_k));
+  const size_t per_k = prod_plane_bytes(f32, n_a, n_b, 128) / 128;
+  int64_t kc = std::min<int64_t>(kProdMaxK, (int64_t)(materialize_budget(prod_plane_bytes(f32, n_a, n_b, n_inner)) / per_k));
   if (feed) kc = std::min<int64_t>(kc, std::max<int64_t>((n_inner + 7) / 8, 512));
   kc = std::max<int64_t>(kc / 128 * 128, 128);
   kc = std::min<int64_t>(kc, n_inner);
   // panels of C whose residues take at most 2 GiB
-  const int panel = (int)std::max<int64_t>(1, std::min<int64_t>(J.tiles_a, (int64_t)(((size_t)2 << 30) / prod_residue_row(J, f32))));
+  const size_t residues = std::min((size_t)2 << 30, scratch_cap());
+  const int panel = (int)std::max<int64_t>(1, std::min<int64_t>(J.tiles_a, (int64_t)(residues / prod_residue_row(J, f32))));
   J.kc = kc;
   J.tiles_p = panel;
   const size_t work = product_work_bytes(J, f32, !product_usable_c(J, scratch)), lists = product_list_bytes(J);
-  DevBuf mem(work + lists + sizeof(ProdJob), s);  // one allocation for everything
+  DevBuf mem;  // one allocation for everything
+  try {
+    mem = DevBuf(work + lists + sizeof(ProdJob), s);
+  } catch (const std::bad_alloc&) {
+    cudaGetLastError();
+    return false;
+  }
+  set_sketch_kernel("product");
   uint8_t* base = mem.as<uint8_t>();
   product_set_work(J, base, f32, scratch);
   product_set_lists(J, base + work);
@@ -418,6 +434,7 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
     }
   }
   launch_product_add(&J, dJ, 1, flag.dev(), s);
+  return true;
 }
 
 // feed != nullptr: the rows of dAT / dB are still arriving from the host;
@@ -425,10 +442,9 @@ static void sketch_product(int variant, bool f32, const SketchParams& sp, const 
 static void sketch_device(int variant, const SketchParams& sp, const Codes& codes, int64_t n_a,
                           int64_t n_inner, int64_t n_b, const double* dAT, const double* dB,
                           double* dP, cudaStream_t s, RowFeed* feed = nullptr, double* scratch = nullptr) {
-  if (product_applicable(variant, false, sp, n_a, n_inner, n_b)) {
-    sketch_product(variant, false, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed);
+  if (product_applicable(variant, false, sp, n_a, n_inner, n_b) &&
+      sketch_product(variant, false, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed))
     return;
-  }
   const double2* tw = twiddles(sp.b, s);
   const size_t elem = variant == kVariantFFT ? 16 : 8;
   DevBuf scale;
@@ -503,10 +519,9 @@ static void sketch_device_mixed(int variant, const SketchParams& sp, const Codes
                                 int64_t n_a, int64_t n_inner, int64_t n_b, const float* dAT,
                                 const float* dB, double* dP, cudaStream_t s,
                                 RowFeed* feed = nullptr, double* scratch = nullptr) {
-  if (product_applicable(variant, true, sp, n_a, n_inner, n_b)) {
-    sketch_product(variant, true, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed);
+  if (product_applicable(variant, true, sp, n_a, n_inner, n_b) &&
+      sketch_product(variant, true, sp, codes, n_a, n_inner, n_b, dAT, dB, dP, scratch, s, feed))
     return;
-  }
   if (!(n_inner > 0 && sketch_mixed_applicable(variant, sp.b))) {
     if (feed) feed->wait_all(s);
     DevBuf A64((size_t)n_inner * n_a * 8, s), B64((size_t)n_inner * n_b * 8, s);

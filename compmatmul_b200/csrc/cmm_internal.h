@@ -259,6 +259,10 @@ void topk_dense(const double* dC, int64_t n_a, int64_t n_b, int K, uint32_t* dI,
 
 int num_sms();
 
+// Most bytes of device memory for what is made in chunks (materialized rows,
+// residue planes, residues): 8 GiB, or CMM_MATERIALIZE_BYTES when set and smaller.
+size_t scratch_cap();
+
 inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
   const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
   return na > 0 && nb > 0 && x < y + nb && y < x + na;

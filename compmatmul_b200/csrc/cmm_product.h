@@ -59,6 +59,14 @@ constexpr int64_t kProdMaxEntries = (int64_t)1 << 30;
 bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b);
 bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone);
 
+// bytes of the residue planes of a chunk of k inner indices
+inline size_t prod_plane_bytes(bool f32, int64_t n_a, int64_t n_b, int64_t k) {
+  return (size_t)prod_moduli(f32) * 256 * (size_t)((n_a + 255) / 256 + (n_b + 255) / 256) * (size_t)((k + 127) / 128 * 128);
+}
+// A launch's planes (of 128 inner indices at least), and the partial sketches
+// of its row groups (of one at least), take no more than this.
+constexpr size_t kProdMaxBytes = (size_t)8 << 30;
+
 // Sizes, tiles and additions of a job of kc inner indices (kc <= kProdMaxK)
 // with all rows of C in one panel.  alone: the job has the device for itself
 // (row groups to fill it); otherwise the row groups follow from the job's

@@ -655,7 +655,8 @@ __global__ void __launch_bounds__(256) k_prod_reduce(const ProdJob* __restrict__
 
 bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
   return n_inner > 0 && n_a > 0 && n_b > 0 && n_a <= 0x7fffffff && n_b <= 0x7fffffff && n_a * n_b <= kProdMaxEntries &&
-         b >= 512 && (b <= 65536 || n_b <= 131072);  // what the forms of the additions take
+         b >= 512 && (b <= 65536 || n_b <= 131072) &&  // what the forms of the additions take
+         n_b <= 65535ll * kScCols;                     // blocks of columns in a launch
 }
 
 // Shared memory of a staged or lane CTA: its windows or lists and a ring of up
@@ -726,7 +727,9 @@ void product_geometry(ProdJob& J, int variant, int d, int b, int64_t n_a, int64_
       G = (n_a + 255) / 256;
     }
   }
-  J.G = (int)std::max<int64_t>(1, std::min(G, most));
+  // (16384 rows of 16384 columns, b = 2^24, d = 9: 64 groups would take 77 GB)
+  const int64_t fit = (int64_t)(kProdMaxBytes / ((size_t)d * (size_t)b * 8));
+  J.G = (int)std::max<int64_t>(1, std::min({G, most, fit}));
 }
 
 // --------------------------------------------------------------- device memory
