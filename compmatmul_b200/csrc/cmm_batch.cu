@@ -764,6 +764,11 @@ struct BatchPlan {
   std::vector<int> by_product;        // per product: 1 if it is one of them
   std::vector<char> shared_c;         // per product: its dense output overlaps another output
   std::vector<ProdJob> pjobs;
+  struct PWhere {
+    int product;
+    size_t work, lists;  // offsets in pmem and plists
+  };
+  std::vector<PWhere> pwhere;  // per job
   std::vector<std::pair<int, int>> pruns;  // [first, last) jobs
   DevBuf pmem, plists, pdev, pflags;
   std::unique_ptr<WaitFlag> waits;
@@ -915,55 +920,83 @@ bool outputs_meet_inputs(BatchPlan& B) {
   return meet;
 }
 
-// The jobs of the products that take the product sketch, their memory and
-// their sorted columns.  A run's work space takes at most a third of the free
-// device memory or 8 GiB; C is formed in the product's own dense output where
-// there is one.
-void make_product_jobs(BatchPlan& B, cudaStream_t s) {
+// Chooses the products that take the product sketch, in by_product, and reserves
+// their memory.  They run in groups that share a work space of at most a third of
+// the free device memory or scratch_cap(); C is formed in the product's own dense
+// output where there is one.  A product that needs more by itself takes the
+// transforms, and all do when the memory is not to be had.
+void reserve_product_jobs(BatchPlan& B, cudaStream_t s) {
+  B.by_product.assign((size_t)B.count, 0);
+  B.shared_c.assign((size_t)B.count, 0);
+  // (they write sketches and dense outputs while other products' inputs are still
+  // to be read, so none where those share memory)
+  if (outputs_meet_inputs(B)) return;
   std::vector<int> order;
-  for (int i = 0; i < B.count; ++i)
-    if (B.by_product[(size_t)i]) order.push_back(i);
+  for (int i = 0; i < B.count; ++i) {
+    const cmm_batch_product& q = B.prods[(size_t)i];
+    if (q.n_inner <= kProdMaxK && product_supported(q.b, q.n_a, q.n_inner, q.n_b) &&
+        product_faster(q.variant, B.f32, q.d, q.b, q.n_a, q.n_inner, q.n_b, false))
+      order.push_back(i);
+  }
   if (order.empty()) return;
-  B.waits.reset(new WaitFlag());
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return B.prods[(size_t)a].n_inner > B.prods[(size_t)b].n_inner; });
   size_t free_b = 0, total_b = 0;
   CMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const size_t budget = std::min<size_t>(free_b / 3, (size_t)8 << 30);
+  const size_t budget = std::min<size_t>(free_b / 3, scratch_cap());
   size_t lists = 0, work = 0, most = 0;
-  std::vector<size_t> at_work, at_list;
-  for (size_t k = 0; k < order.size(); ++k) {
-    const cmm_batch_product& q = B.prods[(size_t)order[k]];
+  for (int i : order) {
+    const cmm_batch_product& q = B.prods[(size_t)i];
     ProdJob J{};
     product_geometry(J, q.variant, q.d, q.b, q.n_a, q.n_b, q.n_inner, false, num_sms());
-    double* room = B.shared_c[(size_t)order[k]] ? nullptr : q.C;
-    const size_t need = product_work_bytes(J, B.f32, !product_usable_c(J, room));
+    const size_t need = product_work_bytes(J, B.f32, !product_usable_c(J, B.shared_c[(size_t)i] ? nullptr : q.C));
+    if (need > budget) continue;
+    const int k = (int)B.pjobs.size();
     if (B.pruns.empty() || work + need > budget) {
-      B.pruns.push_back({(int)k, (int)k});
+      B.pruns.push_back({k, k});
       work = 0;
     }
-    J.A = q.AT;
-    J.B = q.B;
-    J.codesA = B.codes.as<uint32_t>() + B.off_codesA[(size_t)order[k]];
-    J.codesB = B.codes.as<uint32_t>() + B.off_codesB[(size_t)order[k]];
-    J.p = q.p;
-    at_work.push_back(work);
-    at_list.push_back(lists);
+    B.pwhere.push_back({i, work, lists});
     work += need;
     most = std::max(most, work);
     lists += product_list_bytes(J);
     B.pjobs.push_back(J);
-    B.pruns.back().second = (int)k + 1;
+    B.pruns.back().second = k + 1;
   }
-  B.pmem = DevBuf(most, s);
-  B.plists = DevBuf(lists, s);
-  B.pdev = DevBuf(B.pjobs.size() * sizeof(ProdJob), s);
-  B.pflags = DevBuf(B.pjobs.size() * sizeof(int), s);
-  for (size_t k = 0; k < order.size(); ++k) {
+  if (B.pjobs.empty()) return;
+  try {
+    B.pmem = DevBuf(most, s);
+    B.plists = DevBuf(lists, s);
+    B.pdev = DevBuf(B.pjobs.size() * sizeof(ProdJob), s);
+    B.pflags = DevBuf(B.pjobs.size() * sizeof(int), s);
+  } catch (const std::bad_alloc&) {
+    cudaGetLastError();
+    B.pmem = DevBuf();
+    B.plists = DevBuf();
+    B.pdev = DevBuf();
+    B.pjobs.clear();
+    B.pruns.clear();
+    B.pwhere.clear();
+    return;
+  }
+  B.waits.reset(new WaitFlag());
+  for (const auto& w : B.pwhere) B.by_product[(size_t)w.product] = 1;
+}
+
+// Their jobs and sorted columns, once the hash codes are there.
+void make_product_jobs(BatchPlan& B, cudaStream_t s) {
+  if (B.pjobs.empty()) return;
+  for (size_t k = 0; k < B.pjobs.size(); ++k) {
+    const auto& w = B.pwhere[k];
+    const cmm_batch_product& q = B.prods[(size_t)w.product];
     ProdJob& J = B.pjobs[k];
-    product_set_work(J, B.pmem.as<uint8_t>() + at_work[k], B.f32,
-                     B.shared_c[(size_t)order[k]] ? nullptr : B.prods[(size_t)order[k]].C);
-    product_set_lists(J, B.plists.as<uint8_t>() + at_list[k]);
+    J.A = q.AT;
+    J.B = q.B;
+    J.codesA = B.codes.as<uint32_t>() + B.off_codesA[(size_t)w.product];
+    J.codesB = B.codes.as<uint32_t>() + B.off_codesB[(size_t)w.product];
+    J.p = q.p;
+    product_set_work(J, B.pmem.as<uint8_t>() + w.work, B.f32, B.shared_c[(size_t)w.product] ? nullptr : q.C);
+    product_set_lists(J, B.plists.as<uint8_t>() + w.lists);
     J.flag = B.pflags.as<int>() + k;
   }
   for (const auto& run : B.pruns) product_layout(B.pjobs.data() + run.first, run.second - run.first, B.f32);
@@ -1079,17 +1112,7 @@ BatchPlan* batch_create(const cmm_batch_product* products, int count, bool f32, 
   B->ctas = f32 ? resident_ctas<float>() : resident_ctas<double>();
   B->tw4096 = twiddles(1 << kBFftLog, s);
 
-  // ---- products whose sketch is taken from the product itself
-  // (they write sketches and dense outputs while other products' inputs are still
-  // to be read, so none where those share memory)
-  B->by_product.assign((size_t)count, 0);
-  B->shared_c.assign((size_t)count, 0);
-  const bool apart = !outputs_meet_inputs(*B);
-  for (int i = 0; i < count && apart; ++i) {
-    const cmm_batch_product& q = B->prods[(size_t)i];
-    B->by_product[(size_t)i] = q.n_inner <= kProdMaxK && product_supported(q.b, q.n_a, q.n_inner, q.n_b) &&
-                               product_faster(q.variant, f32, q.d, q.b, q.n_a, q.n_inner, q.n_b, false);
-  }
+  reserve_product_jobs(*B, s);
 
   // ---- validation, hash parameters, buffer offsets
   std::vector<uint8_t> blob;

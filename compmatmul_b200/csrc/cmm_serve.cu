@@ -149,7 +149,7 @@ namespace {
 
 // shape-dependent parts of a request; identical for a request alone and in
 // any mix
-void geometry(Request& q, bool f32) {
+void geometry(Request& q, bool f32, size_t cap) {
   const cmm_request& r = q.r;
   q.log2b = ilog2i(r.b);
   q.product = r.n_inner <= kProdMaxK && product_supported(r.b, r.n_a, r.n_inner, r.n_b) &&
@@ -165,7 +165,8 @@ void geometry(Request& q, bool f32) {
     need += product_work_bytes(q.job, f32, true) + round256(d * (size_t)r.b * 8);
     q.logL = -1;  // no slab: tells the cached lists of the two forms apart
     q.need = need;
-    return;
+    if (need <= cap) return;
+    q.product = false;  // the transforms take less memory
   }
   const int lmax = r.variant == kVariantFFT ? kBatchFftLog : kBatchWhtLog;
   int logL = std::min(q.log2b, lmax), radix = 8, tc = 1;
@@ -598,7 +599,7 @@ uint64_t server_submit(Server* S, const cmm_request* req) {
   if (!r.p) throw invalid_argument("p is null");
   auto q = std::make_shared<Request>();
   q->r = r;
-  geometry(*q, S->cfg.f32 != 0);
+  geometry(*q, S->cfg.f32 != 0, S->cfg.mem_cap_bytes);
   if (q->need > S->cfg.mem_cap_bytes)
     throw invalid_argument("request needs " + std::to_string(q->need) + " device bytes, above the admission cap of " +
                            std::to_string(S->cfg.mem_cap_bytes));

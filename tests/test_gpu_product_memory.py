@@ -122,6 +122,61 @@ def test_panels_and_chunks(gpu, monkeypatch, variant, f32):
     assert (parts - whole).abs().max() <= (1e-7 if f32 else 1e-13) * whole.abs().max()
 
 
+def random(k, n_a, n_b, seed):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn((k, n), device="cuda", generator=g) for n in (n_a, n_b)]
+
+
+def test_request_between_the_needs_of_both_routes(gpu):
+    """1024-square FP32 requests, b = 8192, d = 5: the product sketch holds 35 MB, the
+    transforms 12.  Under a cap of 20 MB they are served by the transforms."""
+    from compmatmul_b200 import device
+    from compmatmul_b200.serve import Server
+    AT, B = random(1024, 1024, 1024, 5)
+    ref = device.compressed_product(AT.double(), B.double(), 5, 8192, 9).cpu().numpy()
+    got = []
+    for cap in (20 << 20, 1 << 30):
+        srv = Server(mem_cap_bytes=cap, f32=True, streams=2, max_wave=4)
+        ids = [srv.submit(AT, B, 5, 8192, 9) for _ in range(3)]
+        got.append([srv.result(i, timeout=60) for i in ids])
+        st = srv.stats()
+        srv.close()
+        assert (st["max_mem_in_use"] > 20 << 20) == (cap > 20 << 20), st
+    for p in got[0] + got[1]:
+        assert np.abs(p - ref).max() <= 2e-5 * np.abs(ref).max()
+        assert np.array_equal(p, got[0][0]) or np.array_equal(p, got[1][0])
+
+
+def test_plan_with_products_above_the_scratch_limit(gpu, monkeypatch):
+    """A limit that the small product's work space fits and the large one's does
+    not: the large one takes the transforms."""
+    import torch
+
+    from compmatmul_b200.batch import BatchPlan
+    prods = [dict(AT=m[0], B=m[1], d=5, b=8192, seed=3 + i) for i, m in
+             enumerate([random(200, 300, 310, 1), random(1500, 1024, 1024, 2), random(200, 310, 300, 3)])]
+
+    def run(limit):
+        if limit:
+            monkeypatch.setenv("CMM_MATERIALIZE_BYTES", str(limit))
+        plan = BatchPlan(prods, f32=True, tune=False)
+        plan.run()
+        torch.cuda.synchronize()
+        out = [(q["p"].clone(), q["C"].clone()) for q in plan.products]
+        plan.close()
+        return out
+
+    whole, some, none = run(0), run(16 << 20), run(1 << 20)  # (the small ones need 5 MB each, the large one 60)
+    for k in range(3):
+        same = torch.equal(whole[k][0], some[k][0])
+        assert same == (k != 1)  # the same route gives the same bits
+        assert not torch.equal(whole[k][0], none[k][0])
+        for a, b, c in zip(whole[k], some[k], none[k]):
+            for x in (b, c):
+                assert (a - x).abs().max() <= 2e-5 * whole[k][0].abs().max()
+
+
 if __name__ == "__main__":
     sys.path.insert(0, os.getcwd())
     {"full": full, "buckets": buckets}[sys.argv[1]]()
