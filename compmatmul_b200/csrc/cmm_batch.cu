@@ -934,9 +934,7 @@ void reserve_product_jobs(BatchPlan& B, cudaStream_t s) {
   std::vector<int> order;
   for (int i = 0; i < B.count; ++i) {
     const cmm_batch_product& q = B.prods[(size_t)i];
-    if (q.n_inner <= kProdMaxK && product_supported(q.b, q.n_a, q.n_inner, q.n_b) &&
-        product_faster(q.variant, B.f32, q.d, q.b, q.n_a, q.n_inner, q.n_b, false))
-      order.push_back(i);
+    if (product_among_others(q.variant, B.f32, q.d, q.b, q.n_a, q.n_inner, q.n_b)) order.push_back(i);
   }
   if (order.empty()) return;
   std::stable_sort(order.begin(), order.end(),

@@ -310,7 +310,7 @@ static size_t materialize_budget(size_t need) {
 // and the residue segments fit in shared memory; false -> the slab kernels.
 // CMM_SKETCH_KERNELS = cluster | slab | product forces one family where it applies
 // (for comparisons); unset or "auto" takes the measured-faster choice.
-static int sketch_kernel_choice() {
+int sketch_kernel_choice() {
   static const int choice = [] {
     const char* e = getenv("CMM_SKETCH_KERNELS");
     if (e && !strcmp(e, "cluster")) return 1;

@@ -262,6 +262,10 @@ int num_sms();
 // Most bytes of device memory for what is made in chunks (materialized rows,
 // residue planes, residues): 8 GiB, or CMM_MATERIALIZE_BYTES when set and smaller.
 size_t scratch_cap();
+// Kernels that CMM_SKETCH_KERNELS asks for (read once): 0 the faster ones, 1
+// cluster, 2 slab, 3 product; for batch plans and serving 1 and 2 are their own
+// transform kernel.
+int sketch_kernel_choice();
 
 inline bool overlap(const void* a, size_t na, const void* b, size_t nb) {
   const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);

@@ -868,4 +868,10 @@ bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_
          transforms_us(variant, f32, d, b, (double)n_inner, (double)(n_a + n_b), alone);
 }
 
+bool product_among_others(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
+  const int choice = sketch_kernel_choice();
+  return (choice == 0 || choice == 3) && n_inner <= kProdMaxK && product_supported(b, n_a, n_inner, n_b) &&
+         (choice == 3 || product_faster(variant, f32, d, b, n_a, n_inner, n_b, false));
+}
+
 }  // namespace cmm

@@ -58,6 +58,8 @@ constexpr int64_t kProdMaxEntries = (int64_t)1 << 30;
 // be faster than the transforms (alone: with both forms' fixed costs).
 bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b);
 bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone);
+// whether a product of a batch plan or a request takes it
+bool product_among_others(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b);
 
 // bytes of the residue planes of a chunk of k inner indices
 inline size_t prod_plane_bytes(bool f32, int64_t n_a, int64_t n_b, int64_t k) {

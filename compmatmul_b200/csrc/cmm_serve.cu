@@ -152,8 +152,7 @@ namespace {
 void geometry(Request& q, bool f32, size_t cap) {
   const cmm_request& r = q.r;
   q.log2b = ilog2i(r.b);
-  q.product = r.n_inner <= kProdMaxK && product_supported(r.b, r.n_a, r.n_inner, r.n_b) &&
-              product_faster(r.variant, f32, r.d, r.b, r.n_a, r.n_inner, r.n_b, false);
+  q.product = product_among_others(r.variant, f32, r.d, r.b, r.n_a, r.n_inner, r.n_b);
   if (q.product) {
     product_geometry(q.job, r.variant, r.d, r.b, r.n_a, r.n_b, r.n_inner, false, num_sms());
     const size_t esz = f32 ? 4 : 8, d = (size_t)r.d;
