@@ -9,9 +9,9 @@
 // walsh_wak in natural order; golden values in tests.cpp:621-671).
 //
 // Rows are contiguous, so both forms work on tiles of 8192 elements (8192 / L
-// rows), seen as 64 blocks of 128: H_L = H_{L/128} (x) H_128, whose factors
-// commute.
-//   * Index bits 7 and up: thread c holds element c of all 64 blocks in
+// rows; one row where there are few), seen as 64 blocks of 128: H_L = H_{L/128}
+// (x) H_128, whose factors commute.
+//   * Index bits 7 and up: thread c holds element c of all blocks in
 //     registers, as they come from global memory (coalesced over c), and runs
 //     the L/128-point transforms there.
 //   * Index bits 0-6: Y = H_128 X for the 128 x 64 matrix of the tile, on the
@@ -49,27 +49,28 @@
 namespace cmm {
 namespace {
 
-constexpr int kTile = 8192;   // elements per tile: 64 blocks of 128
-constexpr int kBlocks = 64;
+// A tile is NB blocks of 128: 64, or those of one row where there are few rows
+// (wht_launch_rows).
 
-// element c of the tile's 64 blocks (zero beyond `left` elements)
-__device__ __forceinline__ void load_column(const float* __restrict__ src, int c, int64_t left, float (&v)[kBlocks]) {
-  if (left >= kTile) {
+// element c of the tile's blocks (zero beyond `left` elements)
+template <int NB>
+__device__ __forceinline__ void load_column(const float* __restrict__ src, int c, int64_t left, float (&v)[NB]) {
+  if (left >= NB * 128) {
 #pragma unroll
-    for (int g = 0; g < kBlocks; ++g) v[g] = __ldcs(src + g * 128 + c);
+    for (int g = 0; g < NB; ++g) v[g] = __ldcs(src + g * 128 + c);
   } else {
 #pragma unroll
-    for (int g = 0; g < kBlocks; ++g) v[g] = g * 128 + c < left ? __ldcs(src + g * 128 + c) : 0.f;
+    for (int g = 0; g < NB; ++g) v[g] = g * 128 + c < left ? __ldcs(src + g * 128 + c) : 0.f;
   }
 }
 // index bits 7 and up: transforms over the F = L / 128 blocks of each row
-template <int LOGL>
-__device__ __forceinline__ void block_transform(float (&v)[kBlocks]) {
+template <int LOGL, int NB>
+__device__ __forceinline__ void block_transform(float (&v)[NB]) {
   constexpr int F = 1 << (LOGL - 7);
 #pragma unroll
   for (int h = 1; h < F; h <<= 1)
 #pragma unroll
-    for (int g = 0; g < kBlocks; ++g)
+    for (int g = 0; g < NB; ++g)
       if (!(g & h)) {
         const float a = v[g], b = v[g + h];
         v[g] = a + b;
@@ -78,40 +79,42 @@ __device__ __forceinline__ void block_transform(float (&v)[kBlocks]) {
 }
 
 // ---------------------------------------------------------------- CUDA cores
-// 128 threads per tile; the 128-point transforms as 64-point transforms in
-// registers (thread = half a block, through shared memory) and one exchange
-// between neighbouring lanes.  X[g][c] at g 130 + c + c / 64: both access
-// patterns touch every bank once.
+// 128 threads per tile; the 128-point transforms as NB-point transforms in
+// registers (TP = 128 / NB threads a block, through shared memory) and exchanges
+// between those neighbouring lanes.  X[g][c] at g (128 + TP) + c + c / NB: both
+// access patterns touch every bank once (NB = 16: one of them twice).
 constexpr int kCcThreads = 128;
-__device__ __forceinline__ int cc_at(int g, int c) { return g * 130 + c + (c >> 6); }
 
-template <int LOGL>
+template <int LOGL, int NB>
 __global__ void __launch_bounds__(kCcThreads, 5) k_wht_rows(const float* x, float* y, int64_t elements) {
-  __shared__ float X[kBlocks * 130];
+  constexpr int TP = 128 / NB, kTile = NB * 128, kRow = 128 + TP;
+  __shared__ float X[NB * kRow];
   const int tid = threadIdx.x;
   for (int64_t e0 = (int64_t)blockIdx.x * kTile; e0 < elements; e0 += (int64_t)gridDim.x * kTile) {
     const int64_t left = elements - e0;
-    float v[kBlocks];
-    load_column(x + e0, tid, left, v);
-    block_transform<LOGL>(v);
+    float v[NB];
+    load_column<NB>(x + e0, tid, left, v);
+    block_transform<LOGL, NB>(v);
 #pragma unroll
-    for (int g = 0; g < kBlocks; ++g) X[cc_at(g, tid)] = v[g];
+    for (int g = 0; g < NB; ++g) X[g * kRow + tid + tid / NB] = v[g];
     __syncthreads();
-    const int g = tid >> 1, half = tid & 1;
+    const int part = tid % TP, at = tid / TP * kRow + part * (NB + 1);
 #pragma unroll
-    for (int j = 0; j < 64; ++j) v[j] = X[g * 130 + half * 65 + j];
-    dev::whtr<float, 64>(v);
+    for (int j = 0; j < NB; ++j) v[j] = X[at + j];
+    dev::whtr<float, NB>(v);
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      const float o = __shfl_xor_sync(0xffffffffu, v[j], 1);
-      v[j] = half ? o - v[j] : v[j] + o;
-    }
+    for (int h = 1; h < TP; h <<= 1)
 #pragma unroll
-    for (int j = 0; j < 64; ++j) X[g * 130 + half * 65 + j] = v[j];
+      for (int j = 0; j < NB; ++j) {
+        const float o = __shfl_xor_sync(0xffffffffu, v[j], h);
+        v[j] = part & h ? o - v[j] : v[j] + o;
+      }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) X[at + j] = v[j];
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < kBlocks; ++q)
-      if (left >= kTile || q * 128 + tid < left) __stcs(y + e0 + q * 128 + tid, X[cc_at(q, tid)]);
+    for (int q = 0; q < NB; ++q)
+      if (left >= kTile || q * 128 + tid < left) __stcs(y + e0 + q * 128 + tid, X[q * kRow + tid + tid / NB]);
     __syncthreads();
   }
 }
@@ -131,16 +134,17 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t saddr, int unit) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(unit >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
 }
 // instruction descriptor, kind::f16: D FP32 (bits 4-5 = 1), A and B BF16 (bits
-// 7-9 and 10-12 = 1), both K-major, N = 64 (>> 3 at bit 17), M = 128 (>> 4 at
-// bit 24)
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+// 7-9 and 10-12 = 1), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
+template <int N>
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)N >> 3) << 17) | ((128u >> 4) << 24);
 
+template <int N>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate));
+      "l"(adesc), "l"(bdesc), "r"(kIdesc<N>), "r"(accumulate));
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -172,8 +176,9 @@ __device__ __forceinline__ uint32_t take_bf16x2(float& a, float& b) {
   return w;
 }
 
-template <int LOGL>
+template <int LOGL, int NB>
 __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, float* y, int64_t elements, int* timeout) {
+  constexpr int kTile = NB * 128;
   extern __shared__ __align__(128) unsigned char wsm[];
   unsigned char* As = reinterpret_cast<unsigned char*>(((uintptr_t)wsm + 127) & ~(uintptr_t)127);
   unsigned char* Bs = As + 16 * kUnitA;
@@ -218,16 +223,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     const int w = tid >> 7, c = tid & 127;
     unsigned it = w;
     for (int64_t e0 = ((int64_t)blockIdx.x + (int64_t)w * gridDim.x) * kTile; e0 < elements; e0 += 2 * step, it += 2) {
-      float v[kBlocks];
-      load_column(x + e0, c, elements - e0, v);
-      block_transform<LOGL>(v);
+      float v[NB];
+      load_column<NB>(x + e0, c, elements - e0, v);
+      block_transform<LOGL, NB>(v);
       const unsigned buf = it % kBufs;
       if (!__all_sync(0xffffffffu, bar_wait(&empty[buf], ((it / kBufs) & 1u) ^ 1u, wait))) break;
       // neighbouring lanes trade, so that each holds the pair (c, c + 1) of
       // half of the blocks: 4-byte stores, eight lanes 32 contiguous bytes
       unsigned char* dst = Bs + buf * kBufBytes + (c >> 3) * kUnitB + (c & 1) * 16 + ((c & 7) >> 1) * 4;
 #pragma unroll
-      for (int g = 0; g < kBlocks; g += 2) {
+      for (int g = 0; g < NB; g += 2) {
         const float o = __shfl_xor_sync(0xffffffffu, c & 1 ? v[g] : v[g + 1], 1);
         float a = c & 1 ? o : v[g], b = c & 1 ? v[g + 1] : o;
 #pragma unroll
@@ -247,19 +252,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
       const int64_t left = elements - e0;
       float* out = y + e0 + 32 * q + lane;
 #pragma unroll
-      for (int n0 = 0; n0 < kBlocks; n0 += 32) {
+      for (int n0 = 0; n0 < NB; n0 += 32) {  // (NB = 16: the other columns are not used)
         uint32_t a[32], b[32];
         const uint32_t t = tbase + ((uint32_t)(32 * q) << 16) + ab * 128u + n0;
         tmem_ld32(t, a);
         tmem_ld32(t + 64, b);
         tmem_ld_wait(a, b);
-        if (n0 + 32 == kBlocks) {  // the accumulators are read
+        if (n0 + 32 >= NB) {  // the accumulators are read
           tc_fence_before();
           __syncwarp();
           if (lane == 0) bar_arrive(&accempty[ab]);
         }
 #pragma unroll
-        for (int u = 0; u < 32; ++u) {
+        for (int u = 0; u < (NB < 32 ? NB : 32); ++u) {
           const int at = (n0 + u) * 128;
           if (left >= kTile || at + 32 * q + lane < left) __stcs(out + at, __uint_as_float(a[u]) + __uint_as_float(b[u]));
         }
@@ -281,7 +286,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
 #pragma unroll
           for (int half = 0; half < 2; ++half) {  // 16 elements of K: two units
             const int u = 2 * (4 * half + k);
-            mma_bf16(tbase + ab * 128u + half * 64u, da + (uint64_t)(u * (kUnitA >> 4)),
+            mma_bf16<NB>(tbase + ab * 128u + half * 64u, da + (uint64_t)(u * (kUnitA >> 4)),
                      db + (uint64_t)(s * (kSplitBytes >> 4) + u * (kUnitB >> 4)), s == 2 && k == 0 ? 0u : 1u);
           }
       mma_commit(&empty[buf]);
@@ -301,17 +306,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wht_rows_tc(const float* x, f
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(256u) : "memory");
 }
 
-template <int LOGL>
+template <int LOGL, int NB>
 void wht_launch(bool tc, const float* x, float* y, int64_t rows, int* timeout, cudaStream_t s) {
-  const int64_t elements = rows << LOGL, tiles = (elements + kTile - 1) / kTile;
+  const int64_t elements = rows << LOGL, tiles = (elements + NB * 128 - 1) / (NB * 128);
   if (tc) {
-    CMM_CUDA(cudaFuncSetAttribute(k_wht_rows_tc<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-    k_wht_rows_tc<LOGL><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kTcThreads, kTcSmem, s>>>(x, y, elements, timeout);
+    CMM_CUDA(cudaFuncSetAttribute(k_wht_rows_tc<LOGL, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
+    k_wht_rows_tc<LOGL, NB><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kTcThreads, kTcSmem, s>>>(x, y, elements, timeout);
   } else {
-    k_wht_rows<LOGL><<<(unsigned)std::min<int64_t>(tiles, (int64_t)num_sms() * 5), kCcThreads, 0, s>>>(x, y, elements);
+    k_wht_rows<LOGL, NB><<<(unsigned)std::min<int64_t>(tiles, (int64_t)num_sms() * 5), kCcThreads, 0, s>>>(x, y, elements);
   }
   CMM_CUDA(cudaGetLastError());
   count_launch();
+}
+// Few rows of 2^11 and 2^12: a tile a row, since four (two) rows one after another
+// in a CTA take longer than side by side, as long as the CTAs are there at once
+// (tensor form: one per SM).  A call with 148 rows of 2^11: CUDA cores 16.6 -> 15.6
+// us, tensor 19.1 -> 17.7; with 500 in the tensor form, 64 blocks a tile take
+// 18.8, 16 take 20.3.
+template <int LOGL>
+void wht_launch_rows(bool tc, const float* x, float* y, int64_t rows, int* timeout, cudaStream_t s) {
+  constexpr int kRowBlocks = 1 << (LOGL - 7);
+  if (rows <= (tc ? 1 : 2) * (int64_t)num_sms()) wht_launch<LOGL, kRowBlocks>(tc, x, y, rows, timeout, s);
+  else wht_launch<LOGL, 64>(tc, x, y, rows, timeout, s);
 }
 
 // host-mapped timeout flag of the calling host thread (one per thread, so
@@ -350,9 +366,9 @@ void wht_rows_f32(const float* x, float* y, int64_t rows, int log2n, int method,
   *hflag = 0;
   const bool tc = method == 1;
   switch (log2n) {
-    case 11: wht_launch<11>(tc, x, y, rows, dflag, s); break;
-    case 12: wht_launch<12>(tc, x, y, rows, dflag, s); break;
-    default: wht_launch<13>(tc, x, y, rows, dflag, s); break;
+    case 11: wht_launch_rows<11>(tc, x, y, rows, dflag, s); break;
+    case 12: wht_launch_rows<12>(tc, x, y, rows, dflag, s); break;
+    default: wht_launch<13, 64>(tc, x, y, rows, dflag, s); break;
   }
   CMM_CUDA(cudaStreamSynchronize(s));
   if (tc) {
