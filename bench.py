@@ -54,6 +54,7 @@ def parse(argv=None):
     ap.add_argument("--e2e-steps", type=int, default=2, help="0 skips the end-to-end legs")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-legs", action="store_true", help="headline workload only")
+    ap.add_argument("--leg-seconds", type=float, default=150.0, help="deadline of each leg")
     ap.add_argument("--ref-fraction", type=float, default=0.125,
                     help="share of one product (inner indices and decompressed rows) per CPU reference step")
     ap.add_argument("--n", type=int, default=0, help="override the workload size")
@@ -87,6 +88,40 @@ def measured_peaks():
             m = json.load(f)
         return float(m.get("hbm_gbs", HBM_PEAK_FALLBACK)), "measured (MEASURED_PEAKS.json hbm_gbs)"
     return HBM_PEAK_FALLBACK, "fallback (6.65 TB/s, earlier copy measurement on this GPU type)"
+
+
+MIXED = "f32 inputs (mixed: int8 residue products or FP32 transforms, FP64 sums and inverse)"
+
+
+def reference_unavailable(why):
+    print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+
+
+class LegDeadline:
+    """Ends the process when a leg does not: the line is printed with the legs
+    that ended (a stuck kernel holds every CUDA call of this process)."""
+
+    def __init__(self, line, legs, seconds):
+        self.line, self.legs, self.seconds = line, legs, seconds
+        self.name, self.t0, self.lock = None, 0.0, threading.Lock()
+        threading.Thread(target=self._watch, daemon=True).start()
+
+    def start(self, name):
+        with self.lock:
+            self.name, self.t0 = name, time.perf_counter()
+
+    def stop(self):
+        with self.lock:
+            self.name = None
+
+    def _watch(self):
+        while True:
+            time.sleep(1.0)
+            with self.lock:
+                if self.name and time.perf_counter() - self.t0 > self.seconds:
+                    self.legs[self.name] = {"error": f"did not end within {self.seconds:g} s"}
+                    print(json.dumps(dict(self.line, legs=self.legs)), flush=True)
+                    os._exit(0)
 
 
 class ClockSampler:
@@ -439,7 +474,10 @@ def run_batch(args, reps, warm, steps, compare_fp64, e2e_steps):
 def bench_batch(args, world, rank, local):
     if args.impl == "reference":
         if rank == 0:
-            print(json.dumps(batch_reference(args)), flush=True)
+            try:
+                print(json.dumps(batch_reference(args)), flush=True)
+            except FileNotFoundError as e:
+                reference_unavailable(f"the reference's sources are absent here, so its library is not built ({e})")
         return
     from compmatmul_b200.replicas import Replicas
     reps = Replicas()
@@ -447,7 +485,7 @@ def bench_batch(args, world, rank, local):
     if rank == 0:
         line = {"metric": METRIC, "value": r.pop("value"), "unit": "products/s", "n_gpus": world,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": "f32 (mixed: FP32 transforms, FP64 reduction)", "data": "synthetic",
+                "dtype": MIXED, "data": "synthetic",
                 "config": batch_config(args.batch_count), "cpu_baseline": None}
         line.update(r)
         print(json.dumps(line), flush=True)
@@ -480,7 +518,9 @@ def serve_stream(srv, pool, arrivals, poll_every=64):
                 srv._live.pop(out.popleft(), None)
     while out:
         rid = out.popleft()
-        done, l = srv.wait(rid, None)
+        done, l = srv.wait(rid, 60.0)
+        if not done:
+            raise TimeoutError(f"request {rid} did not end within 60 s")
         lat.append(l)
         srv._live.pop(rid, None)
     span = time.perf_counter() - t0
@@ -525,7 +565,7 @@ def run_serve(args, rank, extra, compare_fp64, compare_fp64_window=1e9):
         # device pools (and, when enabled, the code/plan residency)
         warm = [srv.submit(q["AT"], q["B"], q["d"], q["b"], q["seed"], q["variant"]) for q in pool_]
         for w in warm:
-            srv.result(w)
+            srv.result(w, timeout=60.0)
         serve_stream(srv, pool_, arr[arr < 1.0])  # one untimed second of the same stream
         st0 = srv.stats()
         l0 = L.cmm_launch_count()
@@ -603,7 +643,7 @@ def bench_serve(args, world, rank, local):
     if rank == 0:
         line = {"metric": METRIC, "value": r.pop("value"), "unit": "products/s", "n_gpus": world,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": "f32 (mixed: FP32 transforms, FP64 reduction)", "data": "synthetic",
+                "dtype": MIXED, "data": "synthetic",
                 "config": serve_config(args), "roofline": None, "cpu_baseline": None}
         line.update(r)
         print(json.dumps(line), flush=True)
@@ -712,15 +752,16 @@ def leg_wht_rows(rows=16384, log2n=13, warm=3, steps=1000):
     return out
 
 
-def run_legs(args, reps, dAT, dB, dC, L):
+def run_legs(args, reps, dAT, dB, dC, L, legs, deadline):
     """Short legs of the other configurations (single GPU, after the
-    headline): every one reports its own steps, clocks and result check."""
+    headline), into `legs`: every one reports its own steps, clocks and result
+    check, and has a deadline."""
     import torch
     from compmatmul_b200.planted import WORKLOADS, planted_problem
-    legs = {}
 
     def guard(name, fn):
         t0 = time.perf_counter()
+        deadline.start(name)
         try:
             legs[name] = fn()
         except Exception as e:  # a failing leg is reported, not hidden
@@ -728,6 +769,7 @@ def run_legs(args, reps, dAT, dB, dC, L):
         legs[name]["leg_wall_s"] = time.perf_counter() - t0
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
+        deadline.stop()
 
     w = WORKLOADS["config2_n16384"]
     if dAT is not None:  # the headline's device inputs (config 2, n = 16384)
@@ -765,7 +807,6 @@ def run_legs(args, reps, dAT, dB, dC, L):
     guard("config5", lambda: dict(run_serve(sargs, reps.rank, extra=False, compare_fp64=1,
                                             compare_fp64_window=2.0),
                                   config=serve_config(sargs)))
-    return legs
 
 
 def reference_single(args, w, n, variant, config):
@@ -827,7 +868,10 @@ def main():
 
     if args.impl == "reference":
         if rank == 0:
-            reference_single(args, w, n, variant, config)
+            try:
+                reference_single(args, w, n, variant, config)
+            except FileNotFoundError as e:
+                reference_unavailable(f"the reference's sources are absent here, so its library is not built ({e})")
         return
 
     import torch
@@ -989,10 +1033,6 @@ def main():
                 "hbm": {"achieved": achieved_gb, "peak": hbm_peak, "unit": "GB/s", "frac": achieved_gb / hbm_peak,
                         "peak_source": hbm_kind, "algorithmic_bytes_per_launch": alg_bytes}}
 
-    legs = None
-    if world == 1 and not args.no_legs and args.workload == "config2_n16384" and not args.n and not args.inner:
-        legs = run_legs(args, reps, dAT if not mixed else None, dB, dC, L)
-
     if rank != 0:
         reps.close()
         return
@@ -1011,7 +1051,7 @@ def main():
         "metric": METRIC, "value": value, "unit": "products/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 (mixed: FP32 transforms, FP64 reduction)" if mixed else "f64",
+        "dtype": MIXED if mixed else "f64",
         "data": "synthetic", "config": config,
         "roofline": roofline,
         "kernel_ms_per_step": {k: v[0] / max(1, args.steps) for k, v in fam.items()},
@@ -1026,8 +1066,10 @@ def main():
         line["plain_fp64_same_inputs"] = {"ms_per_step": fp64_ms, "speedup": fp64_ms / ms_per_step}
     if phases is not None:
         line["cluster_phase_cycles"] = phases
-    if legs is not None:
-        line["legs"] = legs
+    if world == 1 and not args.no_legs and args.workload == "config2_n16384" and not args.n and not args.inner:
+        line["legs"] = {}
+        run_legs(args, reps, dAT if not mixed else None, dB, dC, L, line["legs"],
+                 LegDeadline(line, line["legs"], args.leg_seconds))
     print(json.dumps(line), flush=True)
     reps.close()
 
