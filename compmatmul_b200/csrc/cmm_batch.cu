@@ -924,7 +924,8 @@ bool outputs_meet_inputs(BatchPlan& B) {
 // their memory.  They run in groups that share a work space of at most a third of
 // the free device memory or scratch_cap(); C is formed in the product's own dense
 // output where there is one.  A product that needs more by itself takes the
-// transforms, and all do when the memory is not to be had.
+// transforms, and all do when they are too few to pay for the launches or the
+// memory is not to be had.
 void reserve_product_jobs(BatchPlan& B, cudaStream_t s) {
   B.by_product.assign((size_t)B.count, 0);
   B.shared_c.assign((size_t)B.count, 0);
@@ -961,6 +962,15 @@ void reserve_product_jobs(BatchPlan& B, cudaStream_t s) {
     B.pjobs.push_back(J);
     B.pruns.back().second = k + 1;
   }
+  auto drop = [&] {
+    B.pmem = DevBuf();
+    B.plists = DevBuf();
+    B.pdev = DevBuf();
+    B.pjobs.clear();
+    B.pruns.clear();
+    B.pwhere.clear();
+  };
+  if (!products_pay(B.pjobs.data(), (int)B.pjobs.size(), B.f32, (int)B.pjobs.size() < B.count)) drop();
   if (B.pjobs.empty()) return;
   try {
     B.pmem = DevBuf(most, s);
@@ -969,12 +979,7 @@ void reserve_product_jobs(BatchPlan& B, cudaStream_t s) {
     B.pflags = DevBuf(B.pjobs.size() * sizeof(int), s);
   } catch (const std::bad_alloc&) {
     cudaGetLastError();
-    B.pmem = DevBuf();
-    B.plists = DevBuf();
-    B.pdev = DevBuf();
-    B.pjobs.clear();
-    B.pruns.clear();
-    B.pwhere.clear();
+    drop();
     return;
   }
   B.waits.reset(new WaitFlag());

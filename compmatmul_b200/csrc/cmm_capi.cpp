@@ -362,7 +362,7 @@ static bool product_applicable(int variant, bool f32, const SketchParams& sp, in
   if (sketch_kernel_choice() != 0) return false;
   if (sketch_cluster_applicable(variant, f32, sp.b) && (double)n_a * (double)n_b * (double)n_inner < 1e7)
     return false;
-  return product_faster(variant, f32, sp.d, sp.b, n_a, n_inner, n_b, true);
+  return product_faster(variant, f32, sp.d, sp.b, n_a, n_inner, n_b);
 }
 
 // The caller's dense output as room for C, which it holds until the estimate is

@@ -811,27 +811,59 @@ namespace {
 
 // Additions: a warp's step over one row and window costs the same with one entry
 // or twenty, so sparse rows (few columns, many buckets) pay per step.
-double additions_us(const ProdJob& J, bool alone, int sms) {
+struct AddCost {
+  double spread;   // work that any number of SMs share
+  double cta, row; // of a CTA: its rows, us for one
+  double load;     // CTAs per place on the device
+};
+AddCost additions_cost(const ProdJob& J, int sms) {
   const double db = (double)J.d * (double)(1u << J.log2b), wins = (double)((1u << J.log2b) >> J.logW);
   const double cols = (double)std::min<int64_t>(J.n_b, 4096);
-  double t = (double)J.G * db * 8.0 * 1.5 / 6.5e6;  // partial sketches, written and read
-  if (J.form == kAddGather)
-    return t + 7e-6 * db + (double)J.n_a * J.d * (wins * 1.09e-4 + (double)J.n_b * 2.0e-6);
-  const double ctas = J.d * (J.form == kAddLane ? 1.0 : std::ceil(wins / 16.0));
-  const double load = ctas * (double)J.G / ((double)J.per_sm * sms);  // CTAs per slot
-  const double row = J.form == kAddLane ? 0.3 + 2.1e-4 * cols
-                     : J.per_sm == 1   ? 0.43 + 1.5e-3 * cols / wins
-                                       : 0.5 + 3.6e-3 * cols / wins;
-  return t + (alone ? std::max(1.0, load) : load) * (double)J.n_a / J.G * J.blocks * row;
+  AddCost c{(double)J.G * db * 8.0 * 1.5 / 6.5e6, 0, 0, 0};  // partial sketches, written and read
+  if (J.form == kAddGather) {
+    c.spread += 7e-6 * db + (double)J.n_a * J.d * (wins * 1.09e-4 + (double)J.n_b * 2.0e-6);
+    return c;
+  }
+  c.cta = (double)J.n_a / J.G * J.blocks;
+  c.row = J.form == kAddLane ? 0.3 + 2.1e-4 * cols : J.per_sm == 1 ? 0.43 + 1.5e-3 * cols / wins : 0.5 + 3.6e-3 * cols / wins;
+  c.load = J.d * (J.form == kAddLane ? 1.0 : std::ceil(wins / 16.0)) * (double)J.G / ((double)J.per_sm * sms);
+  return c;
+}
+double product_work(const ProdJob& J, bool f32, int64_t n_inner, double per_plane, double per_entry) {
+  const double na = (double)J.n_a, nb = (double)J.n_b, k = (double)n_inner;
+  return 65536.0 * J.tiles_a * J.tiles_b * std::ceil(k / 128.0) * 128.0 * 2.0 * prod_moduli(f32) / 3.0e9 +
+         k * (na + nb) * per_plane + na * nb * per_entry;
+}
+double product_us(const ProdJob& J, bool f32, int64_t n_inner, int sms) {
+  const AddCost c = additions_cost(J, sms);
+  return 85.0 + product_work(J, f32, n_inner, 9.3e-6, f32 ? 1e-5 : 2e-5) + c.spread + std::max(1.0, c.load) * c.cta * c.row;
 }
 
-double product_us(const ProdJob& J, bool f32, int64_t n_inner, bool alone, int sms) {
-  const double na = (double)J.n_a, nb = (double)J.n_b, k = (double)n_inner;
-  const double gemm = 65536.0 * J.tiles_a * J.tiles_b * std::ceil(k / 128.0) * 128.0 * 2.0 * prod_moduli(f32) / 3.0e9;
-  const double planes = k * (na + nb), entries = na * nb;
-  // among other jobs there are no launches to wait for, and every kernel fills the device
-  if (!alone) return 5.0 + gemm + planes * (f32 ? 5e-6 : 8e-6) + entries * (f32 ? 4e-6 : 9e-6) + additions_us(J, alone, sms);
-  return 85.0 + gemm + planes * 9.3e-6 + entries * (f32 ? 1e-5 : 2e-5) + additions_us(J, alone, sms);
+// Among other jobs, fitted to plans of 1 to 32 equal products (240 of them, 9 % rms;
+// transforms 20): the work of all, a chain of launches, and the longest CTA of the
+// additions, however few there are.
+struct JobCost {
+  double work, load, chain;
+};
+JobCost job_cost(const ProdJob& J, bool f32, int sms) {
+  const AddCost c = additions_cost(J, sms);
+  const double wins = (double)((1u << J.log2b) >> J.logW), cols = (double)std::min<int64_t>(J.n_b, 4096);
+  const double row = J.form == kAddLane ? 0.155 + 9.6e-5 * cols : 0.155 + 4.2e-3 * cols / wins + 7e-3 * std::min(wins, 16.0);
+  return {1.61 * (product_work(J, f32, J.kc, f32 ? 5e-6 : 8e-6, f32 ? 4e-6 : 9e-6) + c.spread), 1.07 * c.load * c.cta * c.row,
+          c.cta * row};
+}
+// the batch transform kernel: fixed, per 4096 buckets, per d k b log b, per d k (n_a +
+// n_b), per d b log b; FFT FP64, FP32, FWHT FP64, FP32
+struct BatchCost {
+  double fixed, buckets, work, rows, inverse;
+};
+constexpr BatchCost kBatchCost[4] = {{75, 17.3, 9.6e-7, 2.6e-5, 1.45e-6}, {58, 14.2, 5.4e-7, 1.27e-5, 1.3e-7},
+                                     {86, 2.4, 6.2e-7, 1.7e-5, 0}, {63, 1.3, 4.05e-7, 1.24e-5, 0}};
+const BatchCost& batch_cost(int variant, bool f32) { return kBatchCost[(variant == kVariantFFT ? 0 : 2) + (f32 ? 1 : 0)]; }
+double batch_transforms_us(const ProdJob& J, bool f32) {
+  const BatchCost& c = batch_cost(J.variant, f32);
+  const double blog = (double)(1u << J.log2b) * J.log2b;
+  return J.d * ((double)J.kc * (c.work * blog + c.rows * (double)(J.n_a + J.n_b)) + c.inverse * blog);
 }
 
 // The transform kernels that would run: launches and plan, the inverse per d b
@@ -839,12 +871,11 @@ double product_us(const ProdJob& J, bool f32, int64_t n_inner, bool alone, int s
 struct TransformCost {
   double fixed, inverse, work, work32, rows;
 };
-double transforms_us(int variant, bool f32, int d, int b, double k, double n, bool alone) {
+double transforms_us(int variant, bool f32, int d, int b, double k, double n) {
   const bool fft = variant == kVariantFFT;
   double log2b = 0;
   while ((1 << (int)log2b) < b) ++log2b;
   const double blog = (double)b * log2b;
-  if (!alone) return d * k * ((fft && !f32 ? 0.85e-6 : 0.5e-6) * blog + 7e-6 * n);  // the batch kernel
   static const TransformCost kSmall[2] = {{55, 0, 2.6e-6, 2.4e-6, 4.5e-6}, {52, 0, 2.2e-6, 2.1e-6, 7.5e-6}};
   static const TransformCost kSlab[2] = {{135, 7e-6, 7.2e-7, 4.2e-7, 8e-6}, {138, 2e-6, 3.6e-7, 4.4e-7, 6e-6}};
   static const TransformCost kGroup[2] = {{135, 7.6e-6, 8e-7, 4.2e-7, 8e-6}, {132, 4e-6, 4.5e-7, 3.1e-7, 1.3e-5}};
@@ -861,17 +892,36 @@ double transforms_us(int variant, bool f32, int d, int b, double k, double n, bo
 
 }  // namespace
 
-bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone) {
+bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
   ProdJob J{};
-  product_geometry(J, variant, d, b, n_a, n_b, std::min(n_inner, kProdMaxK), alone, num_sms());
-  return product_us(J, f32, n_inner, alone, num_sms()) <
-         transforms_us(variant, f32, d, b, (double)n_inner, (double)(n_a + n_b), alone);
+  product_geometry(J, variant, d, b, n_a, n_b, std::min(n_inner, kProdMaxK), true, num_sms());
+  return product_us(J, f32, n_inner, num_sms()) <
+         transforms_us(variant, f32, d, b, (double)n_inner, (double)(n_a + n_b));
 }
 
 bool product_among_others(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b) {
   const int choice = sketch_kernel_choice();
-  return (choice == 0 || choice == 3) && n_inner <= kProdMaxK && product_supported(b, n_a, n_inner, n_b) &&
-         (choice == 3 || product_faster(variant, f32, d, b, n_a, n_inner, n_b, false));
+  if (choice == 1 || choice == 2 || n_inner > kProdMaxK || !product_supported(b, n_a, n_inner, n_b)) return false;
+  if (choice == 3) return true;
+  ProdJob J{};
+  product_geometry(J, variant, d, b, n_a, n_b, n_inner, false, num_sms());
+  const JobCost c = job_cost(J, f32, num_sms());
+  return 5.0 + c.work + c.load < batch_transforms_us(J, f32);
+}
+
+bool products_pay(const ProdJob* jobs, int count, bool f32, bool others) {
+  if (sketch_kernel_choice() == 3) return true;
+  double work = 57.0, load = 0.0, chain = 0.0, transforms = 0.0, fixed = 0.0;
+  for (int i = 0; i < count; ++i) {
+    const JobCost c = job_cost(jobs[i], f32, num_sms());
+    work += c.work;
+    load += c.load;
+    chain = std::max(chain, c.chain);
+    transforms += batch_transforms_us(jobs[i], f32);
+    const BatchCost& b = batch_cost(jobs[i].variant, f32);
+    fixed = std::max(fixed, b.fixed + b.buckets * (double)(1u << jobs[i].log2b) / 4096.0);
+  }
+  return work + std::sqrt(std::hypot(load * load, chain * chain)) < transforms + (others ? 0.0 : fixed);
 }
 
 }  // namespace cmm

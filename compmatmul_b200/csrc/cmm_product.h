@@ -39,7 +39,7 @@ struct ProdJob {
   uint32_t* ent;          //   and entries, 2 d x n_b
   double *part, *p;       // G x d x b partial sketches; d x b
   int d, log2b, variant;
-  int form;               // which additions (plan_product_sketch)
+  int form;               // which additions (product_geometry)
   int logW, G;            // window of a warp, row groups
   int per_sm;             // CTAs of the additions per SM
   int add_begin, add_x;   // their first CTA in the launch of their kind, CTAs per (t, row group)
@@ -54,12 +54,14 @@ inline size_t prod_residue_row(const ProdJob& J, bool f32) { return (size_t)prod
 // the largest n_a n_b whose product is formed (8 GiB of FP64)
 constexpr int64_t kProdMaxEntries = (int64_t)1 << 30;
 
-// Whether the product sketch takes these sizes, and whether it is estimated to
-// be faster than the transforms (alone: with both forms' fixed costs).
+// Whether the product sketch takes these sizes, and whether it is estimated to be
+// faster than the transforms: for a single call, for a product of a batch plan or
+// a request, and for the products of a plan together, whose launches come on top
+// (others: the plan runs transforms for other products anyway).
 bool product_supported(int b, int64_t n_a, int64_t n_inner, int64_t n_b);
-bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b, bool alone);
-// whether a product of a batch plan or a request takes it
+bool product_faster(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b);
 bool product_among_others(int variant, bool f32, int d, int b, int64_t n_a, int64_t n_inner, int64_t n_b);
+bool products_pay(const ProdJob* jobs, int count, bool f32, bool others);
 
 // bytes of the residue planes of a chunk of k inner indices
 inline size_t prod_plane_bytes(bool f32, int64_t n_a, int64_t n_b, int64_t k) {

@@ -155,7 +155,7 @@ def test_plan_with_products_above_the_scratch_limit(gpu, monkeypatch):
 
     from compmatmul_b200.batch import BatchPlan
     prods = [dict(AT=m[0], B=m[1], d=5, b=8192, seed=3 + i) for i, m in
-             enumerate([random(200, 300, 310, 1), random(1500, 1024, 1024, 2), random(200, 310, 300, 3)])]
+             enumerate([random(600, 300, 310, 1), random(1500, 1024, 1024, 2), random(600, 310, 300, 3)])]
 
     def run(limit):
         if limit:
@@ -167,7 +167,7 @@ def test_plan_with_products_above_the_scratch_limit(gpu, monkeypatch):
         plan.close()
         return out
 
-    whole, some, none = run(0), run(16 << 20), run(1 << 20)  # (the small ones need 5 MB each, the large one 60)
+    whole, some, none = run(0), run(16 << 20), run(1 << 20)  # (the small ones need 7 MB each, the large one 60)
     for k in range(3):
         same = torch.equal(whole[k][0], some[k][0])
         assert same == (k != 1)  # the same route gives the same bits

@@ -78,7 +78,7 @@ def test_only_the_callers_thread_reports_it(gpu, monkeypatch):
     assert np.abs(seen["after"] - good).max() <= 1e-13 * np.abs(good).max()
 
 
-def problems(count, f32, lo=256, hi=700):
+def problems(count, f32, lo=400, hi=1200):
     import torch
 
     from compmatmul_b200.planted import batch_shapes, planted_problem_device
@@ -98,7 +98,7 @@ def test_only_the_plan_reports_it(gpu, monkeypatch, where, own_stream):
     import torch
 
     from compmatmul_b200.batch import BatchPlan
-    probs = problems(4, True)
+    probs = problems(12, True)
     good, bad = BatchPlan(probs, f32=True, tune=False), BatchPlan(probs, f32=True, tune=False)
     stream = None if own_stream else torch.cuda.Stream()
     monkeypatch.setenv("CMM_TEST_PRODUCT_WAIT", where)  # (captured with the kernels of the first run)
