@@ -774,6 +774,7 @@ struct BatchPlan {
   std::unique_ptr<WaitFlag> waits;
   int64_t max_hash_total = 0, max_inner = 0;
   const double2* tw4096 = nullptr;
+  cudaEvent_t ran = nullptr;  // the last run, on a caller's stream
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int64_t launches_per_run = 0;
@@ -1323,7 +1324,11 @@ void batch_run(BatchPlan* B, cudaStream_t user) {
     CMM_CUDA(cudaGraphLaunch(B->exec, s));
   }
   count_launch((int)B->launches_per_run);
-  if (user) return;
+  if (user) {
+    if (!B->ran) CMM_CUDA(cudaEventCreateWithFlags(&B->ran, cudaEventDisableTiming));
+    CMM_CUDA(cudaEventRecord(B->ran, s));
+    return;
+  }
   CMM_CUDA(cudaStreamSynchronize(s));
   if (B->waits && B->waits->take()) throw runtime_error("product sketch: a wait ran out; its sketches are invalid");
 }
@@ -1360,6 +1365,10 @@ void batch_config(const BatchPlan* B, int i, int* log2_slab, int* radix, int* gr
 void batch_destroy(BatchPlan* B) {
   if (!B) return;
   cudaStream_t s = B->stream;
+  if (B->ran) {  // its kernels still use the buffers and the flag
+    cudaEventSynchronize(B->ran);
+    cudaEventDestroy(B->ran);
+  }
   if (s) cudaStreamSynchronize(s);
   delete B;  // buffers are released on s
   if (s) {

@@ -616,7 +616,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kProdThreads, 1)
 // 2^2T < 0.34 M keeps S / M 0.16 away from a tie), modulo 2^128 (2^64).  The
 // top limb of 15 moduli needs 32 bits only.  Thread = column j, four rows i at a
 // time.  Bound by the multiply-adds of the limbs (4096 x 4096, 15 moduli: 168
-// us with a fixed-point sum for t and 64-bit top limbs, @C now).
+// us with a fixed-point sum for t and 64-bit top limbs, 153 now).
 template <int N, int I>
 __device__ __forceinline__ void crt_terms(const uint32_t (&w)[16], uint32_t pick, unsigned long long (&s)[3], uint32_t& top) {
   constexpr U128 P = mod_product(N, I);
