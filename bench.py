@@ -1,8 +1,8 @@
 """Benchmark of the compressed product on B200.
 
 One step = one compressed product of a planted-entry workload: hash codes,
-per-k balancing, fused sketch/transform/accumulate, inverse, dense median
-decompression of all n_a x n_b entries into HBM, and device top-K recovery
+per-k balancing, the sketch (residue products and additions, or fused
+sketch/transform/accumulate and inverse), dense median decompression of all n_a x n_b entries into HBM, and device top-K recovery
 (K = planted count).  Default workload: n = 16384 square FP64, b = 2^16,
 d = 9, FFT variant, K = 256 (inputs 4.3 GB > L2, so no flush is needed).
 

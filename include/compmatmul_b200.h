@@ -132,7 +132,12 @@ int cmm_hash_params(int hash_kind, int n, uint64_t buckets, uint64_t seed, void*
  * reference is host-only).  All pointers are device pointers.
  * ------------------------------------------------------------------- */
 
-/* Sketch only: dP (d x b FP64) from dAT, dB. */
+/* Sketch only: dP (d x b FP64) from dAT, dB.  Where the product sketch is
+ * the faster form, the product of the inputs (each column scaled and rounded
+ * to 2^-58 of its norm) is formed exactly by int8 residue products on the
+ * tensor cores and added up in FP64; else the FP64 transforms run.  The calls
+ * return before their kernels do; a bounded wait in them that runs out makes
+ * the sketch NaN and is reported by the thread's next product call. */
 int cmm_dev_compressed_product(int variant, int hash_kind, int64_t n_a, int64_t n_inner,
                                int64_t n_b, const double* dAT, const double* dB, int d, int b,
                                uint64_t seed, double* dP, void* stream);
@@ -187,7 +192,9 @@ int cmm_dev_sketch_topk(int variant, int hash_kind, int64_t n_a, int64_t n_b, in
 int cmm_dev_decompress_dense(int variant, int hash_kind, int64_t n_a, int64_t n_b, int d, int b,
                              uint64_t seed, const double* dP, double* dC, void* stream);
 
-/* Compressed product + dense decompression (matmul_fft / matmul_fwht). */
+/* Compressed product + dense decompression (matmul_fft / matmul_fwht).  dC
+ * may hold the product of the inputs until the estimate is written; where it
+ * shares memory with an input it is written after both were read. */
 int cmm_dev_matmul(int variant, int hash_kind, int64_t n_a, int64_t n_inner, int64_t n_b,
                    double* dC, const double* dAT, const double* dB, int d, int b, uint64_t seed,
                    void* stream);
